@@ -13,7 +13,7 @@ void count_launch();
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRowsPerCta = 512;   // gather: ids staged per CTA
+constexpr int kRowsPerCta = 512;   // gather: most ids staged per CTA
 constexpr int kMaxStagedIds = 8192;  // bag-mean: ids staged per CTA (int32)
 
 __device__ __forceinline__ uint4 ld_nc_v4(const uint4* p) {
@@ -38,14 +38,14 @@ template <typename I>
 __global__ void __launch_bounds__(kThreads)
 gather_rows_kernel(const uint4* __restrict__ table, int64_t vocab_rows, int chunks, const void* __restrict__ ids,
                    int64_t n, int64_t seq_len, int64_t ids_batch_stride, uint4* __restrict__ out,
-                   int64_t out_stride_chunks, int out_col0_chunks, int lanes_per_row) {
+                   int64_t out_stride_chunks, int out_col0_chunks, int lanes_per_row, int rows_per_cta) {
     __shared__ int32_t ids_s[kRowsPerCta];
     const int tid = threadIdx.x;
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kRowsPerCta;
-    const int here = static_cast<int>(n - base < kRowsPerCta ? n - base : kRowsPerCta);
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * rows_per_cta;
+    const int here = static_cast<int>(n - base < rows_per_cta ? n - base : rows_per_cta);
     for (int j = tid; j < here; j += kThreads) {
         const int64_t i = base + j;
-        const int64_t b = i / seq_len;
+        const int64_t b = i < seq_len ? 0 : i / seq_len;
         const int64_t l = i - b * seq_len;
         int64_t id = load_id<I>(ids, b * ids_batch_stride + l);
         id = id < 0 ? 0 : (id > vocab_rows - 1 ? vocab_rows - 1 : id);
@@ -136,7 +136,7 @@ bag_mean_kernel(BagArgs a, const void* __restrict__ ids, T* __restrict__ out) {
     const int lane_g = tid % G;
     const int n_groups = kThreads / G;
     const int chunks = a.chunks;
-    constexpr int U = 4;  // table rows in flight per lane
+    constexpr int U = 8;  // table rows in flight per lane: the ids of a usual bag in one round
 
     if (a.max_bag == 1) {
         // One id per bag (the field bank of single-valued features): the pooled row is the table row itself, so a lane
@@ -384,8 +384,15 @@ int bag_launch(BagArgs a, const void* ids, int ids_dtype, void* out, cudaStream_
     int per = kMaxStagedIds / a.max_bag;
     if (per < 1) return TB200_ERR_UNSUPPORTED;
     if (per > 256) per = 256;
-    a.bags_per_cta = per;
     a.lanes_per_row = lanes_for(a.chunks);
+    // The rows of a bag are a chain "id -> row": with few bags the chip is only full when every lane group has one bag and
+    // all SMs have CTAs (8192 bags of 8 ids, 128 fp16 columns: 32 CTAs of 256 bags took 29.8 us, 512 CTAs of 16 take 5.6 us);
+    // with many bags, 256 per CTA keep the id reads long.
+    const int groups = kThreads / a.lanes_per_row;
+    const int64_t share = (a.n_bags + 8ll * device_info().sm_count - 1) / (8ll * device_info().sm_count);
+    const int64_t want = (share + groups - 1) / groups * groups;
+    if (want < per) per = static_cast<int>(want);
+    a.bags_per_cta = per;
     const int64_t grid = (a.n_bags + per - 1) / per;
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     const size_t smem = static_cast<size_t>(per) * a.max_bag * sizeof(int32_t);
@@ -502,18 +509,24 @@ extern "C" int tb200_gather_rows(const void* table, int64_t vocab_rows, int32_t 
         return TB200_ERR_ALIGN;
     if (!device_info().valid) return TB200_ERR_DEVICE;
     const int chunks = dim * es / 16;
-    const int64_t grid = (n + kRowsPerCta - 1) / kRowsPerCta;
-    if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int G = lanes_for(chunks);
+    // a round of a CTA is four rows per lane group; few rows are spread over all SMs, many take 512 per CTA so that the id
+    // reads stay long
+    const int round = 4 * (kThreads / G);
+    const int64_t share = (n + 8ll * device_info().sm_count - 1) / (8ll * device_info().sm_count);
+    int64_t rows_per_cta = (share + round - 1) / round * round;
+    if (rows_per_cta > kRowsPerCta) rows_per_cta = kRowsPerCta;
+    const int64_t grid = (n + rows_per_cta - 1) / rows_per_cta;
+    if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (ids_dtype == TB200_I64)
         gather_rows_kernel<int64_t><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(
             static_cast<const uint4*>(table), vocab_rows, chunks, ids, n, seq_len, ids_batch_stride,
-            static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G);
+            static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G, static_cast<int>(rows_per_cta));
     else
         gather_rows_kernel<int32_t><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(
             static_cast<const uint4*>(table), vocab_rows, chunks, ids, n, seq_len, ids_batch_stride,
-            static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G);
+            static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G, static_cast<int>(rows_per_cta));
     count_launch();
     return launch_status();
 }

@@ -1,21 +1,21 @@
 // Attention backward for the padded (B, H, L, D) layout: dq, dk, dv from q, k, v, o and the upstream gradient, with
 // the same mask rule as the forward kernels (valid prefix, always-valid suffix, causal, key-validity map, padded
-// queries that return their own value row).  It is the first, plain form of the training-side kernel (the reference's
-// is `flash_attention_backward`, accelerators/attention/kernels/tilelang.py:440-701): fp32 arithmetic on the CUDA
-// cores, scores recomputed instead of stored, two kernels and no atomics, so the gradients do not depend on
-// scheduling:
+// queries that return their own value row); the reference's is `flash_attention_backward`
+// (accelerators/attention/kernels/tilelang.py:440-701).  16-bit tensors of head_dim 32 / 64 / 128 take the tensor-core
+// kernels of attn_bwd_mma.cu; this file holds the entry point and the plain form that serves the rest (fp32 tensors, other
+// head dims, rows off the 16-byte grid): fp32 arithmetic on the CUDA cores, scores recomputed instead of stored, two
+// kernels and no atomics, so the gradients do not depend on scheduling:
 //   query kernel   one warp per (sample, head, query i):  scores -> row maximum and sum (their log2 "lse" and
 //                  delta_i = dO_i . O_i go to a workspace), ds_ij = p_ij (dO_i . v_j - delta_i),
 //                  dq_i = scale * sum_j ds_ij k_j
 //   key kernel     one warp per (sample, head, key j):    p_ij = exp2(s_ij - lse_i) for the queries that see j,
 //                  dv_j = sum_i p_ij dO_i,  dk_j = scale * sum_i ds_ij q_i
 // A padded query (forward: o_i = v_i) passes its gradient straight to dv_i and has no dq; a query without a visible
-// key (forward: zeros) has no gradient at all.  Work is O(Lq Lk D) per kernel without tensor cores: meant for
-// correctness and for small training shapes, not for the serving path.
+// key (forward: zeros) has no gradient at all.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "attn_common.cuh"
+#include "attn_bwd.cuh"
 #include "tb200_common.cuh"
 
 namespace tb200 {
@@ -27,17 +27,6 @@ constexpr int kMaxD = 256;
 constexpr int kMaxL = 4096;
 constexpr float kSelfRow = INFINITY;      // lse marker: padded query, gradient goes to its own value row
 constexpr float kEmptyRow = -INFINITY;    // lse marker: no visible key
-
-struct BwdArgs {
-    AttnArgs a;                 // q, k, v, o and their strides, the mask
-    const void* d_o;            // strides of o
-    void* dq;                   // strides of q
-    void* dk;                   // strides of k
-    void* dv;                   // strides of v
-    float* lse;                 // [B, H, Lq]
-    float* delta;               // [B, H, Lq]
-    float scale;
-};
 
 template <typename T>
 __device__ __forceinline__ float to_f(T x) { return static_cast<float>(x); }
@@ -61,29 +50,6 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
-}
-
-struct RowMask {
-    int valid_len, ns_start, lk;
-    bool causal;
-    const uint8_t* kvalid;
-    __device__ __forceinline__ bool sees(int query, int key) const {
-        return kvalid != nullptr ? (kvalid[key] != 0 && (!causal || key <= query))
-                                 : attn_visible(query, key, valid_len, ns_start, lk, causal);
-    }
-    __device__ __forceinline__ bool padded_query(int pos) const {
-        return kvalid != nullptr ? kvalid[pos] == 0 : (pos >= valid_len && pos < ns_start);
-    }
-};
-
-__device__ __forceinline__ RowMask make_mask(const AttnArgs& a, int b) {
-    RowMask m;
-    m.lk = a.Lk;
-    m.valid_len = a.seq_len != nullptr ? min(max(a.seq_len[b], 0), a.Lk) : a.Lk;
-    m.ns_start = min(a.ns_start, a.Lk);
-    m.causal = a.causal != 0;
-    m.kvalid = a.key_valid != nullptr ? a.key_valid + static_cast<int64_t>(b) * a.Lk : nullptr;
-    return m;
 }
 
 constexpr int kWarpsQ = 4;
@@ -298,6 +264,7 @@ extern "C" int tb200_attn_bwd(const void* q, const void* k, const void* v, const
     g.delta = g.lse + static_cast<int64_t>(B) * H * Lq;
     g.scale = scale;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (attn_bwd_mma_supported(g, D, dtype)) return attn_bwd_mma(g, D, dtype, s);
     switch (dtype) {
         case TB200_F32: return launch<float>(g, D, s);
         case TB200_F16: return launch<__half>(g, D, s);

@@ -5,6 +5,7 @@
 // region only copy their value rows.  The tcgen05 kernel covers the head_dim-64 bf16 hot shape;
 // this one covers everything else.
 #include "attn_common.cuh"
+#include "attn_mma_tile.cuh"
 #include "tb200_common.cuh"
 
 namespace tb200 {
@@ -16,71 +17,6 @@ constexpr int kBM = 64;  // query rows per CTA (16 per warp)
 constexpr int kBN = 64;
 constexpr int kKvStages = 2;  // K / V ring depth (three stages were measured: no faster)
 constexpr int kThreads = 128;
-
-template <int D>
-__device__ __forceinline__ int swz(int row, int chunk) {  // element offset of a 16-byte chunk
-    constexpr int CH = D / 8;
-    if (CH >= 8) return row * D + ((chunk ^ (row & 7)) << 3);
-    if (CH == 4) return row * D + ((chunk ^ ((row >> 1) & 3)) << 3);
-    return row * D + ((chunk ^ ((row >> 2) & 1)) << 3);
-}
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
-    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-    const int bytes = pred ? 16 : 0;  // src-size 0 -> zero fill
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
-    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(s));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
-    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(s));
-}
-
-template <typename T>
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma16816<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
-                                                        uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma16816<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-template <typename T>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi);
-template <>
-__device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
-template <>
-__device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
-    __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-}
 
 // rows [row0, row0 + 64) of a [*, D] strided matrix -> swizzled shared tile; rows >= n_rows are zero
 template <typename T, int D>
@@ -495,12 +431,6 @@ attn_tiny_kernel(const AttnArgs a) {
 // the other in the same warp.  Masks: packed batches only (every key valid), causal aligned at the end when
 // the queries have their own offsets.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ float fq_ex2(float x) {   // 2^x, -inf -> 0
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 constexpr int kFqWarps = 4;
 constexpr int kFqStages = 3;
 constexpr int kFqRows = 16;    // keys per tile = queries per tile
@@ -638,14 +568,14 @@ attn_fewq_kernel(const AttnArgs a) {
                 mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
                 const float m_new = fmaxf(m_run[hr], mx);
                 const float ms = (m_new == -INFINITY ? 0.f : m_new) * a.scale_log2;
-                const float corr = fq_ex2(m_run[hr] * a.scale_log2 - ms);   // first tile: exp2(-inf) = 0
+                const float corr = ex2_approx(m_run[hr] * a.scale_log2 - ms);   // first tile: exp2(-inf) = 0
                 m_run[hr] = m_new;
                 float sum = 0.f;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const float p = fq_ex2(s[j][2 * hr + e] * a.scale_log2 - ms);
+                        const float p = ex2_approx(s[j][2 * hr + e] * a.scale_log2 - ms);
                         s[j][2 * hr + e] = p;
                         sum += p;
                     }

@@ -327,10 +327,20 @@ int tb200_attn_fwd(const void* q, const void* k, const void* v, void* o, int32_t
                    const int32_t* cu_rows_q, const uint8_t* key_valid, int32_t ns_start, int32_t causal, int32_t padded_query_self, float scale, int dtype,
                    int32_t kernel, int64_t total_rows, int32_t* status_word, void* stream);
 
+/* Describes bool masks [B, H, Lq, Lk] (one byte per element, strides in bytes, unit stride along the keys; stride_h 0 = one mask
+ * for all heads) by lengths, as `_plan_tilelang_flash_attention_mask` does (accelerators/attention/flash_attention.py:149-198)
+ * and beyond it for an always-valid suffix of keys.  lens: device int32 [B] = valid prefix (Lk where nothing is padded).
+ * verdict: 16-byte aligned int32 [B, 4] that the device can write and the host reads after synchronising (pinned host
+ * memory), per sample: form (0 = not recognised, 1 = the same keys for every query, 2 = causal over the valid keys with
+ * padded queries seeing themselves), prefix, suffix, and whether the sample has padding (1), none (0) or is the identity (2). */
+int tb200_mask_plan(const uint8_t* mask, int64_t stride_b, int64_t stride_h, int64_t stride_q, int32_t B, int32_t H, int32_t Lq,
+                    int32_t Lk, int32_t* lens, int32_t* verdict, void* stream);
+
 /* Attention backward for the padded (B, H, L, D) layout: dq, dk, dv from q, k, v, o and the upstream gradient d_o,
- * under the same mask arguments as tb200_attn_fwd (no packed batches).  First, plain form of the reference's
- * `flash_attention_backward` (accelerators/attention/kernels/tilelang.py:440-701; preprocess :395-437): fp32 arithmetic,
- * scores recomputed, two kernels (per query row, per key row), no atomics.  strides: the 12 values of tb200_attn_fwd;
+ * under the same mask arguments as tb200_attn_fwd (no packed batches): the reference's `flash_attention_backward`
+ * (accelerators/attention/kernels/tilelang.py:440-701; preprocess :395-437), scores recomputed, two kernels (per query
+ * row, per key row), no atomics.  16-bit tensors of head_dim 32 / 64 / 128 with 16-byte aligned rows run on the tensor cores
+ * with P and dS kept in two 16-bit parts, the rest in fp32 on the CUDA cores.  strides: the 12 values of tb200_attn_fwd;
  * d_o uses o's strides, dq / dk / dv those of q / k / v.  workspace: tb200_attn_bwd_workspace_bytes(B, H, Lq) bytes
  * of device memory (log-sum-exp and dO.O per query row).  D <= 256, Lq, Lk <= 4096; fp32, fp16 or bf16. */
 int64_t tb200_attn_bwd_workspace_bytes(int32_t B, int32_t H, int32_t Lq);

@@ -9,6 +9,7 @@ for an accelerated backend that is unavailable
 from __future__ import annotations
 
 import ctypes
+import importlib
 import threading
 from pathlib import Path
 
@@ -48,6 +49,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_bias_act_rows": (_INT, [_P, _I64, _I32, _P, _I64, _I32, _INT, _P]),
     "tb200_bag_mean_fwd": (_INT, [_P, _I64, _I32, _P, _INT, _I64, _I32, _P, _INT, _P]),
     "tb200_bag_mean_bwd": (_INT, [_P, _INT, _P, _P, _P, _I64, _I32, _I32, _I64, _INT, _P]),
+    "tb200_mask_plan": (_INT, [_P, _I64, _I64, _I64, _I32, _I32, _I32, _I32, _P, _P, _P]),
     "tb200_attn_bwd_workspace_bytes": (_I64, [_I32, _I32, _I32]),
     "tb200_attn_bwd": (_INT, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I32, _I32, _I32, _I32, _I32, _P, _P, _P, _I32, _I32, _I32,
                               _F, _INT, _P]),
@@ -109,6 +111,15 @@ def load() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = lib
         return lib
+
+
+def native():
+    """The host module (``_native.so``: the operator calls and the engine's forward in C++ on torch tensors)."""
+    load()
+    try:
+        return importlib.import_module("taac_2026_b200._native")
+    except ImportError as err:
+        raise RuntimeError(f"cuda backend requested but the host module does not load ({err}); run `python -m taac_2026_b200.build`") from err
 
 
 def strerror(code: int) -> str:

@@ -75,6 +75,20 @@ def set_kernel_timing(sink: list | None) -> None:
     _TIMING = sink
 
 
+class _LazyHost:
+    """Stands for the host module until the first call."""
+
+    def __getattr__(self, name: str):
+        global _host
+        _host = _lib.native()
+        return getattr(_host, name)
+
+
+# The plain form of an operator call (contiguous CUDA tensors of one type, nothing timed) goes to the host module, which
+# answers None for every other form and for what the library rejects; the code below then handles it or words the error.
+_host: Any = _LazyHost()
+
+
 class _timed:
     __slots__ = ("name", "meta", "start")
 
@@ -167,6 +181,10 @@ def rms_norm(
     ``in_bias`` (an extension, [cols]) is added to every row in fp32 before the statistics:
     ``rms_norm(x + in_bias)`` without the pass that would form the sum.
     """
+    if _TIMING is None and in_bias is None and backend == "cuda":
+        fast = _host.rms_norm(x, weight, eps)
+        if fast is not None:
+            return fast
     matrix, normalized_weight, original_shape = _normalize_rms_norm_inputs(x, weight)
     resolved_rms_norm_backend(matrix, backend, eps=eps, block_rows=block_rows)
     if in_bias is None and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad) and norm_backward_supported(matrix):
@@ -313,6 +331,10 @@ def layer_norm(
 
     ``pre_silu=True`` (an extension) normalises ``silu(x)`` instead, the SiLU result rounded to the tensor's
     dtype as a separate activation would leave it: the ``Linear -> SiLU -> LayerNorm`` tail in one pass."""
+    if _TIMING is None and backend == "cuda":
+        fast = _host.layer_norm(x, weight, bias, eps, pre_silu)
+        if fast is not None:
+            return fast
     matrix, normalized_weight, normalized_bias, original_shape = _normalize_layer_norm_inputs(x, weight, bias)
     resolved_layer_norm_backend(matrix, backend, eps=eps, block_rows=block_rows)
     if not pre_silu and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or bias.requires_grad) \
@@ -372,6 +394,10 @@ def embedding_bag_mean(
     block_cols: int | None = None,
 ) -> torch.Tensor:
     """Fixed-hotness bag mean with padding id 0 (``F.embedding_bag(..., mode="mean", padding_idx=0)``)."""
+    if backend == "cuda":
+        fast = _host.embedding_bag_mean(embedding_weight, values)
+        if fast is not None:
+            return fast
     weight, ids = _normalize_embedding_bag_mean_inputs(embedding_weight, values)
     resolved_embedding_bag_mean_backend(weight, ids, backend, block_rows=block_rows, block_cols=block_cols)
     out = torch.empty((ids.shape[0], weight.shape[1]), dtype=weight.dtype, device=weight.device)
@@ -389,6 +415,9 @@ def embedding_bag_mean_backward(values: torch.Tensor, grad_out: torch.Tensor, nu
     of shape ``[num_embeddings, dim]`` with one entry per bag position, ``grad_out[b] / valid_count[b]`` at the looked-up
     row — what `SparseEmbeddingBagMean.backward` returns (modeling/embeddings.py:34-62); padded positions name row 0
     with zeros instead of being dropped, so the layout is fixed and no compaction pass is needed."""
+    fast = _host.embedding_bag_mean_backward(values, grad_out, num_embeddings)
+    if fast is not None:
+        return fast
     _require_backend("embedding_bag_mean_backward", "cuda")
     _require_cuda_tensors("cuda embedding_bag_mean_backward", values, grad_out)
     if values.ndim != 2 or grad_out.ndim != 2 or grad_out.shape[0] != values.shape[0]:
@@ -848,6 +877,11 @@ def varlen_attention(
     sample's row count.  fp16 / bf16 run on the tensor-core kernels; fp32 tensors take a plain fp32 kernel meant
     for score-parity runs against the reference's fp32 torch path (``flash_attention`` keeps the reference's
     policy of computing fp32 callers in bf16)."""
+    if _TIMING is None and cu_rows is None and cu_rows_q is None and key_valid is None and out is None and not check \
+            and layout in ("bhld", "blhd"):
+        fast = _host.varlen_attention(q, k, v, seq_len, ns_start, causal, padded_query_self, scale, layout == "blhd", kernel, status)
+        if fast is not None:
+            return fast
     _require_backend("varlen_attention", "cuda")
     _require_cuda_tensors("cuda varlen_attention", q, k, v, seq_len, cu_rows)
     if q.dtype not in _DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype:
@@ -943,6 +977,10 @@ def flash_attention(
     backend (accelerators/attention/flash_attention.py:249-252).  The tile-shape arguments are
     accepted for signature compatibility; the kernel owns its tiling."""
     del block_m, block_n, num_stages, threads
+    if _TIMING is None and backend == "cuda" and dropout_p == 0.0:
+        fast = _host.flash_attention(q, k, v, attn_mask, is_causal)
+        if fast is not None:
+            return fast
     q, k, v = _normalize_flash_attention_inputs(q, k, v)
     resolved_flash_attention_backend(
         q, k, v, backend, attn_mask=attn_mask, dropout_p=dropout_p, training=training, is_causal=is_causal
@@ -1102,6 +1140,11 @@ def ffn_mx(x: torch.Tensor, weights: MxFfnWeights, *, residual: torch.Tensor | N
     """bf16 [..., d] -> bf16 [..., d_out] like ``ffn_fp8``, with power-of-two block scales applied inside the
     block-scaled tensor-core instruction: quantise, GEMM 1 with fused (gated) SiLU and re-quantisation, GEMM 2 with
     fused bias / residual."""
+    if _TIMING is None and not check:
+        fast = _host.ffn_mx(x, weights.w_up, weights.a_up, weights.b_up, weights.w_down, weights.a_down, weights.b_down,
+                            weights.hidden, weights.gated, residual, status)
+        if fast is not None:
+            return fast
     shape = x.shape
     x2 = x.reshape(-1, shape[-1])
     xq, xa = quantize_activation_mx(x2)
@@ -1316,6 +1359,12 @@ def ffn_fp8(x: torch.Tensor, weights: Fp8FfnWeights, *, residual: torch.Tensor |
     per 1 x 128 block, and only GEMM 2 is e4m3.  Two of the four e4m3 roundings of the default mode (x and
     W_up, the two largest terms of its error) disappear: 3.5e-2 instead of 6.2e-2 relative to the bf16 FFN
     for the gated layer, for about 1.8 x the time."""
+    if _TIMING is None and not check and not (precise and weights.w_up_bf16 is None):
+        call = _host.ffn_fp8_precise if precise else _host.ffn_fp8
+        fast = call(x, weights.w_up_bf16 if precise else weights.w_up, weights.s_up, weights.b_up, weights.w_down, weights.s_down,
+                    weights.b_down, weights.hidden, weights.gated, residual, status)
+        if fast is not None:
+            return fast
     shape = x.shape
     x2 = x.reshape(-1, shape[-1])
     if precise:

@@ -1,0 +1,56 @@
+"""The host module's mask recognition (one kernel over the mask) against the tensor-arithmetic planner, at row widths around
+its 16-byte pieces, and the refusal of masks that neither recognises."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import gpu_ready
+from oracle import reference_ops as R
+from taac_2026_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _need_gpu():
+    if not gpu_ready():
+        pytest.fail("gpu tests need an sm_100 device and a built libtb200.so")
+
+
+def _qkv(batch, heads, length, seed):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(batch, heads, length, 64, generator=g).bfloat16().cuda() for _ in range(3))
+
+
+@pytest.mark.parametrize("length", [1, 2, 15, 16, 17, 33, 64, 130, 265])
+@pytest.mark.parametrize("form", ["key", "causal", "causal_ns", "full", "identity"])
+def test_recognised_masks_give_the_planned_attention(length, form):
+    batch, heads = 5, 2
+    q, k, v = _qkv(batch, heads, length, length)
+    ns = min(9, length - 1) if form == "causal_ns" else 0
+    g = torch.Generator().manual_seed(length + 1)
+    lens = torch.randint(0, length - ns + 1, (batch,), generator=g)
+    if form == "full":
+        lens[:] = length
+    if form == "identity":
+        lens[:] = 0
+    causal = form != "key"
+    mask = R.structured_attention_mask(lens, length, length - ns, causal, causal)[:, None].cuda()
+    for m in (mask.expand(-1, heads, -1, -1), mask.repeat(1, heads, 1, 1)):
+        plan = ops.plan_attention_mask(q, k, m, is_causal=False)
+        want = ops.varlen_attention(q, k, v, seq_len=plan.seq_len, ns_start=plan.ns_start, causal=plan.causal,
+                                    padded_query_self=plan.padded_query_self)
+        assert ops._host.flash_attention(q, k, v, m, False) is not None      # not left to the tensor-arithmetic planner
+        assert torch.equal(ops.flash_attention(q, k, v, attn_mask=m), want)
+
+
+@pytest.mark.parametrize("flip", [(0, 0, 20), (3, 40, 40), (1, 64, 2), (4, 30, 31)])
+def test_one_wrong_element_is_refused(flip):
+    batch, heads, length = 5, 2, 65
+    q, k, v = _qkv(batch, heads, length, 3)
+    mask = R.structured_attention_mask(torch.tensor([65, 50, 30, 41, 9]), length, length, True, True)[:, None].clone().cuda()
+    b, i, j = flip
+    mask[b, 0, i, j] ^= True
+    with pytest.raises(RuntimeError, match="cuda flash_attention"):
+        ops.flash_attention(q, k, v, attn_mask=mask.expand(-1, heads, -1, -1))

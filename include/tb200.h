@@ -439,12 +439,43 @@ int tb200_packed_token_index(const int64_t* values, const int64_t* timestamps, c
 int tb200_pyramid_plan(const int64_t* lengths, int32_t batch, int32_t max_len, const int32_t* widths, int32_t n_layers,
                        int32_t ns, int64_t* start, int64_t* n0, int64_t* counts, int64_t* cu, int32_t* cu32,
                        int64_t* meta, int64_t* ns_rows0, void* stream);
+/* The same with meta in memory that the host reads after synchronising (pinned host memory) where that saves a copy, and with
+ * the rows of the non-sequence tokens at every layer, token-major: ns_rows[l, j, b] = cu[l, b] + counts[l, b] + j (may be NULL). */
+int tb200_pyramid_plan_rows(const int64_t* lengths, int32_t batch, int32_t max_len, const int32_t* widths, int32_t n_layers,
+                            int32_t ns, int64_t* start, int64_t* n0, int64_t* counts, int64_t* cu, int32_t* cu32,
+                            int64_t* meta, int64_t* ns_rows0, int64_t* ns_rows, void* stream);
 
 /* Rows of layer l kept for layer l + 1, from two consecutive rows of the plan above (cu0 = cu[l], cu1 = cu[l + 1], ...):
  * src[cu1[b] + r] = cu0[b] + (counts0[b] - counts1[b]) + r;  ns_rows1[b, j] = cu1[b] + counts1[b] + j;  row_dst
  * (optional, int32 [rows of layer l]) = the destination of every row of layer l, -1 for the dropped ones. */
 int tb200_pyramid_kept_rows(const int64_t* cu0, const int64_t* cu1, const int64_t* counts0, const int64_t* counts1,
                             int32_t batch, int32_t ns, int64_t* src, int64_t* ns_rows1, int32_t* row_dst, void* stream);
+
+/* ---- row kernels around the engine's blocks ---------------------------------------------------
+ * out[r] = LayerNorm(SiLU(w x_r + bias)) gamma + beta in fp32, x_r = [values[r, :n], mask[r, :n] != 0 as 1 / 0 (mask may be NULL)]:
+ * `DenseTokenProjector.forward` (modeling/tokenizers.py:101-111) and the statistics projector.  w [d, in_dim] fp32 with in_dim = n or
+ * 2 n; out rows out_stride elements apart, of type dtype.  8 (in_dim + d) floats must fit 48 KB. */
+int tb200_small_token_fwd(const float* values, int32_t n, int64_t value_stride, const uint8_t* mask, int64_t mask_stride, int32_t in_dim,
+                          const float* w, const float* bias, const float* gamma, const float* beta, void* out, int64_t out_stride,
+                          int64_t rows, int32_t d, float eps, int dtype, void* stream);
+/* LayerNorm(SiLU(x)) (as tb200_layernorm_silu_fwd) with output rows y_stride elements apart; cols of at most 640 16-byte pieces. */
+int tb200_layernorm_silu_strided_fwd(const void* x, const void* gamma, const void* beta, void* y, int64_t rows, int32_t cols,
+                                     int64_t y_stride, float eps, int dtype, void* stream);
+/* ns_tokens [batch, ns, d]: row (b, j) goes to tokens[token_rows[j, b]], rmsnorm(row) gamma to normed[normed_rows[j, b]] and to
+ * token_major[j, b] (row ids [ns, batch], token_major [ns, batch, d]). */
+int tb200_ns_rows_fwd(const void* ns_tokens, int64_t batch, int32_t ns, int32_t d, const void* gamma, float eps, const int64_t* token_rows,
+                      void* tokens, const int64_t* normed_rows, void* normed, void* token_major, int dtype, void* stream);
+/* Means of rmsnorm(row) gamma (the final norm and the masked means of experiments/onetrans/model.py:349-356) in fp32: over the
+ * counts[b] sequence rows from cu[b] on -> seq_mean [batch, d] (0 for none) and over the ns rows behind them -> ns_mean [batch, d].
+ * cu == NULL: rows are token-major [ns, batch, d], no sequence rows. */
+int tb200_pool_rows_fwd(const void* rows, const int64_t* cu, const int64_t* counts, int64_t batch, int32_t ns, int32_t d, const void* gamma,
+                        float eps, float* seq_mean, float* ns_mean, int dtype, void* stream);
+/* joined [batch, 2 d] fp32 = [seq (NULL: zeros), ns]; joined_cast (may be NULL): the same as dtype. */
+int tb200_join_summaries(const float* seq, const float* ns, float* joined, void* joined_cast, int64_t batch, int32_t d, int dtype,
+                         void* stream);
+/* logits = h w^T + bias, probs = sigmoid(logits); h [batch, d] of dtype, the rest fp32 (w [actions, d]). */
+int tb200_head_fwd(const void* h, const float* w, const float* bias, float* logits, float* probs, int64_t batch, int32_t d, int32_t actions,
+                   int dtype, void* stream);
 
 /* ---- per-token (grouped) bf16 linear layers with a fused epilogue ----------------------------
  * out[g] = act(a[g] @ w[g]^T + bias[g]) (+ residual[g]) for g in [0, groups): the token-specific projections

@@ -49,6 +49,12 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_bias_act_rows": (_INT, [_P, _I64, _I32, _P, _I64, _I32, _INT, _P]),
     "tb200_bag_mean_fwd": (_INT, [_P, _I64, _I32, _P, _INT, _I64, _I32, _P, _INT, _P]),
     "tb200_bag_mean_bwd": (_INT, [_P, _INT, _P, _P, _P, _I64, _I32, _I32, _I64, _INT, _P]),
+    "tb200_small_token_fwd": (_INT, [_P, _I32, _I64, _P, _I64, _I32, _P, _P, _P, _P, _P, _I64, _I64, _I32, _F, _INT, _P]),
+    "tb200_layernorm_silu_strided_fwd": (_INT, [_P, _P, _P, _P, _I64, _I32, _I64, _F, _INT, _P]),
+    "tb200_ns_rows_fwd": (_INT, [_P, _I64, _I32, _I32, _P, _F, _P, _P, _P, _P, _P, _INT, _P]),
+    "tb200_pool_rows_fwd": (_INT, [_P, _P, _P, _I64, _I32, _I32, _P, _F, _P, _P, _INT, _P]),
+    "tb200_join_summaries": (_INT, [_P, _P, _P, _P, _I64, _I32, _INT, _P]),
+    "tb200_head_fwd": (_INT, [_P, _P, _P, _P, _P, _I64, _I32, _I32, _INT, _P]),
     "tb200_mask_plan": (_INT, [_P, _I64, _I64, _I64, _I32, _I32, _I32, _I32, _P, _P, _P]),
     "tb200_attn_bwd_workspace_bytes": (_I64, [_I32, _I32, _I32]),
     "tb200_attn_bwd": (_INT, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I32, _I32, _I32, _I32, _I32, _P, _P, _P, _I32, _I32, _I32,
@@ -57,6 +63,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_quant_act_mx": (_INT, [_P, _P, _P, _I64, _I32, _P]),
     "tb200_mx_gemm": (_INT, [_P, _P, _P, _P, _P, _P, _P, _P, _I64, _I32, _I32, _I32, _P, _P]),
     "tb200_pyramid_plan": (_INT, [_P, _I32, _I32, _P, _I32, _I32, _P, _P, _P, _P, _P, _P, _P, _P]),
+    "tb200_pyramid_plan_rows": (_INT, [_P, _I32, _I32, _P, _I32, _I32, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "tb200_pyramid_kept_rows": (_INT, [_P, _P, _P, _P, _I32, _I32, _P, _P, _P, _P]),
     "tb200_host_compact_offsets": (_INT, [_P, _I32, _I32, _P]),
     "tb200_host_compact_sequence": (_INT, [_P, _P, _P, _P, _I32, _I32, _I32, _P, _I64, _P, _I32]),

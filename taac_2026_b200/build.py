@@ -84,7 +84,7 @@ def _compile_host(src: Path, verbose: bool) -> Path:
         return obj
     cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
     paths = [*include_paths(), sysconfig.get_paths()["include"], str(cuda_include)]
-    _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+    _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native",
           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{p}" for p in paths), "-c", str(src), "-o", str(obj)],
          f"host compiler for {src.name}", verbose)
     return obj

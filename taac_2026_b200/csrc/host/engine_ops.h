@@ -1,0 +1,148 @@
+// The engine's launches: each function allocates its result, enqueues the library's kernel on the current stream and, while
+// kernel timing is on, brackets the launch with the timing records of the Python operators (same names and fields).
+#pragma once
+#include <ATen/cuda/EmptyTensor.h>
+#include <pybind11/stl.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <cmath>
+
+#include "native.h"
+
+namespace tb200_host {
+namespace py = pybind11;
+using namespace pybind11::literals;
+using OptTensor = std::optional<Tensor>;
+
+// Timing is switched per forward; the records belong to the list installed with `ops.set_kernel_timing`.
+struct Timing {
+    static bool& on() {
+        static thread_local bool flag = false;
+        return flag;
+    }
+};
+class Timed {
+public:
+    Timed(const char* name, const py::dict& meta) : scope_(py::module_::import("taac_2026_b200.ops").attr("timed")(name, **meta)) {
+        scope_.attr("__enter__")();
+    }
+    ~Timed() { scope_.attr("__exit__")(py::none(), py::none(), py::none()); }
+
+private:
+    py::object scope_;
+};
+#define TB200_TIMED(name, ...)   \
+    std::optional<Timed> timed_; \
+    if (Timing::on()) timed_.emplace(name, py::dict(__VA_ARGS__))
+
+inline Tensor make(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
+    return at::detail::empty_cuda(sizes, type, device, std::nullopt);
+}
+inline Tensor make_like(at::IntArrayRef sizes, const Tensor& t) { return make(sizes, t.scalar_type(), t.device()); }
+
+template <typename P>
+P* data(const Tensor& t) { return static_cast<P*>(t.data_ptr()); }
+template <typename P>
+P* data(const OptTensor& t) { return t.has_value() ? static_cast<P*>(t->data_ptr()) : nullptr; }
+
+inline Tensor gather_rows(const Tensor& table, const Tensor& ids) {   // table [V, d], ids int64 [n]
+    const int64_t n = ids.numel(), dim = table.size(1);
+    Tensor out = make_like({n, dim}, table);
+    TB200_TIMED("gather_rows", "ids"_a = ids, "dim"_a = dim, "esize"_a = table.element_size());
+    check(tb200_gather_rows(ptr(table), table.size(0), static_cast<int32_t>(dim), ptr(ids), TB200_I64, n, std::max<int64_t>(n, 1), 0, ptr(out), dim, 0,
+                            dtype_code(table.scalar_type()), stream_of(table)), "cuda gather_rows");
+    return out;
+}
+inline void gather_rows_into(const Tensor& table, const int64_t* ids, const Tensor& ids_meta, const Tensor& out, int64_t col0) {
+    const int64_t n = out.size(0), dim = table.size(1);
+    TB200_TIMED("gather_rows", "ids"_a = ids_meta, "dim"_a = dim, "esize"_a = table.element_size());
+    check(tb200_gather_rows(ptr(table), table.size(0), static_cast<int32_t>(dim), ids, TB200_I64, n, std::max<int64_t>(n, 1), 0, ptr(out), out.size(1),
+                            static_cast<int32_t>(col0), dtype_code(table.scalar_type()), stream_of(table)), "cuda gather_rows");
+}
+// dst[ids[i], col0 ..] = src[i] (+ bias[i / rows per bias row]) (+ residual[ids[i]])
+inline void scatter_rows(const Tensor& dst, const Tensor& ids, const Tensor& src, const OptTensor& bias = std::nullopt,
+                         const OptTensor& residual = std::nullopt) {
+    const int64_t n = ids.numel(), dim = src.numel() / std::max<int64_t>(n, 1);
+    const int64_t per_group = bias.has_value() ? std::max<int64_t>(n / (bias->numel() / dim), 1) : 1;
+    TB200_TIMED("scatter_rows", "rows"_a = n, "dim"_a = dim, "esize"_a = dst.element_size());
+    check(tb200_scatter_rows(ptr(dst), dst.size(0), dst.size(1), 0, data<int64_t>(ids), ptr(src), n, static_cast<int32_t>(dim), ptr(bias), per_group,
+                             ptr(residual), residual.has_value() ? residual->size(1) : 0, dtype_code(dst.scalar_type()), stream_of(dst)),
+          "cuda scatter_rows");
+}
+inline Tensor rms_norm(const Tensor& x, const Tensor& w, const OptTensor& in_bias = std::nullopt) {   // [rows, d], eps 1e-6
+    const auto cols = static_cast<int32_t>(x.size(-1));
+    const int64_t rows = x.numel() / cols;
+    Tensor out = make_like(x.sizes(), x);
+    const int dt = dtype_code(x.scalar_type());
+    TB200_TIMED("rms_norm", "rows"_a = rows, "cols"_a = cols, "esize"_a = x.element_size());
+    check(in_bias.has_value() ? tb200_rmsnorm_bias_fwd(ptr(x), ptr(*in_bias), ptr(w), ptr(out), rows, cols, 1e-6f, dt, stream_of(x))
+                              : tb200_rmsnorm_fwd(ptr(x), ptr(w), ptr(out), rows, cols, 1e-6f, dt, stream_of(x)), "cuda rms_norm");
+    return out;
+}
+inline Tensor layer_norm(const Tensor& x, const Tensor& w, const Tensor& b, bool pre_silu) {
+    const auto cols = static_cast<int32_t>(x.size(-1));
+    const int64_t rows = x.numel() / cols;
+    Tensor out = make_like(x.sizes(), x);
+    const int dt = dtype_code(x.scalar_type());
+    TB200_TIMED("layer_norm", "rows"_a = rows, "cols"_a = cols, "esize"_a = x.element_size());
+    check(pre_silu ? tb200_layernorm_silu_fwd(ptr(x), ptr(w), ptr(b), ptr(out), rows, cols, 1e-5f, dt, stream_of(x))
+                   : tb200_layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(out), rows, cols, 1e-5f, dt, stream_of(x)), "cuda layer_norm");
+    return out;
+}
+
+// One layer: weight [N, K] ([G, N, K] grouped) in the compute type, bias in fp32 for this library's GEMM and in the compute
+// type for the library's
+struct Layer {
+    Tensor w;
+    OptTensor b32, b;
+};
+
+// out[g] = act(x[g] w[g]^T + b[g]) (+ residual[g]); x [G, M, K] or [M, K]; `out` may be the residual
+inline Tensor grouped(const Tensor& x, const Tensor& w, const OptTensor& b32, bool silu, const OptTensor& residual, const OptTensor& out_in,
+                      const Tensor& status) {
+    const int64_t k = x.size(-1), m = x.size(-2), g = x.dim() == 3 ? x.size(0) : 1, n = w.size(-2);
+    Tensor out = out_in.has_value() ? *out_in : (x.dim() == 3 ? make_like({g, m, n}, x) : make_like({m, n}, x));
+    TB200_TIMED("gemm_bf16", "groups"_a = g, "m"_a = m, "n"_a = n, "k"_a = k, "silu"_a = silu, "residual"_a = residual.has_value());
+    check(tb200_gemm_bf16_grouped(ptr(x), ptr(w), data<float>(b32), ptr(residual), ptr(out), static_cast<int32_t>(g), m, static_cast<int32_t>(n),
+                                  static_cast<int32_t>(k), silu ? 1 : 0, data<int32_t>(status), stream_of(x)), "cuda grouped_linear");
+    return out;
+}
+
+// x = act(x + bias[group]) in place, act = SiLU or identity; x [groups, rows, cols]
+inline Tensor bias_act_rows(const Tensor& x, const Tensor& bias, bool silu) {
+    const int64_t cols = x.size(-1), rows = x.numel() / cols, groups = bias.numel() / cols;
+    TB200_TIMED("bias_act_rows", "rows"_a = rows, "cols"_a = cols, "esize"_a = x.element_size());
+    check(tb200_bias_act_rows(ptr(x), rows, static_cast<int32_t>(cols), ptr(bias), std::max<int64_t>(rows / groups, 1), silu ? 1 : 0,
+                              dtype_code(x.scalar_type()), stream_of(x)), "cuda bias_act_rows");
+    return x;
+}
+
+// Packed attention: q, k, v strided [rows, H, D] views, sample b owns rows [cu[b], cu[b + 1]); with cu_q the queries are the last
+// cu_q[b + 1] - cu_q[b] rows of the sample.  Causal.
+inline Tensor packed_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu, int64_t max_rows, const OptTensor& cu_q,
+                               int64_t max_rows_q, int kernel, const Tensor& status) {
+    Tensor out = make_like(q.sizes(), q);
+    int64_t s[12];
+    int i = 0;
+    for (const Tensor* t : {&q, &k, &v, static_cast<const Tensor*>(&out)}) {
+        s[i++] = 0;
+        s[i++] = t->stride(1);
+        s[i++] = t->stride(0);
+    }
+    const auto b = static_cast<int32_t>(cu.size(0) - 1), h = static_cast<int32_t>(q.size(1)), d = static_cast<int32_t>(q.size(2));
+    const int64_t lq = cu_q.has_value() ? max_rows_q : max_rows;
+    const bool small = lq <= 32 && max_rows <= 32 && d == 64;
+    const char* name = small ? "attention_small"
+                       : cu_q.has_value() ? (d == 64 ? "attention_fewq" : "attention_mma")
+                                          : (d == 64 && q.scalar_type() == at::kBFloat16 && lq >= 128 ? "attention_tc05" : "attention_mma");
+    TB200_TIMED(name, "seq_len"_a = py::none(), "cu_rows"_a = cu, "cu_rows_q"_a = cu_q, "key_valid"_a = py::none(), "batch"_a = b, "heads"_a = h,
+                "lq"_a = lq, "lk"_a = max_rows, "dim"_a = d, "ns_start"_a = max_rows, "causal"_a = true, "self_rows"_a = false,
+                "esize"_a = q.element_size());
+    check(tb200_attn_fwd(ptr(q), ptr(k), ptr(v), ptr(out), b, h, static_cast<int32_t>(lq), static_cast<int32_t>(max_rows), d, s, nullptr,
+                         data<int32_t>(cu), data<int32_t>(cu_q), nullptr, static_cast<int32_t>(max_rows), 1, 0,
+                         static_cast<float>(1.0 / std::sqrt(static_cast<double>(d))), dtype_code(q.scalar_type()), kernel, k.size(0),
+                         data<int32_t>(status), stream_of(q)), "cuda varlen_attention");
+    return out;
+}
+
+}  // namespace tb200_host

@@ -1,6 +1,7 @@
 // Shared declarations of the host module: C-ABI calls on torch tensors (allocation, current stream, status checks).
 #pragma once
 #include <ATen/ATen.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -31,7 +32,7 @@ inline void* ptr(const std::optional<Tensor>& t) { return t.has_value() ? t->dat
 inline bool dense(const Tensor& t, at::ScalarType type) {
     return t.defined() && t.is_cuda() && t.scalar_type() == type && t.is_contiguous();
 }
-inline bool wants_grad(const Tensor& t) { return t.requires_grad() && at::GradMode::is_enabled(); }
+inline bool wants_grad(const Tensor& t) { return t.requires_grad() && c10::GradMode::is_enabled(); }
 
 inline void check(int code, const char* what) {
     TORCH_CHECK(code == 0, what, ": ", tb200_strerror(code), " (status ", code, ")");

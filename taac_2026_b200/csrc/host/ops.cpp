@@ -10,6 +10,7 @@
 #include <cmath>
 #include <limits>
 
+#include "module.h"
 #include "native.h"
 
 namespace tb200_host {
@@ -532,4 +533,10 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Host side of the operat
 }  // namespace
 }  // namespace tb200_host
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&tb200_host::module); }
+PyMODINIT_FUNC PyInit__native() {
+    HANDLE_TH_ERRORS
+    PyObject* m = PyModule_Create(&tb200_host::module);
+    if (m != nullptr) tb200_host::bind_engine(m);
+    return m;
+    END_HANDLE_TH_ERRORS
+}

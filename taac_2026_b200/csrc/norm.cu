@@ -453,7 +453,7 @@ norm_rowwarp_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const 
 template <typename T, bool LAYER, int PRE>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_rowwarp_vec_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
-                        T* __restrict__ y, int64_t rows, int cols, float eps) {
+                        T* __restrict__ y, int64_t rows, int cols, int64_t y_stride, float eps) {
     constexpr int N = Vec16<T>::N;
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
@@ -467,7 +467,7 @@ norm_rowwarp_vec_kernel(const T* __restrict__ x, const T* __restrict__ gamma, co
     const uint4* b4 = reinterpret_cast<const uint4*>(beta);
     for (int64_t row = warp; row < rows; row += n_warps) {
         const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
-        uint4* yr = reinterpret_cast<uint4*>(y + row * cols);
+        uint4* yr = reinterpret_cast<uint4*>(y + row * y_stride);
         float acc = 0.f;   // LayerNorm: sum of the row; RMSNorm: sum of squares
         for (int c = lane; c < chunks; c += 32) {
             uint4 p = ld_nc_u4(xr + c);
@@ -568,6 +568,26 @@ int launch_tma(const void* x, const void* gamma, const void* beta, void* y, int6
     return launch_tma_exact<T, LAYER, CPL, RU, PRE, POST, false>(x, gamma, beta, y, rows, cols, eps, lanes_per_row, stream, post);
 }
 
+// rows of up to 640 pieces: up to 10 KB of row per warp, 80 KB per block
+template <typename T, bool LAYER, int PRE>
+int launch_rowwarp_vec(const void* x, const void* gamma, const void* beta, void* y, int64_t rows, int cols, int64_t y_stride, float eps,
+                       cudaStream_t stream) {
+    const DeviceInfo& dev = device_info();
+    const size_t smem = static_cast<size_t>(kMaxThreads / 32) * (cols / Vec16<T>::N) * 16;
+    static bool attr_set[64] = {};
+    if (!attr_set[dev.index]) {
+        cudaFuncSetAttribute(norm_rowwarp_vec_kernel<T, LAYER, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+        attr_set[dev.index] = true;
+    }
+    int64_t blocks = (rows + (kMaxThreads / 32) - 1) / (kMaxThreads / 32);
+    const int64_t cap = static_cast<int64_t>(dev.sm_count) * (smem > 56 * 1024 ? 2 : (smem > 36 * 1024 ? 4 : 6));
+    if (blocks > cap) blocks = cap;
+    norm_rowwarp_vec_kernel<T, LAYER, PRE><<<static_cast<unsigned>(blocks), kMaxThreads, smem, stream>>>(
+        static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows, cols, y_stride, eps);
+    count_launch();
+    return launch_status();
+}
+
 template <typename T, bool LAYER, int PRE>
 int norm_dispatch(const void* x, const void* gamma, const void* beta, void* y, int64_t rows, int cols, float eps,
                   cudaStream_t stream) {
@@ -592,20 +612,7 @@ int norm_dispatch(const void* x, const void* gamma, const void* beta, void* y, i
     if (blocks < 1) blocks = 1;
     const bool wide_vec = (cols % N == 0) && aligned16(x) && aligned16(y) && aligned16(gamma) &&
                           ((!LAYER && PRE != kPreBias) || aligned16(beta)) && (cols / N) <= 640;
-    if (wide_vec) {   // up to 10 KB of row per warp, 80 KB per block
-        const size_t smem = static_cast<size_t>(kMaxThreads / 32) * (cols / N) * 16;
-        static bool attr_set[64] = {};
-        if (!attr_set[dev.index]) {
-            cudaFuncSetAttribute(norm_rowwarp_vec_kernel<T, LAYER, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-            attr_set[dev.index] = true;
-        }
-        const int64_t cap_vec = static_cast<int64_t>(dev.sm_count) * (smem > 56 * 1024 ? 2 : (smem > 36 * 1024 ? 4 : 6));
-        if (blocks > cap_vec) blocks = cap_vec;
-        norm_rowwarp_vec_kernel<T, LAYER, PRE><<<static_cast<unsigned>(blocks), kMaxThreads, smem, stream>>>(
-            static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows, cols, eps);
-        count_launch();
-        return launch_status();
-    }
+    if (wide_vec) return launch_rowwarp_vec<T, LAYER, PRE>(x, gamma, beta, y, rows, cols, cols, eps, stream);
     norm_rowwarp_kernel<T, LAYER, PRE><<<static_cast<unsigned>(blocks), kMaxThreads, 0, stream>>>(
         static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows,
         cols, eps);
@@ -703,4 +710,26 @@ extern "C" int tb200_token_tail_fwd(const void* x, const void* ln_gamma, const v
                                     int64_t rows, int32_t cols, float ln_eps, float rms_eps, int dtype, void* stream) {
     return tb200_token_tail_select_fwd(x, ln_gamma, ln_beta, table_a, rows_a, ids_a, table_b, rows_b, ids_b, rms_gamma,
                                        nullptr, 0, tokens, normed, rows, cols, ln_eps, rms_eps, dtype, stream);
+}
+
+// LayerNorm(SiLU(x)) whose output rows lie y_stride elements apart
+extern "C" int tb200_layernorm_silu_strided_fwd(const void* x, const void* gamma, const void* beta, void* y, int64_t rows, int32_t cols,
+                                                int64_t y_stride, float eps, int dtype, void* stream) {
+    using namespace tb200;
+    if (rows < 0 || cols < 1 || y_stride < cols) return TB200_ERR_SHAPE;
+    if (rows == 0) return TB200_OK;
+    const int es = dtype_size(dtype);
+    if (es == 0) return TB200_ERR_DTYPE;
+    if (x == nullptr || gamma == nullptr || beta == nullptr || y == nullptr) return TB200_ERR_NULL;
+    if ((static_cast<int64_t>(cols) * es) % 16 != 0 || (y_stride * es) % 16 != 0 || !aligned16(x) || !aligned16(gamma) || !aligned16(beta) ||
+        !aligned16(y))
+        return TB200_ERR_ALIGN;
+    if (static_cast<int64_t>(cols) * es > 640 * 16) return TB200_ERR_UNSUPPORTED;
+    if (!device_info().valid) return TB200_ERR_DEVICE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    switch (dtype) {
+        case TB200_F32: return launch_rowwarp_vec<float, true, kPreSilu>(x, gamma, beta, y, rows, cols, y_stride, eps, s);
+        case TB200_F16: return launch_rowwarp_vec<__half, true, kPreSilu>(x, gamma, beta, y, rows, cols, y_stride, eps, s);
+        default: return launch_rowwarp_vec<__nv_bfloat16, true, kPreSilu>(x, gamma, beta, y, rows, cols, y_stride, eps, s);
+    }
 }

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kPlanThreads)
 pyramid_plan_kernel(const int64_t* __restrict__ lengths, int batch, int max_len, PlanWidths widths, int ns,
                     int64_t* __restrict__ start, int64_t* __restrict__ n0_out, int64_t* __restrict__ counts,
                     int64_t* __restrict__ cu, int32_t* __restrict__ cu32, int64_t* __restrict__ meta,
-                    int64_t* __restrict__ ns_rows0) {
+                    int64_t* __restrict__ ns_rows0, int64_t* __restrict__ ns_rows) {
     __shared__ int64_t warp_sum[32];
     __shared__ int64_t warp_max[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -286,6 +286,8 @@ pyramid_plan_kernel(const int64_t* __restrict__ lengths, int batch, int max_len,
             cu32_l[b] = static_cast<int32_t>(first_row);
             if (l == 0)
                 for (int j = 0; j < ns; ++j) ns_rows0[static_cast<int64_t>(b) * ns + j] = first_row + c + j;
+            if (ns_rows != nullptr)
+                for (int j = 0; j < ns; ++j) ns_rows[(static_cast<int64_t>(l) * ns + j) * batch + b] = first_row + c + j;
         }
         running += tile_total;
         __syncthreads();                                    // warp_sum is rewritten by the next tile
@@ -331,6 +333,12 @@ pyramid_kept_rows_kernel(const int64_t* __restrict__ cu0, const int64_t* __restr
 extern "C" int tb200_pyramid_plan(const int64_t* lengths, int32_t batch, int32_t max_len, const int32_t* widths,
                                   int32_t n_layers, int32_t ns, int64_t* start, int64_t* n0, int64_t* counts, int64_t* cu,
                                   int32_t* cu32, int64_t* meta, int64_t* ns_rows0, void* stream) {
+    return tb200_pyramid_plan_rows(lengths, batch, max_len, widths, n_layers, ns, start, n0, counts, cu, cu32, meta, ns_rows0, nullptr, stream);
+}
+
+extern "C" int tb200_pyramid_plan_rows(const int64_t* lengths, int32_t batch, int32_t max_len, const int32_t* widths,
+                                       int32_t n_layers, int32_t ns, int64_t* start, int64_t* n0, int64_t* counts, int64_t* cu,
+                                       int32_t* cu32, int64_t* meta, int64_t* ns_rows0, int64_t* ns_rows, void* stream) {
     using namespace tb200;
     if (batch < 0 || max_len < 0 || n_layers < 0 || n_layers > kPlanMaxLayers || ns < 0) return TB200_ERR_SHAPE;
     if (widths == nullptr || start == nullptr || n0 == nullptr || counts == nullptr || cu == nullptr || cu32 == nullptr ||
@@ -345,7 +353,7 @@ extern "C" int tb200_pyramid_plan(const int64_t* lengths, int32_t batch, int32_t
     if ((static_cast<int64_t>(widths[0]) + ns) * batch > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
     pyramid_plan_kernel<<<static_cast<unsigned>(n_layers + 1), kPlanThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        lengths, batch, max_len, w, ns, start, n0, counts, cu, cu32, meta, ns_rows0);
+        lengths, batch, max_len, w, ns, start, n0, counts, cu, cu32, meta, ns_rows0, ns_rows);
     count_launch();
     return launch_status();
 }

@@ -30,7 +30,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
-from taac_2026_b200 import ops
+from taac_2026_b200 import _lib, ops
 from taac_2026_b200.inputs import OneTransSpec
 
 # Gap-time bucket edges in seconds (the constant table of modeling/time_features.py:16-28).
@@ -201,9 +201,10 @@ class OneTransInference:
         # sequence tokenizer as ONE kernel (`ops.token_project`) instead of the row gather, the projection GEMM and the
         # fused tail.  Off by default: measured on 1 M rows the one-kernel form takes 1.27 ms against 0.79 ms.
         self.fused_tokenizer = bool(fused_tokenizer)
-        self._meta_ring: list[torch.Tensor] = []
         self._copy_stream: torch.cuda.Stream | None = None
-        self._meta_next = 0
+        self._native = None
+        self._schedules: dict[int, list[int]] = {}
+        self._esize = torch.empty(0, dtype=dtype).element_size()
         if ffn not in ("bf16", "fp8", "fp8_precise", "fp8_mx"):
             raise ValueError(f"unknown ffn mode {ffn}")
         # "fp8_mx": power-of-two block scales applied inside the block-scaled tensor-core instruction (ops.ffn_mx)
@@ -259,7 +260,6 @@ class OneTransInference:
         # a kernel whose bounded wait gives up raises it.  Passing it costs nothing per call; it is read back by
         # `raise_if_incomplete` (one small device-to-host copy), which `score_stream` calls for the caller.
         self.status_word = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._hash_buckets: dict[str, torch.Tensor] = {}   # per sequence domain: how each feature's ids are hashed
 
     # ------------------------------------------------------------------ weights
     def _p(self, name: str) -> torch.Tensor:
@@ -305,7 +305,7 @@ class OneTransInference:
         self.blocks = []
         for layer in range(self.n_blocks):
             p = f"blocks.{layer}"
-            blk = {"p": p}
+            blk = {"p": p, "attn_norm": self._p(p + ".attn_norm.weight"), "ffn_norm": self._p(p + ".ffn_norm.weight")}
             if self.ffn_mode == "fp8":
                 if self.ffn_mx:
                     blk["ffn_fp8"] = ops.MxFfnWeights(
@@ -321,6 +321,10 @@ class OneTransInference:
                 folded = copy.copy(blk["ffn_fp8"])
                 folded.b_down = (folded.b_down + self.w[p + ".attention.out.bias"].float()).contiguous()
                 blk["ffn_fp8_folded"] = folded
+            else:
+                for i, layer_name in ((1, ".ffn.shared.net.0"), (2, ".ffn.shared.net.3")):
+                    blk[f"ffn_w{i}"] = self._p(p + layer_name + ".weight")
+                    blk[f"ffn_b{i}"] = self.w[p + layer_name + ".bias"].float().contiguous()
             blk["out_w_t"] = self._p(p + ".attention.out.weight").t()
             blk["out_b"] = self._p(p + ".attention.out.bias")
             # shared projections as `nn.Linear` weights ([out, in], contiguous row blocks) with fp32 biases: what the
@@ -583,51 +587,112 @@ class OneTransInference:
         return logits, embeddings
 
     @torch.inference_mode()
-    def predict(self, inputs, prepared: dict | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+    def predict(self, inputs, prepared=None) -> tuple[torch.Tensor, torch.Tensor]:
         """(logits [B, action_num], pooled embeddings [B, 2 d]) in fp32 — `PCVROneTrans.predict`.  ``prepared`` is
         what ``prepare(inputs)`` returned for these inputs (the serving loop computes it ahead of time)."""
         if self.packed and len(self.domains) == 1:
-            return self._predict_packed(inputs, prepared)
+            return self._predict_packed(inputs, prepared)[:2]
         return self._predict_padded(inputs)
 
     @torch.inference_mode()
-    def prepare(self, inputs) -> dict | None:
+    def prepare(self, inputs):
         """Everything of a forward that the host has to wait for, enqueued on the current stream: duplicate removal
-        and statistics of the behaviour sequence, the row plan of the packed layout, and the asynchronous copy of the
-        plan's per-layer totals into pinned host memory (with an event).  A serving loop calls this for batch i + 1 on
-        a side stream while batch i is being scored; the forward of batch i + 1 then finds its buffer sizes on the
-        host already and never drains the device.  None when the engine does not run the packed layout.  At most
-        three results may be outstanding at a time: the pinned landing buffers are a ring of four."""
+        and statistics of the behaviour sequence and the row plan of the packed layout, whose per-layer totals the
+        kernel writes into pinned host memory.  A serving loop calls this for batch i + 1 on a side stream while batch
+        i is being scored; the forward of batch i + 1 then finds its buffer sizes on the host already and never drains
+        the device.  None when the engine does not run the packed layout.  At most three results may be outstanding
+        at a time: the pinned landing buffers are a ring of four."""
         if not (self.packed and len(self.domains) == 1):
             return None
         seq = inputs.sequences[self.domains[0]]
-        ns = self.num_ns
-        lengths, src_map, stats = ops.sequence_prepare(seq.values, seq.lengths, seq.timestamps, inputs.request_timestamp)
-        max_len = seq.values.shape[2]
+        return self._executor().prepare(seq.values, seq.lengths, seq.timestamps, inputs.request_timestamp,
+                                        self._schedule(seq.values.shape[2]), ops.kernel_timing_on())
+
+    def _schedule(self, max_len: int) -> list[int]:
+        """Static schedule of padded sequence widths (layer 0 .. end) for inputs of ``max_len`` positions."""
         width = min(max_len, self.seq_keep)            # padded sequence width S[0] after the tail crop
-        widths = [width]                               # static schedule of padded widths
-        for layer in range(self.n_blocks):
-            widths.append(pyramid_keep_count(widths[-1], layer, self.n_blocks, ns))
-        plan = ops.pyramid_plan(lengths.to(torch.long), max_len, widths, ns)
-        # pinned landing buffers are kept in a small ring: allocating pinned memory per batch can stall on the device
-        # when the host runs a batch ahead (a buffer comes round again four batches later, long after its forward
-        # has read it)
-        ring = self._meta_ring
-        if not ring or ring[0].shape != plan["meta"].shape:
-            ring[:] = [torch.empty(plan["meta"].shape, dtype=torch.int64, pin_memory=True) for _ in range(4)]
-        meta_host = ring[self._meta_next % len(ring)]
-        self._meta_next += 1
-        meta_host.copy_(plan["meta"], non_blocking=True)
-        ready = torch.cuda.Event()
-        ready.record(torch.cuda.current_stream(self.device))
-        return {"src_map": src_map, "stats": stats, "plan": plan, "widths": widths, "meta_host": meta_host, "ready": ready,
-                "batch": int(lengths.shape[0])}
+        widths = self._schedules.get(width)
+        if widths is None:
+            widths = [width]
+            for layer in range(self.n_blocks):
+                widths.append(pyramid_keep_count(widths[-1], layer, self.n_blocks, self.num_ns))
+            self._schedules[width] = widths
+        return widths
 
     @staticmethod
-    def prepared_tensors(prepared: dict) -> list[torch.Tensor]:
+    def prepared_tensors(prepared) -> list[torch.Tensor]:
         """Device tensors of a ``prepare`` result (for ``Tensor.record_stream`` when it was made on another stream)."""
-        plan = prepared["plan"]
-        return [prepared["src_map"], prepared["stats"], plan["start"], plan["cu32"]]   # plan's int64 outputs share one allocation
+        return prepared.tensors()
+
+    def _small_token(self, linear: str, norm: str) -> dict:
+        """Linear -> SiLU -> LayerNorm of a handful of fp32 inputs, kept in fp32."""
+        f32 = lambda name: self.w[name].float().contiguous()  # noqa: E731
+        return {"w": f32(linear + ".weight"), "b": f32(linear + ".bias"), "gamma": f32(norm + ".weight"), "beta": f32(norm + ".bias")}
+
+    def _entity_tokens(self, prefix: str, bank: _Bank, n_tokens: int, groups) -> dict | None:
+        """What the executor needs to build an entity's tokens itself: one projection of all pooled fields.  None for the other
+        forms (hashed ids, tokens per group, no fields), which `_ns_tokens` builds."""
+        n_groups = len(list(groups)) or bank.n_fields
+        if bank.fields is None or bank.hashed or bank.fields.max_bag < 1 or n_tokens <= 0 \
+                or not (self.spec.force_auto_split or n_tokens != n_groups) or n_tokens * self.d * self._esize > 640 * 16:
+            return None
+        key = prefix + ".missing_embeddings"
+        f = bank.fields
+        return {"ptrs": f.ptrs, "rows": f.rows, "offsets": f.offsets, "lengths": f.lengths, "n_fields": f.n_fields, "max_bag": f.max_bag,
+                "dim": f.dim, "n_tokens": n_tokens, "missing_rows": self._p(key)[: f.n_fields].contiguous() if key in self.w else None,
+                "w": self._p(prefix + ".project.0.weight"), "b32": self.w[prefix + ".project.0.bias"].float().contiguous(),
+                "gamma": self._p(prefix + ".project.2.weight"), "beta": self._p(prefix + ".project.2.bias")}
+
+    def _executor(self):
+        """The native executor of the packed layout (built on first use; it shares this engine's weights)."""
+        if self._native is not None:
+            return self._native
+        spec = self.spec
+        domain = self.domains[0]
+        prefix = f"sequence_tokenizers.{domain}"
+        entries = self.seq_tables[domain]
+        buckets = torch.tensor([-1 if table is None else (table.shape[0] - 1 if kind == "compressed" else 0) for kind, table in entries],
+                               dtype=torch.long, device=self.device)
+        time_key = prefix + ".time_embedding.weight"
+        user = self._entity_tokens("user_tokenizer", self.user_bank, self.user_tokens, spec.user_ns_groups)
+        item = self._entity_tokens("item_tokenizer", self.item_bank, self.item_tokens, spec.item_ns_groups)
+        dense = {name: self._small_token(name + ".project.0", name + ".project.2") if dim > 0 else None
+                 for name, dim in (("user_dense", spec.user_dense_dim), ("item_dense", spec.item_dense_dim))}
+        fits = all(t is None or 8 * (t["w"].shape[1] + self.d) * 4 <= 48 * 1024 for t in dense.values())
+        modes = {"bf16": 0, "fp8": 2 if self.ffn_precise else (3 if self.ffn_mx else 1)}
+        config = {
+            "d": self.d, "heads": self.heads, "ns": self.num_ns, "emb": spec.emb_dim, "ffn": modes[self.ffn_mode], "status": self.status_word,
+            "edges": self._edges, "final_norm": self._p("final_norm.weight"),
+            "head_w": self.w["classifier.3.weight"].float().contiguous(), "head_b": self.w["classifier.3.bias"].float().contiguous(),
+            "classifier_w": self._p("classifier.0.weight"), "classifier_b": self.w["classifier.0.bias"].float().contiguous(),
+            "classifier_w32": None if self._own_gemm(self.d, 2 * self.d) else self.w["classifier.0.weight"].float().contiguous(),
+            "project_w": self._p(prefix + ".project.0.weight"), "project_b": self.w[prefix + ".project.0.bias"].float().contiguous(),
+            "ln_w": self._p(prefix + ".project.2.weight"), "ln_b": self._p(prefix + ".project.2.bias"),
+            "time_table": self._p(time_key) if time_key in self.w else None, "hash_buckets": buckets,
+            "seq_tables": [table for _kind, table in entries], "stats": self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2"),
+        }
+        if user is not None and item is not None and fits:
+            config.update(user=user, item=item, user_dense=dense["user_dense"], item_dense=dense["item_dense"])
+        self._native = _lib.native().Engine(config)
+        return self._native
+
+    def _entity_inputs(self, inputs):
+        """The entity tensors in the form the executor reads, or None where they are of another one."""
+        parts = []
+        for entity, bank, name, dim in ((inputs.user, self.user_bank, "user_tokenizer", self.spec.user_dense_dim),
+                                        (inputs.item, self.item_bank, "item_tokenizer", self.spec.item_dense_dim)):
+            ids, missing, values, dense_missing = entity.int_values, entity.int_missing_mask, entity.dense_values, entity.dense_missing_mask
+            if ids.dtype not in (torch.int32, torch.int64) or ids.ndim != 2:
+                return None
+            if name + ".missing_embeddings" in self.w and (missing is None or missing.dtype != torch.bool or missing.shape[1] < bank.n_fields):
+                return None
+            if dim > 0:
+                if values.dtype != torch.float32 or values.shape[1] != dim or values.stride(1) != 1:
+                    return None
+                if dense_missing is not None and (dense_missing.dtype != torch.bool or dense_missing.shape[1] < dim or dense_missing.stride(1) != 1):
+                    return None
+            parts.append((ids, missing, values, dense_missing))
+        return tuple(parts)
 
     def _predict_padded(self, inputs) -> tuple[torch.Tensor, torch.Tensor]:
         dev = self.device
@@ -700,232 +765,32 @@ class OneTransInference:
         ns_summary = ns_part.mean(dim=1) if ns_part.shape[1] > 0 else torch.zeros(batch, self.d, device=dev)
         return self._classify(seq_summary, ns_summary)
 
-    def _predict_packed(self, inputs, prepared: dict | None = None) -> tuple[torch.Tensor, torch.Tensor]:
-        """Same forward on valid tokens only (one sequence domain).
+    def _predict_packed(self, inputs, prepared=None) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+        """Same forward on valid tokens only (one sequence domain) -> (logits, embeddings, probabilities).
 
         Sample b owns ``n[b] + ns`` consecutive rows: its valid sequence tokens in order, then its NS
         tokens.  After block i the reference keeps the last ``S[i+1]`` padded positions; in packed form
         that drops the first ``min(n[b], S[i] - S[i+1])`` sequence rows of every sample.  All row counts
         follow from the per-sample lengths and the static pyramid schedule, so one device-to-host read
-        of a few integers sizes every buffer of the forward."""
-        dev = self.device
-        domain = self.domains[0]
+        of a few integers (``prepare``) sizes every buffer of the forward.  The launches are enqueued by the
+        native executor (csrc/host/engine.cpp)."""
         batch = inputs.user.int_values.shape[0]
-        ns = self.num_ns
-        seq = inputs.sequences[domain]
-        request_ts = inputs.request_timestamp
-        # duplicate removal + statistics: one kernel; `src` maps output slots to input positions, so the
-        # compacted [B, F, L] / [B, L] tensors of the reference are never materialised.  The valid counts, row
-        # offsets and totals that the static pyramid schedule implies come from a second kernel; the totals are the
-        # one host read of the forward (already on the host when the serving loop prepared this batch ahead of time)
-        if prepared is None or prepared["batch"] != batch:
+        seq = inputs.sequences[self.domains[0]]
+        if prepared is None or prepared.batch != batch:
             prepared = self.prepare(inputs)
-        src_map, stats, plan, widths = prepared["src_map"], prepared["stats"], prepared["plan"], prepared["widths"]
-        stat_vectors = [self._stats_vector(stats)]
-        values, ts = seq.values, seq.timestamps
-        max_len = values.shape[2]
-        width = widths[0]
-        start, n0 = plan["start"], plan["n0"]          # first kept position / valid sequence tokens at layer 0
-        counts = list(plan["counts"].unbind(0))        # [layers + 1] x [B] valid sequence tokens per sample
-        cu = list(plan["cu"].unbind(0))                # [layers + 1] x [B + 1] row offsets
-        cu_i32 = list(plan["cu32"].unbind(0))
-        prepared["ready"].synchronize()
-        meta = prepared["meta_host"].tolist()
-        totals = [int(m[0]) for m in meta]
-        max_rows = [int(m[1]) for m in meta]
-
-        # ---- sequence tokenizer on the valid events only (modeling/tokenizers.py:156-190).  It works
-        # directly in the packed layout of layer 0: the rows reserved for the NS tokens carry id 0 (the
-        # zero padding row) through the projection and are overwritten afterwards, which costs ns / (n + ns)
-        # extra rows but saves a full scatter of the token matrix.
-        total0 = totals[0]
-        prefix = f"sequence_tokenizers.{domain}"
-        entries = self.seq_tables[domain]
-        n_feat = values.shape[1]
-        emb = self.spec.emb_dim
-        live = [f for f in range(n_feat) if f < len(entries) and entries[f][1] is not None]
-        has_time = prefix + ".time_embedding.weight" in self.w
-        # ids of every feature, position and time-gap bucket of every packed row: one kernel instead of a dozen
-        # index operations over the token rows
-        if domain not in self._hash_buckets:
-            self._hash_buckets[domain] = torch.tensor(
-                [(-1 if f not in live else (entries[f][1].shape[0] - 1 if entries[f][0] == "compressed" else 0))
-                 for f in range(n_feat)], dtype=torch.long, device=dev)
-        ids_all, pos_full, buckets_full = ops.packed_token_index(
-            values, ts if has_time else None, request_ts, src_map, cu[0], n0, start, self._hash_buckets[domain], total0,
-            edges=self._edges if has_time else None)
-        seq_tables = [entries[f][1] if f in live else None for f in range(n_feat)]
-        proj_w = self._p(prefix + ".project.0.weight")
-        # gather -> projection -> SiLU -> LayerNorm -> time / position rows -> first RMSNorm as ONE kernel where the
-        # shapes allow it (bf16, whole-tile widths); else the row gather, the projection GEMM and the fused tail
-        one_kernel = (self.fused_tokenizer and self.dtype == torch.bfloat16 and bool(self.blocks) and bool(live)
-                      and ops.token_project_supported(seq_tables, proj_w))
-        projected = None
-        if not one_kernel:
-            if live:
-                token_input = (torch.empty if len(live) == n_feat else torch.zeros)(
-                    (total0, n_feat * emb), dtype=self.dtype, device=dev)
-                for f in live:
-                    ops.gather_rows(entries[f][1], ids_all[f], out=token_input, col0=f * emb)
-            else:
-                token_input = torch.zeros(total0, max(1, n_feat * emb), dtype=self.dtype, device=dev)
-            # Linear -> SiLU -> LayerNorm, the time-bucket and position rows and the first block's RMSNorm in one pass
-            # over the token matrix (`token_tail`); the NS rows are filled in afterwards
-            projected = self._linear(token_input, prefix + ".project.0")
-        ln_w, ln_b = self._p(prefix + ".project.2.weight"), self._p(prefix + ".project.2.bias")
-        pos_table = self._positions(width).to(self.dtype).contiguous()
-        rows_a, rows_b = (pos_table, pos_full), (None, None)
-        if has_time:
-            rows_a, rows_b = (self._p(prefix + ".time_embedding.weight"), buckets_full), (pos_table, pos_full)
-        first_norm_w = self._p(self.blocks[0]["p"] + ".attn_norm.weight") if self.blocks else None
-
-        def kept_rows(layer: int, want_row_dst: bool = False):
-            """Rows of layer ``layer`` that the pyramid keeps for the next one (in the next layer's order), the NS
-            rows [B, ns] of the next layer and, on request, the destination of every row of this layer (-1 = dropped)."""
-            src, next_ns, dst = ops.pyramid_kept_rows(cu[layer], cu[layer + 1], counts[layer], counts[layer + 1], ns,
-                                                      totals[layer], totals[layer + 1], want_row_dst=want_row_dst)
-            return (src, next_ns, dst) if want_row_dst else (src, next_ns)
-
-        # When the first block is evaluated for the kept rows only, its residual stream is needed for those rows
-        # alone: the fused pass then writes `tokens` already compacted and only `x_first` at full height.
-        first_kept = None
-        fused_tail = one_kernel or (first_norm_w is not None and projected.shape[1] % (16 // projected.element_size()) == 0)
-        if fused_tail and self.select_early and widths[1] < widths[0] and not (ns > 0 and max_rows[0] == ns) \
-                and totals[1] < 2**31:
-            *first_kept, row_dst = kept_rows(0, want_row_dst=True)
-        if one_kernel:
-            key = prefix + ".project.0#b32"
-            if key not in self._cast_cache:
-                self._cast_cache[key] = self.w[prefix + ".project.0.bias"].float().contiguous()
-            tokens, x_first = ops.token_project(seq_tables, ids_all, proj_w, self._cast_cache[key], ln_w, ln_b, rows_a[0],
-                                                rows_a[1], rows_b[0], rows_b[1], first_norm_w,
-                                                row_dst=None if first_kept is None else row_dst,
-                                                rows_out=None if first_kept is None else totals[1],
-                                                status=self.status_word)
-        elif fused_tail:
-            tokens, x_first = ops.token_tail(projected, ln_w, ln_b, rows_a[0], rows_a[1], rows_b[0], rows_b[1], first_norm_w,
-                                             row_dst=None if first_kept is None else row_dst,
-                                             rows_out=None if first_kept is None else totals[1])
-        else:
-            tokens = ops.layer_norm(projected, ln_w, ln_b, 1e-5, pre_silu=True)
-            ops.add_gathered_rows(tokens, rows_a[0], rows_a[1], rows_b[0], rows_b[1])
-            x_first = None
-
-        # ---- the NS tokens take the rows left for them: [seq rows of b | ns rows of b]
-        ns_tokens = self._ns_tokens(inputs, stat_vectors)                          # [B, ns, d]
-        ns_rows = plan["ns_rows0"]                                                 # [B, ns]
-        ns_flat = ns_tokens.reshape(batch * ns, self.d).contiguous()
-        ops.scatter_rows(tokens, (ns_rows if first_kept is None else first_kept[1]).reshape(-1), ns_flat)
-        if x_first is not None:   # the fused pass normalised placeholder rows there
-            ops.scatter_rows(x_first, ns_rows.reshape(-1), ops.rms_norm(ns_flat, first_norm_w, 1e-6))
-
-        d, heads, hd = self.d, self.heads, self.head_dim
-        for layer, blk in enumerate(self.blocks):
-            if ns > 0 and max_rows[layer] == ns:
-                # no sample has a sequence token left from here on: the remaining blocks only see the NS tokens
-                seq_summary = torch.zeros(batch, d, device=dev)
-                ns_summary = self._ns_only_blocks(tokens, layer, batch)
-                return self._classify(seq_summary, ns_summary)
-            p = blk["p"]
-            cu32 = cu_i32[layer]
-            x = x_first if (layer == 0 and x_first is not None) else ops.rms_norm(tokens, self._p(p + ".attn_norm.weight"), 1e-6)
-            flat_ns = ns_rows.t().reshape(-1)                                      # token-major: [ns, B] row ids
-            x_ns = ops.gather_rows(x, flat_ns).view(ns, batch, d)                  # [ns, B, d], contiguous
-            selected = self.select_early and widths[layer + 1] < widths[layer]
-            if selected:
-                # The pyramid keeps only the last rows of every sample after this block, and a row of the block's
-                # output depends on the other rows through its keys and values alone.  So keys and values are
-                # projected for every row, but queries, the attention rows, the output projection, the residual,
-                # the norm and the FFN only for the rows that survive: the same rows, bit for bit in exact
-                # arithmetic, as "whole block, then selection", without the work whose result would be dropped.
-                src, next_ns_rows = first_kept if (layer == 0 and first_kept is not None) else kept_rows(layer)
-                next_flat_ns = next_ns_rows.t().reshape(-1)
-                # every row the pyramid keeps is an NS row: the shared query projection and the shared FeedForward
-                # would be overwritten row for row by the per-token layers, so they are not run at all
-                only_ns_kept = ns > 0 and max_rows[layer + 1] == ns and "g_w1" in blk
-                kv = self._proj(x, blk["kv_w"], blk["kv_b"])                                        # [N, 2d]
-                if only_ns_kept:
-                    qm = torch.empty(totals[layer + 1], d, dtype=self.dtype, device=dev)
-                else:
-                    qm = self._proj(ops.gather_rows(x, src), blk["q_w"], blk["q_b"])                # [N', d]
-                if "g_kv_w" in blk:   # the per-token overrides of the NS rows: grouped GEMM, bias in its epilogue
-                    ops.scatter_rows(kv, flat_ns, self._grouped(x_ns, blk["g_kv_w"], blk["g_kv_b"]).view(ns * batch, 2 * d))
-                    ops.scatter_rows(qm, next_flat_ns, self._grouped(x_ns, blk["g_q_w"], blk["g_q_b"]).view(ns * batch, d))
-                else:
-                    ops.scatter_rows(kv, flat_ns, torch.bmm(x_ns, blk["ns_kv_w"]).view(ns * batch, 2 * d), bias=blk["ns_kv_b"])
-                    ops.scatter_rows(qm, next_flat_ns, torch.bmm(x_ns, blk["ns_q_w"]).view(ns * batch, d), bias=blk["ns_q_b"])
-                q = qm.unflatten(-1, (heads, hd))
-                k, v = (kv[:, i * d : (i + 1) * d].unflatten(-1, (heads, hd)) for i in range(2))
-                attn = ops.varlen_attention(q, k, v, causal=True, cu_rows=cu32, max_rows=max_rows[layer],
-                                            cu_rows_q=cu_i32[layer + 1], max_rows_q=max_rows[layer + 1],
-                                            kernel=self.attention_kernel if self.attention_kernel in (0, 1, 4) else 0, status=self.status_word)
-                if not (layer == 0 and first_kept is not None):   # else the tokenizer already wrote the kept rows only
-                    tokens = ops.gather_rows(tokens, src)
-                ns_rows, flat_ns = next_ns_rows, next_flat_ns
-            else:
-                qkv = self._proj(x, blk["qkv_w"], blk["qkv_b"])                       # [N, 3d]
-                if "g_qkv_w" in blk:
-                    ops.scatter_rows(qkv, flat_ns, self._grouped(x_ns, blk["g_qkv_w"], blk["g_qkv_b"]).view(ns * batch, 3 * d))
-                else:
-                    ops.scatter_rows(qkv, flat_ns, torch.bmm(x_ns, blk["ns_qkv_w"]).view(ns * batch, 3 * d), bias=blk["ns_qkv_b"])
-                q, k, v = (qkv[:, i * d : (i + 1) * d].unflatten(-1, (heads, hd)) for i in range(3))
-                attn = ops.varlen_attention(q, k, v, causal=True, cu_rows=cu32, max_rows=max_rows[layer],
-                                            kernel=self.attention_kernel, status=self.status_word)
-            attn2d = attn.view(-1, d).to(self.dtype)
-            folded = self.ffn_mode == "fp8"
-            if selected and only_ns_kept:
-                # the rest of this block for NS rows only, finishing token-major ([ns, B, d]) as the NS-only blocks
-                # want it: out projection with the residual in its epilogue, norm with the projection's bias added
-                # on the fly, per-token FeedForward with bias (+ that bias) and residual in the epilogues
-                tokens = self._proj(attn2d, blk["out_w"], None, residual=tokens, out=tokens)
-                x = ops.rms_norm(tokens, self._p(p + ".ffn_norm.weight"), 1e-6, in_bias=blk["out_b"])
-                x_ns = ops.gather_rows(x, flat_ns).view(ns, batch, d)
-                tok = ops.gather_rows(tokens, flat_ns).view(ns, batch, d)
-                h = self._grouped(x_ns, blk["g_w1"], blk["g_b1"], silu=True)
-                tok = self._grouped(h, blk["g_w2"], blk["g_b2_folded"], residual=tok, out=tok)
-                seq_summary = torch.zeros(batch, d, device=dev)
-                if layer + 1 == len(self.blocks):
-                    final = ops.rms_norm(tok.view(ns * batch, d), self._p("final_norm.weight"), 1e-6)
-                    return self._classify(seq_summary, final.view(ns, batch, d).mean(dim=0, dtype=torch.float32))
-                return self._classify(seq_summary, self._ns_only_blocks(tok, layer + 1, batch, token_major=True))
-            if folded:
-                # tokens + attention out-projection with the residual inside the GEMM's epilogue, in place; its bias
-                # is added by the norm on the fly and rides on the FFN output biases into the next residual
-                tokens = self._proj(attn2d, blk["out_w"], None, residual=tokens, out=tokens)
-                x = ops.rms_norm(tokens, self._p(p + ".ffn_norm.weight"), 1e-6, in_bias=blk["out_b"])
-                out = self._ffn_fp8(x, blk["ffn_fp8_folded"], tokens)
-            else:
-                tokens = self._proj(attn2d, blk["out_w"], blk["out_b32"], residual=tokens)
-                x = ops.rms_norm(tokens, self._p(p + ".ffn_norm.weight"), 1e-6)
-                out = self._shared_ffn_residual(blk, x, tokens)
-            x_ns = ops.gather_rows(x, flat_ns).view(ns, batch, d)
-            if "g_w1" in blk:   # per-token FeedForward on the grouped GEMM: bias + SiLU, then bias, in the epilogues
-                h = self._grouped(x_ns, blk["g_w1"], blk["g_b1"], silu=True)
-                y_ns = self._grouped(h, blk["g_w2"], blk["g_b2_folded" if folded else "g_b2"]).view(ns * batch, d)
-                ops.scatter_rows(out, flat_ns, y_ns, residual=tokens)              # tokens + b2 + FFN_ns(x)
-            else:
-                h = ops.bias_silu_rows(torch.bmm(x_ns, blk["ns_w1"]), blk["ns_b1"])
-                y_ns = torch.bmm(h, blk["ns_w2"]).view(ns * batch, d)
-                ops.scatter_rows(out, flat_ns, y_ns, bias=blk["ns_b2_folded" if folded else "ns_b2"], residual=tokens)
-            tokens = out
-            if not selected and widths[layer + 1] < widths[layer]:  # pyramid: drop the earliest sequence rows of every sample
-                src, ns_rows = kept_rows(layer)
-                tokens = ops.gather_rows(tokens, src)
-
-        last = len(widths) - 1
-        tokens = ops.rms_norm(tokens, self._p("final_norm.weight"), 1e-6).float()
-        n_last = counts[last]
-        total_seq = totals[last] - batch * ns
-        owner = torch.repeat_interleave(torch.arange(batch, device=dev), n_last, output_size=total_seq)
-        first_seq = torch.zeros(batch + 1, dtype=torch.long, device=dev)
-        first_seq[1:] = torch.cumsum(n_last, dim=0)
-        seq_rows = cu[last][owner] + (torch.arange(total_seq, device=dev) - first_seq[owner])
-        # rows of a sample are consecutive: a segmented sum in row order (no floating-point atomics, so the scores
-        # of a batch do not depend on which GPU or which run computed them)
-        seq_sum = torch.segment_reduce(tokens[seq_rows], "sum", lengths=n_last, axis=0, unsafe=True)
-        seq_summary = seq_sum / n_last.clamp_min(1).to(torch.float32)[:, None]
-        ns_summary = tokens[ns_rows.reshape(-1)].view(batch, ns, d).mean(dim=1)
-        return self._classify(seq_summary, ns_summary)
+        executor = self._executor()
+        timing = ops.kernel_timing_on()
+        entities = self._entity_inputs(inputs) if executor.assembles_ns_tokens() else None
+        ns_tokens = None if entities is not None else self._ns_tokens(inputs, [self._stats_vector(prepared.stats)])
+        tables = [table for _kind, table in self.seq_tables[self.domains[0]]]
+        one_kernel = self.fused_tokenizer and self.dtype == torch.bfloat16 and any(t is not None for t in tables) \
+            and ops.token_project_supported(tables, self._p(f"sequence_tokenizers.{self.domains[0]}.project.0.weight"))
+        done, tokens, layer, token_major, seq_mean, ns_mean = executor.blocks(
+            prepared, seq.values, seq.timestamps, inputs.request_timestamp, entities or (), ns_tokens,
+            self._positions(prepared.widths[0]), self.blocks, self.select_early, one_kernel, self.attention_kernel, timing)
+        if not done:      # no sample has a sequence token left: the remaining blocks only see the NS tokens
+            ns_mean = self._ns_only_blocks(tokens, layer, batch, token_major=True) if token_major else self._ns_only_blocks(tokens, layer, batch)
+        return executor.classify(seq_mean, ns_mean, timing)
 
     def _ns_only_blocks(self, tokens: torch.Tensor, first_layer: int, batch: int, token_major: bool = False) -> torch.Tensor:
         """Blocks ``first_layer`` .. end for a batch whose samples hold nothing but their NS tokens, then the final
@@ -935,47 +800,19 @@ class OneTransInference:
         takes the per-token projections and the per-token FeedForward, and every sample attends causally over
         its ``ns`` tokens.  The block then is six batched or shared matrix products on a token-major
         ``[ns, B, d]`` tensor with no gathers, scatters or shared-weight work that would be overwritten."""
-        ns, d, heads, hd = self.num_ns, self.d, self.heads, self.head_dim
-        tok = tokens if token_major else tokens.view(batch, ns, d).transpose(0, 1).contiguous()            # [ns, B, d]
-        flat = tok.view(ns * batch, d)
-        for blk in self.blocks[first_layer:]:
-            p = blk["p"]
-            x = ops.rms_norm(flat, self._p(p + ".attn_norm.weight"), 1e-6)
-            fused = "g_qkv_w" in blk   # every layer of the block in one tcgen05 GEMM each, epilogues inside
-            if fused:
-                qkv = self._grouped(x.view(ns, batch, d), blk["g_qkv_w"], blk["g_qkv_b"])
-            else:
-                qkv = ops.bias_act_rows(torch.bmm(x.view(ns, batch, d), blk["ns_qkv_w"]), blk["ns_qkv_b"], silu=False)
-            # sample-major views of the token-major tensors: (B, L = ns, H, hd) with strides (3d, B * 3d, hd, 1)
-            q, k, v = (qkv[:, :, i * d : (i + 1) * d].unflatten(-1, (heads, hd)).permute(1, 0, 2, 3) for i in range(3))
-            attn = torch.empty(ns, batch, heads, hd, dtype=q.dtype, device=q.device)
-            ops.varlen_attention(q, k, v, causal=True, layout="blhd", kernel=self.attention_kernel,
-                                 out=attn.permute(1, 0, 2, 3), status=self.status_word)
-            # attention output projection onto the residual stream; its bias is added by the norm on the fly and
-            # rides on the FFN's output bias into the next residual
-            if fused:
-                self._grouped(attn.view(ns * batch, d), blk["g_out_w"], None, residual=flat, out=flat)
-            else:
-                flat.addmm_(attn.view(ns * batch, d).to(self.dtype), blk["out_w_t"])
-            x = ops.rms_norm(flat, self._p(p + ".ffn_norm.weight"), 1e-6, in_bias=blk["out_b"])
-            if fused:
-                h = self._grouped(x.view(ns, batch, d), blk["g_w1"], blk["g_b1"], silu=True)
-                tok = self._grouped(h, blk["g_w2"], blk["g_b2_folded"], residual=tok, out=tok)
-            else:
-                h = ops.bias_act_rows(torch.bmm(x.view(ns, batch, d), blk["ns_w1"]), blk["ns_b1"], silu=True)
-                tok = ops.bias_act_rows(torch.baddbmm(tok, h, blk["ns_w2"]), blk["ns_b2_folded"], silu=False)
-            flat = tok.view(ns * batch, d)
-        final = ops.rms_norm(flat, self._p("final_norm.weight"), 1e-6)
-        return final.view(ns, batch, d).mean(dim=0, dtype=torch.float32)     # widened inside the reduction, no fp32 copy
+        return self._executor().ns_only(tokens, first_layer, batch, token_major, self.blocks, self.attention_kernel, ops.kernel_timing_on())
 
     @torch.inference_mode()
-    def scores(self, inputs, micro_batch: int | None = None, prepared: dict | None = None) -> torch.Tensor:
+    def scores(self, inputs, micro_batch: int | None = None, prepared=None) -> torch.Tensor:
         """Sigmoid conversion probabilities (fp32, on the device): [B] for one action, else [B, actions].
         ``micro_batch`` bounds the rows that go through the network at once (samples are independent,
         so the result does not depend on it); it caps activation memory at large batches.  ``prepared``: the
         result of ``prepare(inputs)`` for a batch that goes through in one piece."""
         batch = inputs.user.int_values.shape[0]
         if micro_batch is None or micro_batch >= batch:
+            if self.packed and len(self.domains) == 1:
+                probs = self._predict_packed(inputs, prepared)[2]
+                return probs.reshape(-1) if probs.shape[1] == 1 else probs
             logits, _ = self.predict(inputs, prepared)
         else:
             logits = torch.cat([self.predict(inputs.slice(lo, min(lo + micro_batch, batch)))[0]

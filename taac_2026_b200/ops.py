@@ -75,6 +75,10 @@ def set_kernel_timing(sink: list | None) -> None:
     _TIMING = sink
 
 
+def kernel_timing_on() -> bool:
+    return _TIMING is not None
+
+
 class _LazyHost:
     """Stands for the host module until the first call."""
 

@@ -57,6 +57,8 @@ constexpr int kWarpsQ = 4;
 template <typename T>
 __global__ void __launch_bounds__(kWarpsQ * 32)
 attn_bwd_query_kernel(const BwdArgs g, const int D) {
+    chain_release();
+    chain_wait();
     extern __shared__ float smem[];
     const AttnArgs& a = g.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -138,6 +140,8 @@ constexpr int kWarpsK = 2;
 template <typename T>
 __global__ void __launch_bounds__(kWarpsK * 32)
 attn_bwd_key_kernel(const BwdArgs g, const int D) {
+    chain_release();
+    chain_wait();
     extern __shared__ float smem[];
     const AttnArgs& a = g.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -214,11 +218,11 @@ int launch(const BwdArgs& g, int D, cudaStream_t stream) {
     }
     const unsigned zq = static_cast<unsigned>((a.Lq + kWarpsQ - 1) / kWarpsQ);
     const unsigned zk = static_cast<unsigned>((a.Lk + kWarpsK - 1) / kWarpsK);
-    attn_bwd_query_kernel<T><<<dim3(a.B, a.H, zq), kWarpsQ * 32, smem_q, stream>>>(g, D);
+    launch_chained(attn_bwd_query_kernel<T>, dim3(a.B, a.H, zq), kWarpsQ * 32, smem_q, stream, g, D);
     count_launch();
     int code = launch_status();
     if (code != TB200_OK) return code;
-    attn_bwd_key_kernel<T><<<dim3(a.B, a.H, zk), kWarpsK * 32, smem_k, stream>>>(g, D);
+    launch_chained(attn_bwd_key_kernel<T>, dim3(a.B, a.H, zk), kWarpsK * 32, smem_k, stream, g, D);
     count_launch();
     return launch_status();
 }

@@ -134,6 +134,8 @@ __device__ __forceinline__ void store_rows(T* gmem, int64_t stride_l, const T* t
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, D <= 64 ? 3 : 2)
 attn_bwd_dq_kernel(const BwdArgs g) {
+    chain_release();
+    chain_wait();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ float s_delta[kM];
     T* sQ = reinterpret_cast<T*>(smem_raw);
@@ -313,6 +315,8 @@ attn_bwd_dq_kernel(const BwdArgs g) {
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, D <= 64 ? 3 : 2)
 attn_bwd_dkv_kernel(const BwdArgs g) {
+    chain_release();
+    chain_wait();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(16) float s_lse[2][kM];
     __shared__ __align__(16) float s_delta[2][kM];
@@ -460,11 +464,11 @@ int launch(const BwdArgs& g, cudaStream_t stream) {
         cudaFuncSetAttribute(attn_bwd_dkv_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         attr_set[dev.index] = true;
     }
-    attn_bwd_dq_kernel<T, D><<<dim3((a.Lq + kM - 1) / kM, a.H, a.B), kThreads, smem, stream>>>(g);
+    launch_chained(attn_bwd_dq_kernel<T, D>, dim3((a.Lq + kM - 1) / kM, a.H, a.B), kThreads, smem, stream, g);
     count_launch();
     const int code = launch_status();
     if (code != TB200_OK) return code;
-    attn_bwd_dkv_kernel<T, D><<<dim3((a.Lk + kM - 1) / kM, a.H, a.B), kThreads, smem, stream>>>(g);
+    launch_chained(attn_bwd_dkv_kernel<T, D>, dim3((a.Lk + kM - 1) / kM, a.H, a.B), kThreads, smem, stream, g);
     count_launch();
     return launch_status();
 }

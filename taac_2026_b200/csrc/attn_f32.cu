@@ -22,6 +22,8 @@ constexpr int kMaxD = 256;
 
 __global__ void __launch_bounds__(kWarps * 32)
 attn_f32_kernel(const AttnArgs a, const int D, const int lk_cap) {
+    chain_release();
+    chain_wait();
     extern __shared__ float smem[];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -125,7 +127,7 @@ int attn_f32_forward(const AttnArgs& a, int head_dim, int max_lq, int max_lk, cu
     const unsigned row_blocks = static_cast<unsigned>((max_lq + kWarps - 1) / kWarps);
     if (a.H > 65535 || row_blocks > 65535) return TB200_ERR_SHAPE;
     dim3 grid(static_cast<unsigned>(a.B), static_cast<unsigned>(a.H), row_blocks);
-    attn_f32_kernel<<<grid, kWarps * 32, smem, stream>>>(a, head_dim, lk_cap);
+    launch_chained(attn_f32_kernel, grid, kWarps * 32, smem, stream, a, head_dim, lk_cap);
     count_launch();
     return launch_status();
 }

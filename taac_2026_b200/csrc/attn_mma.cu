@@ -33,6 +33,8 @@ __device__ __forceinline__ void load_tile(T* smem, const T* gmem, int64_t stride
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, D <= 64 ? 4 : 2) attn_mma_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     T* sQ = reinterpret_cast<T*>(smem_raw);
     T* sK = sQ + kBM * D;              // kKvStages stages
@@ -292,6 +294,8 @@ constexpr int kTinyWarps = 4;
 template <typename T>
 __global__ void __launch_bounds__(kTinyWarps * 32)
 attn_tiny_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
     constexpr int D = 64;
     constexpr int CH = D / 8;
     __shared__ __align__(128) T tiles[kTinyWarps][3][kTinyL * D];   // Q (later the output), K, V per warp
@@ -438,6 +442,8 @@ constexpr int kFqRows = 16;    // keys per tile = queries per tile
 template <typename T>
 __global__ void __launch_bounds__(kFqWarps * 32, 4)
 attn_fewq_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
     constexpr int D = 64;
     constexpr int CH = D / 8;
     extern __shared__ __align__(128) uint8_t fq_smem[];
@@ -638,7 +644,7 @@ int launch(const AttnArgs& a, int max_lq, cudaStream_t stream) {
         attr_set[dev.index] = true;
     }
     dim3 grid((max_lq + kBM - 1) / kBM, a.H, a.B);
-    attn_mma_kernel<T, D><<<grid, kThreads, smem, stream>>>(a);
+    launch_chained(attn_mma_kernel<T, D>, grid, kThreads, smem, stream, a);
     count_launch();
     return launch_status();
 }
@@ -653,8 +659,8 @@ int attn_tiny_forward(const AttnArgs& a, int dtype, cudaStream_t stream) {
     const int64_t pairs = static_cast<int64_t>(a.B) * a.H;
     const int64_t grid = (pairs + kTinyWarps - 1) / kTinyWarps;
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
-    if (dtype == TB200_BF16) attn_tiny_kernel<__nv_bfloat16><<<static_cast<unsigned>(grid), kTinyWarps * 32, 0, stream>>>(a);
-    else attn_tiny_kernel<__half><<<static_cast<unsigned>(grid), kTinyWarps * 32, 0, stream>>>(a);
+    if (dtype == TB200_BF16) launch_chained(attn_tiny_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kTinyWarps * 32, 0, stream, a);
+    else launch_chained(attn_tiny_kernel<__half>, static_cast<unsigned>(grid), kTinyWarps * 32, 0, stream, a);
     count_launch();
     return launch_status();
 }
@@ -682,8 +688,8 @@ int attn_fewq_forward(const AttnArgs& a, int dtype, cudaStream_t stream) {
         cudaFuncSetAttribute(attn_fewq_kernel<__half>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr_set[dev.index] = true;
     }
-    if (dtype == TB200_BF16) attn_fewq_kernel<__nv_bfloat16><<<static_cast<unsigned>(grid), kFqWarps * 32, smem, stream>>>(a);
-    else attn_fewq_kernel<__half><<<static_cast<unsigned>(grid), kFqWarps * 32, smem, stream>>>(a);
+    if (dtype == TB200_BF16) launch_chained(attn_fewq_kernel<__nv_bfloat16>, static_cast<unsigned>(grid), kFqWarps * 32, smem, stream, a);
+    else launch_chained(attn_fewq_kernel<__half>, static_cast<unsigned>(grid), kFqWarps * 32, smem, stream, a);
     count_launch();
     return launch_status();
 }

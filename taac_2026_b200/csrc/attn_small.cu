@@ -37,6 +37,8 @@ __device__ __forceinline__ float ex2(float x) {
 template <typename T, int P>
 __global__ void __launch_bounds__(kWarps * 32)
 attn_small_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
     constexpr int CPL = kChunks / P;      // 16-byte pieces of a row per lane
     constexpr int kRows = kMaxL / P;      // rows one warp can serve
     __shared__ uint4 kv_s[kWarps][2][kMaxL * kChunks];   // per warp: K rows, V rows
@@ -164,9 +166,9 @@ void launch_small(const AttnArgs& a, int64_t grid, cudaStream_t stream) {
     // upper bound of the query rows a warp serves (the keys always fit: kMaxL rows of shared memory per warp)
     const int longest = a.cu_rows_q != nullptr ? a.Lq : (a.Lq > a.Lk ? a.Lq : a.Lk);
     const unsigned g = static_cast<unsigned>(grid);
-    if (longest <= kMaxL / 4) attn_small_kernel<T, 4><<<g, kWarps * 32, 0, stream>>>(a);
-    else if (longest <= kMaxL / 2) attn_small_kernel<T, 2><<<g, kWarps * 32, 0, stream>>>(a);
-    else attn_small_kernel<T, 1><<<g, kWarps * 32, 0, stream>>>(a);
+    if (longest <= kMaxL / 4) launch_chained(attn_small_kernel<T, 4>, g, kWarps * 32, 0, stream, a);
+    else if (longest <= kMaxL / 2) launch_chained(attn_small_kernel<T, 2>, g, kWarps * 32, 0, stream, a);
+    else launch_chained(attn_small_kernel<T, 1>, g, kWarps * 32, 0, stream, a);
 }
 
 }  // namespace

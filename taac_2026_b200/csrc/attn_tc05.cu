@@ -189,6 +189,8 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    chain_release();   // not before every CTA holds its tensor memory (see launch_chained)
+    chain_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
@@ -592,7 +594,7 @@ int attn_tc05_forward(const AttnArgs& a, int max_lq, int64_t total_rows, int32_t
     const int64_t items = static_cast<int64_t>((a.Lq + kBM - 1) / kBM) * a.H * a.B;
     int64_t grid = static_cast<int64_t>(dev.sm_count) * 2;  // persistent: two CTAs per SM
     if (grid > items) grid = items;
-    attn_tc05_kernel<<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(tq, tk, tv, args);
+    launch_chained(attn_tc05_kernel, static_cast<unsigned>(grid), kThreads, smem, stream, tq, tk, tv, args);
     count_launch();
     return launch_status();
 }

@@ -25,6 +25,8 @@ template <typename T, typename IdT, int G>      // G lanes per bag (power of two
 __global__ void __launch_bounds__(256)
 bag_mean_bwd_kernel(const IdT* __restrict__ ids, const T* __restrict__ grad_out, int64_t* __restrict__ rows_out,
                     T* __restrict__ vals_out, int64_t batch, int bag, int dim, int64_t vocab_rows) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int lane = threadIdx.x & 31;
     const int sub = lane / G;
@@ -74,7 +76,7 @@ int launch(const void* ids, const void* grad_out, int64_t* rows_out, void* vals_
     const int64_t cap = static_cast<int64_t>(dev.sm_count) * 8;
     if (grid > cap) grid = cap;
 #define TB200_BB(G_)                                                                                                       \
-    bag_mean_bwd_kernel<T, IdT, G_><<<static_cast<unsigned>(grid), 256, 0, stream>>>(                                      \
+    launch_chained(bag_mean_bwd_kernel<T, IdT, G_>, static_cast<unsigned>(grid), 256, 0, stream,                                      \
         static_cast<const IdT*>(ids), static_cast<const T*>(grad_out), rows_out, static_cast<T*>(vals_out), batch, bag, dim, vocab_rows)
     switch (g) {
         case 1: TB200_BB(1); break;

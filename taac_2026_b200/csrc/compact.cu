@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(256)
 expand_sequence_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ gaps, const int32_t* __restrict__ cu,
                        const int64_t* __restrict__ request_ts, int64_t* __restrict__ values, int64_t* __restrict__ lengths,
                        int64_t* __restrict__ timestamps, int batch, int feats, int max_len, int64_t ids_stride) {
+    chain_release();
+    chain_wait();
     const int pairs = max_len >> 1;                      // max_len is even
     const int64_t total = static_cast<int64_t>(batch) * pairs;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -105,7 +107,7 @@ extern "C" int tb200_expand_sequence(const int32_t* ids, const int32_t* gaps, co
     const int64_t total = static_cast<int64_t>(batch) * (max_len / 2);
     int64_t grid = (total + 255) / 256;
     grid = std::min<int64_t>(grid, static_cast<int64_t>(dev.sm_count) * 16);
-    expand_sequence_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(expand_sequence_kernel, static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream),
         ids, gaps, cu, request_ts, values, lengths, timestamps, batch, feats, max_len, ids_stride);
     count_launch();
     return launch_status();

@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(kThreads)
 small_token_kernel(const float* __restrict__ values, int n, int64_t value_stride, const uint8_t* __restrict__ mask, int64_t mask_stride,
                    int in_dim, const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ gamma,
                    const float* __restrict__ beta, T* __restrict__ out, int64_t out_stride, int64_t rows, int d, float eps) {
+    chain_release();
+    chain_wait();
     extern __shared__ float smem[];
     float* xs = smem;                       // [kWarps][in_dim]
     float* hs = smem + kWarps * in_dim;     // [kWarps][d]
@@ -79,6 +81,8 @@ __global__ void __launch_bounds__(kThreads)
 ns_rows_kernel(const T* __restrict__ ns_tokens, int64_t n, int ns, int64_t batch, int chunks, const T* __restrict__ gamma, float eps,
                const int64_t* __restrict__ token_rows, uint4* __restrict__ tokens, const int64_t* __restrict__ normed_rows,
                uint4* __restrict__ normed, uint4* __restrict__ token_major) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int lane = threadIdx.x & 31;
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
@@ -120,6 +124,8 @@ template <typename T, int CPL>
 __global__ void __launch_bounds__(kThreads)
 pool_rows_kernel(const uint4* __restrict__ rows, const int64_t* __restrict__ cu, const int64_t* __restrict__ counts, int64_t batch, int ns,
                  int chunks, const uint4* __restrict__ gamma, float eps, float* __restrict__ seq_out, float* __restrict__ ns_out) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int lane = threadIdx.x & 31;
     const int64_t b = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
@@ -179,6 +185,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 join_summaries_kernel(const float* __restrict__ seq, const float* __restrict__ ns, float* __restrict__ joined, T* __restrict__ joined_t,
                       int64_t batch, int d) {
+    chain_release();
+    chain_wait();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
     if (i >= batch * 2 * d) return;
     const int64_t b = i / (2 * d);
@@ -193,6 +201,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 head_kernel(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ logits,
             float* __restrict__ probs, int64_t batch, int d, int actions) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int lane = threadIdx.x & 31;
     const int64_t b = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
@@ -237,7 +247,7 @@ extern "C" int tb200_small_token_fwd(const float* values, int32_t n, int64_t val
     const size_t smem = static_cast<size_t>(kWarps) * (in_dim + d) * sizeof(float);
     if (smem > 48 * 1024 || rows > (1ll << 33)) return TB200_ERR_UNSUPPORTED;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    TB200_BY_DTYPE((small_token_kernel<T><<<warps_grid(rows), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+    TB200_BY_DTYPE((launch_chained(small_token_kernel<T>, warps_grid(rows), kThreads, smem, static_cast<cudaStream_t>(stream),
         values, n, value_stride, mask, mask_stride, in_dim, w, bias, gamma, beta, static_cast<T*>(out), out_stride, rows, d, eps)));
     count_launch();
     return launch_status();
@@ -260,7 +270,7 @@ extern "C" int tb200_ns_rows_fwd(const void* ns_tokens, int64_t batch, int32_t n
     if (batch * ns > (1ll << 33)) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
     const int chunks = d * es / 16;
-    TB200_BY_DTYPE((ns_rows_kernel<T><<<warps_grid(batch * ns), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    TB200_BY_DTYPE((launch_chained(ns_rows_kernel<T>, warps_grid(batch * ns), kThreads, 0, static_cast<cudaStream_t>(stream),
         static_cast<const T*>(ns_tokens), batch * ns, ns, batch, chunks, static_cast<const T*>(gamma), eps, token_rows,
         static_cast<uint4*>(tokens), normed_rows, static_cast<uint4*>(normed), static_cast<uint4*>(token_major))));
     count_launch();
@@ -281,7 +291,7 @@ extern "C" int tb200_pool_rows_fwd(const void* rows, const int64_t* cu, const in
     if (chunks > 256 || batch > (1ll << 33)) return TB200_ERR_UNSUPPORTED;
     if (!device_info().valid) return TB200_ERR_DEVICE;
 #define TB200_POOL(CPL_)                                                                                                              \
-    TB200_BY_DTYPE((pool_rows_kernel<T, CPL_><<<warps_grid(batch), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(                 \
+    TB200_BY_DTYPE((launch_chained(pool_rows_kernel<T, CPL_>, warps_grid(batch), kThreads, 0, static_cast<cudaStream_t>(stream),                 \
         static_cast<const uint4*>(rows), cu, counts, batch, ns, chunks, static_cast<const uint4*>(gamma), eps, seq_mean, ns_mean)))
     if (chunks <= 32) { TB200_POOL(1); }
     else if (chunks <= 64) { TB200_POOL(2); }
@@ -301,7 +311,7 @@ extern "C" int tb200_join_summaries(const float* seq, const float* ns, float* jo
     if (batch * 2 * d > (1ll << 38)) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
     const auto grid = static_cast<unsigned>((batch * 2 * d + kThreads - 1) / kThreads);
-    TB200_BY_DTYPE((join_summaries_kernel<T><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(seq, ns, joined, static_cast<T*>(joined_cast),
+    TB200_BY_DTYPE((launch_chained(join_summaries_kernel<T>, grid, kThreads, 0, static_cast<cudaStream_t>(stream), seq, ns, joined, static_cast<T*>(joined_cast),
                                                                                                      batch, d)));
     count_launch();
     return launch_status();
@@ -318,7 +328,7 @@ extern "C" int tb200_head_fwd(const void* h, const float* w, const float* bias, 
     if ((static_cast<int64_t>(d) * es) % 16 != 0 || !aligned16(h)) return TB200_ERR_ALIGN;
     if (batch > (1ll << 33)) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    TB200_BY_DTYPE((head_kernel<T><<<warps_grid(batch), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const T*>(h), w, bias, logits,
+    TB200_BY_DTYPE((launch_chained(head_kernel<T>, warps_grid(batch), kThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const T*>(h), w, bias, logits,
                                                                                                        probs, batch, d, actions)));
     count_launch();
     return launch_status();

@@ -185,6 +185,8 @@ ffn_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    chain_release();   // not before every CTA holds its tensor memory (see launch_chained)
+    chain_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -486,6 +488,8 @@ ffn_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 quant_act_kernel(const uint4* __restrict__ x, uint2* __restrict__ q, float* __restrict__ scales, int64_t n_blocks) {
+    chain_release();
+    chain_wait();
     // 16 lanes x 8 values = one 1 x 128 block
     const int64_t gthread = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
     const int64_t block = gthread >> 4;
@@ -569,7 +573,7 @@ int launch_gemm_impl(const CUtensorMap& ta, const CUtensorMap& tb, const CUtenso
         if (walkers > m_tiles) walkers = m_tiles;
         grid = walkers * n_tiles;
     }
-    ffn_gemm_kernel<MODE, B_RES><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(ta, tb, to, tr, g);
+    launch_chained(ffn_gemm_kernel<MODE, B_RES>, static_cast<unsigned>(grid), kThreads, smem, stream, ta, tb, to, tr, g);
     count_launch();
     return launch_status();
 }
@@ -628,7 +632,7 @@ extern "C" int tb200_quant_act_1x128(const void* x_bf16, void* x_fp8, float* sca
     const int64_t n_blocks = M * (K / 128);
     const int64_t grid = (n_blocks * 16 + 255) / 256;
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
-    quant_act_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(quant_act_kernel, static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream),
         static_cast<const uint4*>(x_bf16), static_cast<uint2*>(x_fp8), scales, n_blocks);
     count_launch();
     return launch_status();

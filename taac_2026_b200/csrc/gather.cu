@@ -39,6 +39,8 @@ __global__ void __launch_bounds__(kThreads)
 gather_rows_kernel(const uint4* __restrict__ table, int64_t vocab_rows, int chunks, const void* __restrict__ ids,
                    int64_t n, int64_t seq_len, int64_t ids_batch_stride, uint4* __restrict__ out,
                    int64_t out_stride_chunks, int out_col0_chunks, int lanes_per_row, int rows_per_cta) {
+    chain_release();
+    chain_wait();
     __shared__ int32_t ids_s[kRowsPerCta];
     const int tid = threadIdx.x;
     const int64_t base = static_cast<int64_t>(blockIdx.x) * rows_per_cta;
@@ -101,6 +103,8 @@ struct BagArgs {
 template <typename T, typename I>
 __global__ void __launch_bounds__(kThreads)
 bag_mean_kernel(BagArgs a, const void* __restrict__ ids, T* __restrict__ out) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     extern __shared__ int32_t bag_ids[];  // [bags_per_cta, max_bag]; 0 = skip
     const int tid = threadIdx.x;
@@ -253,6 +257,8 @@ scatter_rows_kernel(uint4* __restrict__ dst, int64_t dst_stride_chunks, int dst_
                     const int64_t* __restrict__ ids, const uint4* __restrict__ src, int chunks, int64_t n,
                     const uint4* __restrict__ bias, int64_t rows_per_group, const uint4* __restrict__ residual,
                     int64_t res_stride_chunks, int lanes_per_row) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int G = lanes_per_row;
     const int group = threadIdx.x / G;
@@ -295,6 +301,8 @@ __global__ void __launch_bounds__(kThreads)
 add_gathered_rows_kernel(uint4* __restrict__ x, int64_t n, int chunks, const uint4* __restrict__ table_a, int64_t rows_a,
                          const int64_t* __restrict__ ids_a, const uint4* __restrict__ table_b, int64_t rows_b,
                          const int64_t* __restrict__ ids_b, int lanes_per_row) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     const int G = lanes_per_row;
     const int group = threadIdx.x / G;
@@ -335,6 +343,8 @@ template <typename T, bool SILU>
 __global__ void __launch_bounds__(kThreads)
 bias_act_rows_kernel(uint4* __restrict__ x, int64_t rows, int chunks, const uint4* __restrict__ bias,
                      int64_t rows_per_group) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     constexpr int U = 4;   // 16-byte pieces in flight per thread
     // a thread keeps one column piece c and walks down the rows, so its bias piece changes only with the group
@@ -397,9 +407,9 @@ int bag_launch(BagArgs a, const void* ids, int ids_dtype, void* out, cudaStream_
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     const size_t smem = static_cast<size_t>(per) * a.max_bag * sizeof(int32_t);
     if (ids_dtype == TB200_I64)
-        bag_mean_kernel<T, int64_t><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(a, ids, static_cast<T*>(out));
+        launch_chained(bag_mean_kernel<T, int64_t>, static_cast<unsigned>(grid), kThreads, smem, stream, a, ids, static_cast<T*>(out));
     else
-        bag_mean_kernel<T, int32_t><<<static_cast<unsigned>(grid), kThreads, smem, stream>>>(a, ids, static_cast<T*>(out));
+        launch_chained(bag_mean_kernel<T, int32_t>, static_cast<unsigned>(grid), kThreads, smem, stream, a, ids, static_cast<T*>(out));
     count_launch();
     return launch_status();
 }
@@ -520,11 +530,11 @@ extern "C" int tb200_gather_rows(const void* table, int64_t vocab_rows, int32_t 
     const int64_t grid = (n + rows_per_cta - 1) / rows_per_cta;
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (ids_dtype == TB200_I64)
-        gather_rows_kernel<int64_t><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(
+        launch_chained(gather_rows_kernel<int64_t>, static_cast<unsigned>(grid), kThreads, 0, s,
             static_cast<const uint4*>(table), vocab_rows, chunks, ids, n, seq_len, ids_batch_stride,
             static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G, static_cast<int>(rows_per_cta));
     else
-        gather_rows_kernel<int32_t><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(
+        launch_chained(gather_rows_kernel<int32_t>, static_cast<unsigned>(grid), kThreads, 0, s,
             static_cast<const uint4*>(table), vocab_rows, chunks, ids, n, seq_len, ids_batch_stride,
             static_cast<uint4*>(out), out_stride * es / 16, out_col0 * es / 16, G, static_cast<int>(rows_per_cta));
     count_launch();
@@ -555,7 +565,7 @@ extern "C" int tb200_scatter_rows(void* dst, int64_t dst_rows, int64_t dst_strid
     if (grid > cap) grid = cap;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define TB200_SCATTER(T)                                                                                              \
-    scatter_rows_kernel<T><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(                                          \
+    launch_chained(scatter_rows_kernel<T>, static_cast<unsigned>(grid), kThreads, 0, s,                                          \
         static_cast<uint4*>(dst), dst_stride * es / 16, dst_col0 * es / 16, ids, static_cast<const uint4*>(src), chunks, \
         n, static_cast<const uint4*>(bias), rows_per_group < 1 ? 1 : rows_per_group, static_cast<const uint4*>(residual), \
         residual_stride * es / 16, G)
@@ -591,7 +601,7 @@ extern "C" int tb200_add_gathered_rows(void* x, int64_t n, int32_t dim, const vo
     if (grid > cap) grid = cap;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define TB200_ADDG(T)                                                                                                 \
-    add_gathered_rows_kernel<T><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(                                     \
+    launch_chained(add_gathered_rows_kernel<T>, static_cast<unsigned>(grid), kThreads, 0, s,                                     \
         static_cast<uint4*>(x), n, chunks, static_cast<const uint4*>(table_a), rows_a, ids_a,                         \
         static_cast<const uint4*>(table_b), rows_b, ids_b, G)
     switch (dtype) {
@@ -624,10 +634,10 @@ extern "C" int tb200_bias_act_rows(void* x, int64_t rows, int32_t cols, const vo
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define TB200_BSILU(T)                                                                                        \
     if (act == 1)                                                                                             \
-        bias_act_rows_kernel<T, true><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(                       \
+        launch_chained(bias_act_rows_kernel<T, true>, static_cast<unsigned>(grid), kThreads, 0, s,                       \
             static_cast<uint4*>(x), rows, chunks, static_cast<const uint4*>(bias), rows_per_group);           \
     else                                                                                                      \
-        bias_act_rows_kernel<T, false><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(                      \
+        launch_chained(bias_act_rows_kernel<T, false>, static_cast<unsigned>(grid), kThreads, 0, s,                      \
             static_cast<uint4*>(x), rows, chunks, static_cast<const uint4*>(bias), rows_per_group)
     switch (dtype) {
         case TB200_F32: TB200_BSILU(float); break;

@@ -6,47 +6,31 @@
 // one group.  A library batched GEMM leaves the bias, the SiLU and the residual to further passes over the
 // result; here they ride in the epilogue, and the result is written once.
 //
-// Two kernels share the file.  `gemm_bf16_pair_kernel` (further down) is the one that normally runs: clusters of
-// two CTAs on 256 x 256 tiles with tcgen05 cta_group::2.  `gemm_bf16_kernel` is its single-CTA form, used for
-// matrices of at most 128 rows and when TB200_GEMM_PAIR=0 is set in the environment (for comparison):
-// one persistent CTA per SM walks the (group, row tile, column tile) list round-robin, column tiles fastest,
-// so that the CTAs working side by side share the activation rows.  Roles in its CTA of 320 threads:
-//   warp 0      TMA producer: ring of {A 128 x 64, W 256 x 64} bf16 tiles, 128-byte swizzle, 4 stages
-//   warp 1      MMA issuer (one lane): tcgen05.mma kind::f16 128 x 256 x 16, the whole K range of a tile
-//               accumulates in one of two 256-column TMEM buffers
-//   warps 2..9  epilogue: a thread owns one row, reads 32 of its columns from TMEM per round, adds the bias, applies
-//               the activation, adds the residual (read from global memory a round ahead) and writes bf16 into one
-//               of two alternating 128-byte-swizzled 16 KB staging boxes that one thread hands to TMA; meanwhile the
-//               tensor cores fill the other TMEM buffer with the next tile.
+// `gemm_bf16_pair_kernel` runs clusters of two CTAs on 256 x 256 tiles with tcgen05 cta_group::2.  It is the kernel of many
+// rows; gemm_small.cu and gemm_narrow.cu hold those of few rows per group, where the weights are the traffic and a 256-row
+// tile would be mostly padding (the dispatch at the end of this file says where the lines lie).
 // Every wait on an mbarrier is bounded; a wait that gives up raises the status word and all roles drain out
 // through the final barrier, where the TMEM allocation is released.
 #include <cudaTypedefs.h>
-
-#include <cstdlib>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
 
 namespace tb200 {
 void count_launch();
+int gemm_small(const void* a, const void* w, const float* bias, const void* residual, void* out, int groups, int M, int N, int K, int act,
+               cudaStream_t stream);
+int gemm_narrow(const void* a, const void* w, const float* bias, const void* residual, void* out, int groups, int M, int N, int K, int act,
+                int32_t* status, cudaStream_t stream);
 
 namespace {
 
 constexpr int kBM = 128;
 constexpr int kBN = 256;
 constexpr int kBKBytes = 128;            // 64 bf16 per stage: one 128-byte swizzle atom
-constexpr int kStages = 4;
-constexpr int kEpiWarps = 8;
-constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kThreads = 64 + kEpiThreads;
 constexpr uint32_t kABytes = kBM * kBKBytes;   // 16 KB
 constexpr uint32_t kBBytes = kBN * kBKBytes;   // 32 KB
-constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kBoxBytes = kBM * 128;      // staging box: 128 rows x 64 bf16
-constexpr int kBoxes = kBN * 2 / 128;          // 4 boxes per tile, sent one after the other
-constexpr uint32_t kOutBytes = 2 * kBoxBytes;  // two boxes in shared memory: one is stored while the next is filled
 constexpr uint32_t kTmemCols = 512;
-constexpr size_t kSmemBytes = static_cast<size_t>(kStages) * kStageBytes + kOutBytes + 1024;
 
 struct GArgs {
     const float* bias;      // [groups, N] or nullptr
@@ -54,7 +38,6 @@ struct GArgs {
     int32_t groups, N, K;
     int64_t M;
     int32_t act;            // 0 = none, 1 = SiLU, 2 = SiLU-gated pairs (column c gates column c + 128 of its 256-column tile)
-    int32_t has_residual;
 };
 
 // silu(x) = h * tanh(h) + h, h = x / 2 (the result is rounded to bf16)
@@ -66,233 +49,12 @@ __device__ __forceinline__ float2 silu2(float2 x) {
     return __ffma2_rn(h, t, h);
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                 const __grid_constant__ CUtensorMap tmap_o, const GArgs g, const __nv_bfloat16* __restrict__ residual) {
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[kStages];
-    __shared__ uint64_t empty_bar[kStages];
-    __shared__ uint64_t tmem_full[2];
-    __shared__ uint64_t tmem_empty[2];
-    __shared__ uint32_t tmem_base_slot;
-    __shared__ __align__(16) float bias_s[kBN];
-    __shared__ int s_abort;
-
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* ring = smem;
-    uint8_t* out_s = smem + static_cast<size_t>(kStages) * kStageBytes;
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-
-    const int64_t m_tiles = (g.M + kBM - 1) / kBM;
-    const int n_tiles = g.N / kBN;
-    const int k_blocks = g.K / (kBKBytes / 2);
-    const int64_t total = static_cast<int64_t>(g.groups) * m_tiles * n_tiles;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&tmem_full[b], 1);
-            mbar_init(&tmem_empty[b], kEpiThreads);
-        }
-        s_abort = 0;
-        fence_mbar_init();
-    }
-    if (warp == 1) {
-        tmem_alloc(&tmem_base_slot, kTmemCols);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem_base = tmem_base_slot;
-
-    // tile t -> column tile (fastest), row tile, group
-    auto decode = [&](int64_t t, int& n0, int& m0, int& grp) {
-        const int n = static_cast<int>(t % n_tiles);
-        const int64_t rest = t / n_tiles;
-        n0 = n * kBN;
-        m0 = static_cast<int>(rest % m_tiles) * kBM;
-        grp = static_cast<int>(rest / m_tiles);
-    };
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
-            tma_prefetch_desc(&tmap_a);
-            tma_prefetch_desc(&tmap_w);
-            uint32_t it = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                int n0, m0, grp;
-                decode(t, n0, m0, grp);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % kStages;
-                    const uint32_t ph = (it / kStages) & 1;
-                    if (!mbar_wait_sleep(&empty_bar[s], ph ^ 1) || *reinterpret_cast<volatile int*>(&s_abort)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* dst = ring + static_cast<size_t>(s) * kStageBytes;
-                    mbar_expect_tx(&full_bar[s], kStageBytes);
-                    tma_load_3d(dst, &tmap_a, kb * kBKBytes, m0, grp, &full_bar[s]);
-                    tma_load_3d(dst + kABytes, &tmap_w, kb * kBKBytes, n0, grp, &full_bar[s]);
-                }
-            }
-            if (!ok) {
-                s_abort = 1;
-                if (g.status != nullptr) atomicExch(g.status, 1);
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc(1, 1, 0, 0, kBM, kBN);   // bf16 x bf16 -> f32, both K-major
-            const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
-            const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
-            uint32_t s = 0, ph = 0, buf = 0, aph = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-                if (!mbar_wait_sleep(&tmem_empty[buf], aph ^ 1)) { ok = false; break; }
-                const uint32_t d_tmem = tmem_base + buf * kBN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait_sleep(&full_bar[s], ph)) { ok = false; break; }
-                    tc_fence_after_sync();
-                    const uint32_t a_lo = ring_lo + s * (kStageBytes >> 4);
-                    const uint64_t da = desc0 + a_lo;
-                    const uint64_t db = desc0 + a_lo + (kABytes >> 4);
-#pragma unroll
-                    for (int k = 0; k < kBKBytes / 32; ++k) mma_f16_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                    tc_commit(&empty_bar[s]);
-                    if (++s == kStages) {
-                        s = 0;
-                        ph ^= 1;
-                    }
-                }
-                if (!ok) break;
-                tc_commit(&tmem_full[buf]);
-                aph ^= buf;
-                buf ^= 1;
-            }
-            if (!ok) {
-                s_abort = 1;
-                if (g.status != nullptr) atomicExch(g.status, 1);
-            }
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue
-        const int et = threadIdx.x - 64;          // 0..255
-        const bool gated = g.act == 2;
-        const int sub = et >> 7;                  // columns [32 sub, 32 sub + 32) of a round's 64
-        const int quarter = warp & 3;             // TMEM lanes [32 quarter, +32) are visible to this warp
-        const int row_in_tile = quarter * 32 + lane;
-        const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-        const int swz = row_in_tile & 7;
-        uint32_t tile_count = 0;
-        uint32_t round_count = 0;                 // rounds so far: staging box round_count % 2
-        bool ok = true;
-        for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++tile_count) {
-            int n0, m0, grp;
-            decode(t, n0, m0, grp);
-            const uint32_t buf = tile_count & 1;
-            const uint32_t aph = (tile_count >> 1) & 1;
-            bias_s[et] = g.bias != nullptr ? g.bias[static_cast<int64_t>(grp) * g.N + n0 + et] : 0.f;
-            // residual pieces of round r: this thread's row, 32 columns = four 16-byte loads, one round ahead
-            const int64_t row = static_cast<int64_t>(m0) + row_in_tile;
-            const bool has_res = residual != nullptr && row < g.M;
-            const uint4* res_row = reinterpret_cast<const uint4*>(
-                residual + (static_cast<int64_t>(grp) * g.M + (has_res ? row : 0)) * g.N + n0 + sub * 32);
-            uint4 res_cur[4], res_next[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) res_cur[q] = has_res ? res_row[q] : make_uint4(0u, 0u, 0u, 0u);   // plain loads: `out` may be this tensor
-            // A thread whose wait gives up stops waiting but keeps walking the tile list, so that it still meets
-            // every named barrier the other epilogue threads sit in; what it writes is garbage and the status
-            // word says so.
-            if (ok && !mbar_wait_sleep(&tmem_full[buf], aph)) ok = false;
-            tc_fence_after_sync();
-            const int n_rounds = gated ? kBoxes / 2 : kBoxes;   // gated: 128 gate + 128 value columns -> 128 outputs
-#pragma unroll 1
-            for (int r = 0; r < n_rounds; ++r, ++round_count) {
-                const int col = r * 64 + sub * 32;       // first of this thread's 32 columns in the tile
-                uint8_t* box = out_s + (round_count & 1) * kBoxBytes;
-                if (r + 1 < n_rounds) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) res_next[q] = has_res ? res_row[(r + 1) * 8 + q] : make_uint4(0u, 0u, 0u, 0u);
-                }
-                uint32_t acc[32], accv[32];
-                tmem_ld_2x16(tmem_base + buf * kBN + lane_addr + col, acc);
-                if (gated) tmem_ld_2x16(tmem_base + buf * kBN + lane_addr + 128 + col, accv);
-                if (et == 0) bulk_wait_read<1>();   // the store that used this box two rounds ago has read it
-                asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-                tc_wait_ld(acc);
-                if (gated) tc_wait_ld(accv);   // no second wait in hardware terms; it keeps the uses of accv below the wait
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 b0 = *reinterpret_cast<const float4*>(bias_s + col + q * 8);
-                    const float4 b1 = *reinterpret_cast<const float4*>(bias_s + col + q * 8 + 4);
-                    float2 v[4];
-                    v[0] = __fadd2_rn(make_float2(__uint_as_float(acc[8 * q + 0]), __uint_as_float(acc[8 * q + 1])), make_float2(b0.x, b0.y));
-                    v[1] = __fadd2_rn(make_float2(__uint_as_float(acc[8 * q + 2]), __uint_as_float(acc[8 * q + 3])), make_float2(b0.z, b0.w));
-                    v[2] = __fadd2_rn(make_float2(__uint_as_float(acc[8 * q + 4]), __uint_as_float(acc[8 * q + 5])), make_float2(b1.x, b1.y));
-                    v[3] = __fadd2_rn(make_float2(__uint_as_float(acc[8 * q + 6]), __uint_as_float(acc[8 * q + 7])), make_float2(b1.z, b1.w));
-                    if (g.act >= 1) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = silu2(v[e]);
-                    }
-                    if (gated) {   // silu(gate) * value, the value columns sit 128 further right in the accumulator
-                        const float4 c0 = *reinterpret_cast<const float4*>(bias_s + 128 + col + q * 8);
-                        const float4 c1 = *reinterpret_cast<const float4*>(bias_s + 128 + col + q * 8 + 4);
-                        v[0] = __fmul2_rn(v[0], __fadd2_rn(make_float2(__uint_as_float(accv[8 * q + 0]), __uint_as_float(accv[8 * q + 1])), make_float2(c0.x, c0.y)));
-                        v[1] = __fmul2_rn(v[1], __fadd2_rn(make_float2(__uint_as_float(accv[8 * q + 2]), __uint_as_float(accv[8 * q + 3])), make_float2(c0.z, c0.w)));
-                        v[2] = __fmul2_rn(v[2], __fadd2_rn(make_float2(__uint_as_float(accv[8 * q + 4]), __uint_as_float(accv[8 * q + 5])), make_float2(c1.x, c1.y)));
-                        v[3] = __fmul2_rn(v[3], __fadd2_rn(make_float2(__uint_as_float(accv[8 * q + 6]), __uint_as_float(accv[8 * q + 7])), make_float2(c1.z, c1.w)));
-                    }
-                    if (residual != nullptr) {
-                        float2 rr[4];
-                        Vec16<__nv_bfloat16>::unpack2(res_cur[q], rr);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = __fadd2_rn(v[e], rr[e]);
-                    }
-                    *reinterpret_cast<uint4*>(box + row_in_tile * 128 + (((sub * 4 + q) ^ swz) << 4)) = Vec16<__nv_bfloat16>::pack2(v);
-                }
-                if (r == n_rounds - 1) {   // every column of this buffer has been read: the tensor cores may reuse it
-                    tc_fence_before_sync();
-                    mbar_arrive(&tmem_empty[buf]);
-                }
-                fence_proxy_async_smem();
-                asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-                if (et == 0) {
-                    tma_store_3d(&tmap_o, box, (gated ? n0 : 2 * n0) + r * 128, m0, grp);
-                    bulk_commit();
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) res_cur[q] = res_next[q];
-            }
-        }
-        if (et == 0) bulk_wait<0>();
-        if (!ok) {
-            s_abort = 1;
-            if (g.status != nullptr) atomicExch(g.status, 1);
-        }
-    }
-
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
-    }
-}
-
 // ------------------------------------------------------------------------------------------------
-// CTA-pair variant (cluster of two CTAs, tcgen05 cta_group::2).  A pair owns a 256 x 256 output tile: each CTA
+// Cluster of two CTAs, tcgen05 cta_group::2.  A pair owns a 256 x 256 output tile: each CTA
 // loads its own 128 rows of A and one half (128 rows) of the weight tile, the leader (even rank) issues
 // 256 x 256 x 16 MMAs that read A from each CTA's own shared memory and the weight halves from both, and each
-// CTA's TMEM receives its 128 rows.  A stage is then 32 KB per CTA for the same 512 cycles of tensor-core time,
-// so six stages fit where the single-CTA kernel has four: the ring holds 3072 cycles of work, more than the
+// CTA's TMEM receives its 128 rows.  A stage is then 32 KB per CTA for 512 cycles of tensor-core time (a single CTA
+// on 128 x 256 needs 48 KB), so six stages fit: the ring holds 3072 cycles of work, more than the
 // round trip that the K loop otherwise waits for.  Barriers: the "full" barriers live in the leader and count
 // the bytes of both CTAs' loads; "empty" and "accumulator full" are signalled in both CTAs by multicast
 // commits; "accumulator empty" collects one arrival per epilogue warp of both CTAs in the leader.
@@ -396,6 +158,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     cluster_sync_all();                          // both CTAs' barriers exist before anything is signalled remotely
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    chain_release();   // not before every CTA holds its tensor memory (see launch_chained)
+    chain_wait();
 
     auto decode = [&](int64_t t, int& n0, int& m0, int& grp) {
         const int n = static_cast<int>(t % n_tiles);
@@ -646,10 +410,23 @@ extern "C" int tb200_gemm_bf16_grouped(const void* a, const void* w, const float
         return TB200_ERR_ALIGN;
     if (M > 0x7FFFFF00ll || static_cast<int64_t>(groups) * ((M + kBM - 1) / kBM) * (N / kBN) > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    CUtensorMap ta, tw, to;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const DeviceInfo& dev = device_info();
+    // Few rows per group: streaming the weights is what takes the time.  Measured per launch, gemm_small / gemm_narrow /
+    // pair tiles, in us: 9 x (1536 x 512) at M = 8: 5.0 / 5.8 / 9.0, M = 16: 6.0 / 5.8 / 9.0, M = 32: 8.6 / 6.1 / 9.4, M = 64: - / 6.8 / 9.5,
+    // M = 128: - / 8.3 / 9.6, M = 192: - / 10.8 / 10.2; 9 x (512 x 2048) at M = 32: 7.7 / 10.8 / 18, M = 128: - / 19.3 / 20; 1 x (512 x 512)
+    // at M = 32: 3.0 / 5.5 / 9.0.  gemm_small re-reads the activations in every CTA of 16 columns, so the more rows, the fewer
+    // of its CTAs may there be.
+    const int64_t small_ctas = static_cast<int64_t>(groups) * (N / 16);
+    const int64_t small_most = M <= 8 ? INT64_MAX : (M <= 16 ? 6ll * dev.sm_count : (M <= 32 && K <= 2048 ? 2ll * dev.sm_count : 0));
+    if (small_ctas <= small_most && groups <= 65535)
+        return gemm_small(a, w, bias, residual, out, groups, static_cast<int>(M), N, K, act, st);
+    if (M <= 128 && groups <= 65535 && act != 2)
+        return gemm_narrow(a, w, bias, residual, out, groups, static_cast<int>(M), N, K, act, status_word, st);
+    CUtensorMap ta, twh, tow;
     const uint64_t ug = static_cast<uint64_t>(groups), um = static_cast<uint64_t>(M);
-    if (!make_tmap3(&ta, a, 2ull * K, um, ug, kBM) || !make_tmap3(&tw, w, 2ull * K, static_cast<uint64_t>(N), ug, kBN) ||
-        !make_tmap3(&to, out, act == 2 ? static_cast<uint64_t>(N) : 2ull * N, um, ug, kBM))
+    if (!make_tmap3(&ta, a, 2ull * K, um, ug, kBM) || !make_tmap3(&twh, w, 2ull * K, static_cast<uint64_t>(N), ug, kBN / 2) ||
+        !make_tmap3(&tow, out, act == 2 ? static_cast<uint64_t>(N) : 2ull * N, um, ug, 32))
         return TB200_ERR_DRIVER;
     GArgs g{};
     g.bias = bias;
@@ -659,45 +436,24 @@ extern "C" int tb200_gemm_bf16_grouped(const void* a, const void* w, const float
     g.K = K;
     g.M = M;
     g.act = act;
-    g.has_residual = residual != nullptr ? 1 : 0;
-    const DeviceInfo& dev = device_info();
-    static bool attr_set[64] = {};
-    if (!attr_set[dev.index]) {
-        cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes));
-        attr_set[dev.index] = true;
+    static bool pair_attr[64] = {};
+    if (!pair_attr[dev.index]) {
+        cudaFuncSetAttribute(gemm_bf16_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
+        cudaFuncSetAttribute(gemm_bf16_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
+        cudaFuncSetAttribute(gemm_bf16_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
+        pair_attr[dev.index] = true;
     }
-    // CTA pairs by default; TB200_GEMM_PAIR=0 in the environment selects the single-CTA kernel (for comparison)
-    static const bool use_pair = []() { const char* e = getenv("TB200_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
-    if (use_pair && M > kBM) {
-        static bool pair_attr[64] = {};
-        if (!pair_attr[dev.index]) {
-            cudaFuncSetAttribute(gemm_bf16_pair_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
-            cudaFuncSetAttribute(gemm_bf16_pair_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
-            cudaFuncSetAttribute(gemm_bf16_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemPBytes));
-            pair_attr[dev.index] = true;
-        }
-        CUtensorMap twh, tow;
-        if (!make_tmap3(&twh, w, 2ull * K, static_cast<uint64_t>(N), ug, kBN / 2)) return TB200_ERR_DRIVER;
-        if (!make_tmap3(&tow, out, act == 2 ? static_cast<uint64_t>(N) : 2ull * N, um, ug, 32)) return TB200_ERR_DRIVER;
-        const int64_t tiles = static_cast<int64_t>(groups) * ((M + 2 * kBM - 1) / (2 * kBM)) * (N / kBN);
-        int64_t pairs = dev.sm_count / 2;
-        if (pairs > tiles) pairs = tiles;
-        const unsigned grid = static_cast<unsigned>(2 * pairs);
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(residual);
-        if (act == 2)
-            gemm_bf16_pair_kernel<true, false><<<grid, kThreadsP, kSmemPBytes, st>>>(ta, twh, tow, g, res);
-        else if (residual != nullptr)
-            gemm_bf16_pair_kernel<false, true><<<grid, kThreadsP, kSmemPBytes, st>>>(ta, twh, tow, g, res);
-        else
-            gemm_bf16_pair_kernel<false, false><<<grid, kThreadsP, kSmemPBytes, st>>>(ta, twh, tow, g, res);
-        count_launch();
-        return launch_status();
-    }
-    const int64_t total = static_cast<int64_t>(groups) * ((M + kBM - 1) / kBM) * (N / kBN);
-    const int64_t grid = total < dev.sm_count ? total : dev.sm_count;
-    gemm_bf16_kernel<<<static_cast<unsigned>(grid), kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(
-        ta, tw, to, g, static_cast<const __nv_bfloat16*>(residual));
+    const int64_t tiles = static_cast<int64_t>(groups) * ((M + 2 * kBM - 1) / (2 * kBM)) * (N / kBN);
+    int64_t pairs = dev.sm_count / 2;
+    if (pairs > tiles) pairs = tiles;
+    const unsigned grid = static_cast<unsigned>(2 * pairs);
+    const __nv_bfloat16* res = static_cast<const __nv_bfloat16*>(residual);
+    if (act == 2)
+        launch_chained(gemm_bf16_pair_kernel<true, false>, grid, kThreadsP, kSmemPBytes, st, ta, twh, tow, g, res);
+    else if (residual != nullptr)
+        launch_chained(gemm_bf16_pair_kernel<false, true>, grid, kThreadsP, kSmemPBytes, st, ta, twh, tow, g, res);
+    else
+        launch_chained(gemm_bf16_pair_kernel<false, false>, grid, kThreadsP, kSmemPBytes, st, ta, twh, tow, g, res);
     count_launch();
     return launch_status();
 }

@@ -76,6 +76,8 @@ __device__ __forceinline__ RowShape row_shape(const uint8_t* row, int n, int lan
 __global__ void __launch_bounds__(kThreads)
 mask_plan_kernel(const uint8_t* __restrict__ mask, int64_t sb, int64_t sh, int64_t sq, int heads, int lq, int lk,
                  int32_t* __restrict__ lens, int4* __restrict__ verdict) {
+    chain_release();
+    chain_wait();
     __shared__ RowShape s_row[3];   // row 0, the last row, the last row that sees key 0
     __shared__ int s_last0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -153,7 +155,7 @@ extern "C" int tb200_mask_plan(const uint8_t* mask, int64_t stride_b, int64_t st
     if (mask == nullptr || lens == nullptr || verdict == nullptr) return TB200_ERR_NULL;
     if (!aligned16(verdict)) return TB200_ERR_ALIGN;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    mask_plan_kernel<<<B, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(mask, stride_b, stride_h, stride_q, stride_h == 0 ? 1 : H, Lq,
+    launch_chained(mask_plan_kernel, B, kThreads, 0, static_cast<cudaStream_t>(stream), mask, stride_b, stride_h, stride_q, stride_h == 0 ? 1 : H, Lq,
                                                                             Lk, lens, reinterpret_cast<int4*>(verdict));
     count_launch();
     return launch_status();

@@ -103,6 +103,8 @@ template <typename T, bool LAYER, int CPL, int RU, int PRE, bool POST, bool EXAC
 __global__ void __launch_bounds__(kMaxThreads, 3)
 norm_tma_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
                 int64_t rows, int cols, float eps, int lanes_per_row, int* __restrict__ status, const PostArgs post) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t full_bar[kWarps][kStages];
@@ -409,6 +411,8 @@ template <typename T, bool LAYER, int PRE>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_rowwarp_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
                     T* __restrict__ y, int64_t rows, int cols, float eps) {
+    chain_release();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warp = (static_cast<int64_t>(blockIdx.x) * kMaxThreads + threadIdx.x) >> 5;
     const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * kMaxThreads) >> 5;
@@ -454,6 +458,8 @@ template <typename T, bool LAYER, int PRE>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_rowwarp_vec_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
                         T* __restrict__ y, int64_t rows, int cols, int64_t y_stride, float eps) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
@@ -552,7 +558,7 @@ int launch_tma_exact(const void* x, const void* gamma, const void* beta, void* y
     const int64_t useful = (rows + static_cast<int64_t>(tile_rows) * kWarps - 1) / (static_cast<int64_t>(tile_rows) * kWarps);
     if (grid > useful) grid = useful;
     if (grid < 1) grid = 1;
-    norm_tma_kernel<T, LAYER, CPL, RU, PRE, POST, EXACT><<<static_cast<unsigned>(grid), kMaxThreads, smem, stream>>>(
+    launch_chained(norm_tma_kernel<T, LAYER, CPL, RU, PRE, POST, EXACT>, static_cast<unsigned>(grid), kMaxThreads, smem, stream,
         static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows,
         cols, eps, lanes_per_row, nullptr, post);
     count_launch();
@@ -582,7 +588,7 @@ int launch_rowwarp_vec(const void* x, const void* gamma, const void* beta, void*
     int64_t blocks = (rows + (kMaxThreads / 32) - 1) / (kMaxThreads / 32);
     const int64_t cap = static_cast<int64_t>(dev.sm_count) * (smem > 56 * 1024 ? 2 : (smem > 36 * 1024 ? 4 : 6));
     if (blocks > cap) blocks = cap;
-    norm_rowwarp_vec_kernel<T, LAYER, PRE><<<static_cast<unsigned>(blocks), kMaxThreads, smem, stream>>>(
+    launch_chained(norm_rowwarp_vec_kernel<T, LAYER, PRE>, static_cast<unsigned>(blocks), kMaxThreads, smem, stream,
         static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows, cols, y_stride, eps);
     count_launch();
     return launch_status();
@@ -613,7 +619,7 @@ int norm_dispatch(const void* x, const void* gamma, const void* beta, void* y, i
     const bool wide_vec = (cols % N == 0) && aligned16(x) && aligned16(y) && aligned16(gamma) &&
                           ((!LAYER && PRE != kPreBias) || aligned16(beta)) && (cols / N) <= 640;
     if (wide_vec) return launch_rowwarp_vec<T, LAYER, PRE>(x, gamma, beta, y, rows, cols, cols, eps, stream);
-    norm_rowwarp_kernel<T, LAYER, PRE><<<static_cast<unsigned>(blocks), kMaxThreads, 0, stream>>>(
+    launch_chained(norm_rowwarp_kernel<T, LAYER, PRE>, static_cast<unsigned>(blocks), kMaxThreads, 0, stream,
         static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(beta), static_cast<T*>(y), rows,
         cols, eps);
     count_launch();

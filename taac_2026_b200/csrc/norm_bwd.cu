@@ -40,6 +40,8 @@ template <typename T, int CPL, int G, bool LAYER>
 __global__ void __launch_bounds__(kThreads)
 norm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ dy, T* __restrict__ dx,
                 float* __restrict__ partial_w, float* __restrict__ partial_b, int64_t rows, int cols, float eps) {
+    chain_release();
+    chain_wait();
     constexpr int N = Vec16<T>::N;           // elements per 16-byte piece
     constexpr int RPW = 32 / G;              // rows a warp handles at a time
     extern __shared__ float red[];           // [kWarps][cols] (x 2 for LayerNorm)
@@ -196,6 +198,8 @@ template <typename T>
 __global__ void __launch_bounds__(1024)
 norm_bwd_reduce_kernel(const float* __restrict__ partial_w, const float* __restrict__ partial_b, T* __restrict__ dgamma,
                        T* __restrict__ dbeta, int n_partials, int cols) {
+    chain_release();
+    chain_wait();
     __shared__ float sw[32][33], sb[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + tx;
@@ -240,7 +244,7 @@ int launch_one(const void* x, const void* gamma, const void* dy, void* dx, float
         cudaFuncSetAttribute(norm_bwd_kernel<T, CPL, G, LAYER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kWarps * 1024 * static_cast<int>(sizeof(float)));
         attr_set[dev.index] = true;
     }
-    norm_bwd_kernel<T, CPL, G, LAYER><<<grid, kThreads, smem, stream>>>(
+    launch_chained(norm_bwd_kernel<T, CPL, G, LAYER>, grid, kThreads, smem, stream,
         static_cast<const T*>(x), static_cast<const T*>(gamma), static_cast<const T*>(dy), static_cast<T*>(dx), pw, pb, rows, cols, eps);
     count_launch();
     return launch_status();
@@ -307,13 +311,13 @@ int norm_bwd(const void* x, const void* gamma, const void* dy, void* dx, void* d
     const int rgrid = (cols + 31) / 32;
     switch (dtype) {
         case TB200_F32:
-            norm_bwd_reduce_kernel<float><<<rgrid, 1024, 0, s>>>(pw, pb, static_cast<float*>(dgamma), static_cast<float*>(dbeta), grid, cols);
+            launch_chained(norm_bwd_reduce_kernel<float>, rgrid, 1024, 0, s, pw, pb, static_cast<float*>(dgamma), static_cast<float*>(dbeta), grid, cols);
             break;
         case TB200_F16:
-            norm_bwd_reduce_kernel<__half><<<rgrid, 1024, 0, s>>>(pw, pb, static_cast<__half*>(dgamma), static_cast<__half*>(dbeta), grid, cols);
+            launch_chained(norm_bwd_reduce_kernel<__half>, rgrid, 1024, 0, s, pw, pb, static_cast<__half*>(dgamma), static_cast<__half*>(dbeta), grid, cols);
             break;
         default:
-            norm_bwd_reduce_kernel<__nv_bfloat16><<<rgrid, 1024, 0, s>>>(pw, pb, static_cast<__nv_bfloat16*>(dgamma),
+            launch_chained(norm_bwd_reduce_kernel<__nv_bfloat16>, rgrid, 1024, 0, s, pw, pb, static_cast<__nv_bfloat16*>(dgamma),
                                                                           static_cast<__nv_bfloat16*>(dbeta), grid, cols);
             break;
     }

@@ -52,6 +52,8 @@ seqprep_kernel(const int64_t* __restrict__ values, const int64_t* __restrict__ l
                const int64_t* __restrict__ timestamps, const int64_t* __restrict__ request_ts, int n_feat, int max_len,
                int table_size, int64_t* __restrict__ out_len, int32_t* __restrict__ out_src,
                float* __restrict__ out_stats) {
+    chain_release();
+    chain_wait();
     extern __shared__ int32_t smem_i[];
     int32_t* rep = smem_i;                    // [table_size] representative position of the slot, -1 = empty
     int32_t* last = rep + table_size;         // [table_size] largest position that hit the slot
@@ -178,6 +180,8 @@ token_index_kernel(const int64_t* __restrict__ values, const int64_t* __restrict
                    const int64_t* __restrict__ start, const int64_t* __restrict__ edges, int n_edges,
                    const int64_t* __restrict__ hash_buckets, int n_feat, int max_len, int64_t total_rows,
                    int64_t* __restrict__ ids_out, int64_t* __restrict__ pos_out, int64_t* __restrict__ bucket_out) {
+    chain_release();
+    chain_wait();
     const int64_t b = blockIdx.x;
     const int64_t row0 = cu_rows[b];
     const int64_t n_rows = cu_rows[b + 1] - row0;
@@ -241,6 +245,8 @@ pyramid_plan_kernel(const int64_t* __restrict__ lengths, int batch, int max_len,
                     int64_t* __restrict__ start, int64_t* __restrict__ n0_out, int64_t* __restrict__ counts,
                     int64_t* __restrict__ cu, int32_t* __restrict__ cu32, int64_t* __restrict__ meta,
                     int64_t* __restrict__ ns_rows0, int64_t* __restrict__ ns_rows) {
+    chain_release();
+    chain_wait();
     __shared__ int64_t warp_sum[32];
     __shared__ int64_t warp_max[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -313,6 +319,8 @@ __global__ void __launch_bounds__(128)
 pyramid_kept_rows_kernel(const int64_t* __restrict__ cu0, const int64_t* __restrict__ cu1, const int64_t* __restrict__ counts0,
                          const int64_t* __restrict__ counts1, int ns, int64_t* __restrict__ src, int64_t* __restrict__ ns_rows1,
                          int32_t* __restrict__ row_dst) {
+    chain_release();
+    chain_wait();
     const int b = blockIdx.x;
     const int64_t base0 = cu0[b], base1 = cu1[b];
     const int64_t c0 = counts0[b], c1 = counts1[b];
@@ -352,7 +360,7 @@ extern "C" int tb200_pyramid_plan_rows(const int64_t* lengths, int32_t batch, in
     // the int32 offsets must hold the largest total: every sample at most widths[0] + ns rows
     if ((static_cast<int64_t>(widths[0]) + ns) * batch > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    pyramid_plan_kernel<<<static_cast<unsigned>(n_layers + 1), kPlanThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(pyramid_plan_kernel, static_cast<unsigned>(n_layers + 1), kPlanThreads, 0, static_cast<cudaStream_t>(stream),
         lengths, batch, max_len, w, ns, start, n0, counts, cu, cu32, meta, ns_rows0, ns_rows);
     count_launch();
     return launch_status();
@@ -368,7 +376,7 @@ extern "C" int tb200_pyramid_kept_rows(const int64_t* cu0, const int64_t* cu1, c
         (ns > 0 && ns_rows1 == nullptr))
         return TB200_ERR_NULL;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    pyramid_kept_rows_kernel<<<static_cast<unsigned>(batch), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(pyramid_kept_rows_kernel, static_cast<unsigned>(batch), 128, 0, static_cast<cudaStream_t>(stream),
         cu0, cu1, counts0, counts1, ns, src, ns_rows1, row_dst);
     count_launch();
     return launch_status();
@@ -394,7 +402,7 @@ extern "C" int tb200_sequence_prepare(const int64_t* values, const int64_t* leng
         cudaFuncSetAttribute(seqprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr_set[dev.index] = true;
     }
-    seqprep_kernel<<<static_cast<unsigned>(batch), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(seqprep_kernel, static_cast<unsigned>(batch), kThreads, smem, static_cast<cudaStream_t>(stream),
         values, lengths, timestamps, request_ts, n_feat, max_len, table, out_len, out_src, out_stats);
     count_launch();
     return launch_status();
@@ -415,7 +423,7 @@ extern "C" int tb200_packed_token_index(const int64_t* values, const int64_t* ti
     if (bucket_out != nullptr && (timestamps == nullptr || edges == nullptr || n_edges < 1)) return TB200_ERR_NULL;
     if (batch > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    token_index_kernel<<<static_cast<unsigned>(batch), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_chained(token_index_kernel, static_cast<unsigned>(batch), 128, 0, static_cast<cudaStream_t>(stream),
         values, timestamps, request_ts, src, cu_rows, seq_count, start, edges, n_edges, hash_buckets, n_feat, max_len,
         total_rows, ids_out, pos_out, bucket_out);
     count_launch();

@@ -38,6 +38,31 @@ struct DeviceInfo {
 // Cached per device; the first call on a device queries the runtime.
 const DeviceInfo& device_info();
 
+// ---- programmatic dependent launch -----------------------------------------------------------
+// A kernel launched with launch_chained may start while its predecessor in the stream is still running; it must call
+// chain_wait() in every CTA before it touches memory that the predecessor reads or writes (prefetches into the L2 are
+// fine), which returns once the predecessor has finished.  chain_release() lets the successor start: called at the top
+// it hides the successor's launch latency and set-up (2 to 4 us of a small kernel) behind this kernel.  A kernel that
+// allocates tensor memory calls it only after the allocation: a successor's CTA on the same SM could otherwise take the
+// columns first and then wait for this kernel, which would wait for the columns.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // an error stays for launch_status()
+}
+
 // 8 packed 16-bit values or 4 packed fp32 <-> float registers -----------------
 template <typename T>
 struct Vec16;  // one 16-byte chunk

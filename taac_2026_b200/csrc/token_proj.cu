@@ -209,6 +209,8 @@ token_project_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     cluster_sync_all();                          // the peer's shared memory exists before anything is written into it
     tc_fence_after_sync();
     const uint32_t tmem_base = tmem_base_slot;
+    chain_release();   // not before every CTA holds its tensor memory (see launch_chained)
+    chain_wait();
 
     // W: rows [NC rank, NC rank + NC) of the weight, one box per K block, resident for the kernel's life
     if (threadIdx.x == 0) {
@@ -553,7 +555,7 @@ int launch(const CUtensorMap& tw, const CUtensorMap& to, const TPArgs& g, cudaSt
     const int64_t tiles = (g.rows + kRows - 1) / kRows;
     int64_t pairs = dev.sm_count / 2;
     if (pairs > tiles) pairs = tiles;
-    token_project_kernel<N_COLS><<<static_cast<unsigned>(2 * pairs), kThreads, smem, stream>>>(tw, to, g);
+    launch_chained(token_project_kernel<N_COLS>, static_cast<unsigned>(2 * pairs), kThreads, smem, stream, tw, to, g);
     count_launch();
     return launch_status();
 }

@@ -268,6 +268,10 @@ int tb200_gather_rows(const void* table, int64_t vocab_rows, int32_t dim, const 
 int tb200_scatter_rows(void* dst, int64_t dst_rows, int64_t dst_stride, int32_t dst_col0, const int64_t* ids,
                        const void* src, int64_t n, int32_t dim, const void* bias, int64_t rows_per_group,
                        const void* residual, int64_t residual_stride, int dtype, void* stream);
+/* The same with source rows src_stride elements apart. */
+int tb200_scatter_rows_strided(void* dst, int64_t dst_rows, int64_t dst_stride, int32_t dst_col0, const int64_t* ids, const void* src,
+                               int64_t src_stride, int64_t n, int32_t dim, const void* bias, int64_t rows_per_group, const void* residual,
+                               int64_t residual_stride, int dtype, void* stream);
 
 /* x[i, :] = x[i, :] + table_a[ids_a[i], :], then (table_b != NULL) + table_b[ids_b[i], :], in place; ids are
  * clamped into their table and every sum is rounded to `dtype` like a tensor addition of its own.  The
@@ -326,6 +330,12 @@ int tb200_attn_fwd(const void* q, const void* k, const void* v, void* o, int32_t
                    int32_t Lk, int32_t D, const int64_t* strides, const int32_t* seq_len, const int32_t* cu_rows,
                    const int32_t* cu_rows_q, const uint8_t* key_valid, int32_t ns_start, int32_t causal, int32_t padded_query_self, float scale, int dtype,
                    int32_t kernel, int64_t total_rows, int32_t* status_word, void* stream);
+
+/* Causal attention of the last n_q rows of every sample over all its rows, head_dim 64, fp16 or bf16: k and v packed by cu_rows (at most
+ * max_rows rows per sample, at least n_q), query j of sample b at q + b strides[0] + j strides[2] (+ head strides[1]) and its output
+ * likewise, so that both may lie token-major.  strides: the 12 values of tb200_attn_fwd (the batch strides of k and v are not used). */
+int tb200_attn_last_rows_fwd(const void* q, const void* k, const void* v, void* o, int32_t B, int32_t H, int32_t n_q, int32_t max_rows,
+                             const int64_t* strides, const int32_t* cu_rows, float scale, int dtype, void* stream);
 
 /* Describes bool masks [B, H, Lq, Lk] (one byte per element, strides in bytes, unit stride along the keys; stride_h 0 = one mask
  * for all heads) by lengths, as `_plan_tilelang_flash_attention_mask` does (accelerators/attention/flash_attention.py:149-198)
@@ -453,8 +463,8 @@ int tb200_pyramid_kept_rows(const int64_t* cu0, const int64_t* cu1, const int64_
 
 /* ---- row kernels around the engine's blocks ---------------------------------------------------
  * out[r] = LayerNorm(SiLU(w x_r + bias)) gamma + beta in fp32, x_r = [values[r, :n], mask[r, :n] != 0 as 1 / 0 (mask may be NULL)]:
- * `DenseTokenProjector.forward` (modeling/tokenizers.py:101-111) and the statistics projector.  w [d, in_dim] fp32 with in_dim = n or
- * 2 n; out rows out_stride elements apart, of type dtype.  8 (in_dim + d) floats must fit 48 KB. */
+ * `DenseTokenProjector.forward` (modeling/tokenizers.py:101-111) and the statistics projector.  w [in_dim, d] fp32 (the layer's weight transposed)
+ * with in_dim = n or 2 n; out rows out_stride elements apart, of type dtype.  8 (in_dim + d) floats must fit 48 KB. */
 int tb200_small_token_fwd(const float* values, int32_t n, int64_t value_stride, const uint8_t* mask, int64_t mask_stride, int32_t in_dim,
                           const float* w, const float* bias, const float* gamma, const float* beta, void* out, int64_t out_stride,
                           int64_t rows, int32_t d, float eps, int dtype, void* stream);
@@ -494,6 +504,13 @@ int tb200_head_fwd(const void* h, const float* w, const float* bias, float* logi
 int tb200_gemm_bf16_grouped(const void* a, const void* w, const float* bias, const void* residual, void* out,
                             int32_t groups, int64_t M, int32_t N, int32_t K, int32_t act, int32_t* status_word,
                             void* stream);
+
+/* The same for few rows per group (TB200_ERR_UNSUPPORTED beyond about 32: use the call above), act 0 or 1, with two options: one weight
+ * [N, K] and bias [N] for all groups (shared_w), and rmsnorm(a + norm_bias) norm_gamma (norm_gamma [K] bf16, norm_bias NULL or [K] bf16)
+ * as the activations, rounded to bf16 as tb200_rmsnorm_bias_fwd would store them. */
+int tb200_gemm_bf16_few_rows(const void* a, const void* w, const float* bias, const void* residual, void* out, int32_t groups, int64_t M,
+                             int32_t N, int32_t K, int32_t act, int32_t shared_w, const void* norm_gamma, const void* norm_bias,
+                             float norm_eps, void* stream);
 
 /* ---- whole FFN without any allocation --------------------------------------------------------
  * No counterpart in the reference (which has neither an FP8 path nor a C interface).

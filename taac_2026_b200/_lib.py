@@ -55,6 +55,8 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_pool_rows_fwd": (_INT, [_P, _P, _P, _I64, _I32, _I32, _P, _F, _P, _P, _INT, _P]),
     "tb200_join_summaries": (_INT, [_P, _P, _P, _P, _I64, _I32, _INT, _P]),
     "tb200_head_fwd": (_INT, [_P, _P, _P, _P, _P, _I64, _I32, _I32, _INT, _P]),
+    "tb200_gemm_bf16_few_rows": (_INT, [_P, _P, _P, _P, _P, _I32, _I64, _I32, _I32, _I32, _I32, _P, _P, _F, _P]),
+    "tb200_attn_last_rows_fwd": (_INT, [_P, _P, _P, _P, _I32, _I32, _I32, _I32, _P, _P, _F, _INT, _P]),
     "tb200_mask_plan": (_INT, [_P, _I64, _I64, _I64, _I32, _I32, _I32, _I32, _P, _P, _P]),
     "tb200_attn_bwd_workspace_bytes": (_I64, [_I32, _I32, _I32]),
     "tb200_attn_bwd": (_INT, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I32, _I32, _I32, _I32, _I32, _P, _P, _P, _I32, _I32, _I32,
@@ -87,6 +89,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_ffn_fp8_static_status": (_INT, [_P, _P]),
     "tb200_sequence_prepare": (_INT, [_P, _P, _P, _P, _I64, _I32, _I32, _P, _P, _P, _P]),
     "tb200_scatter_rows": (_INT, [_P, _I64, _I64, _I32, _P, _P, _I64, _I32, _P, _I64, _P, _I64, _INT, _P]),
+    "tb200_scatter_rows_strided": (_INT, [_P, _I64, _I64, _I32, _P, _P, _I64, _I64, _I32, _P, _I64, _P, _I64, _INT, _P]),
     "tb200_gather_rows": (_INT, [_P, _I64, _I32, _P, _INT, _I64, _I64, _I64, _P, _I64, _I32, _INT, _P]),
 }
 

@@ -82,3 +82,30 @@ extern "C" int tb200_attn_fwd(const void* q, const void* k, const void* v, void*
         return attn_tc05_forward(a, Lq, total_rows, status_word, s);
     return attn_mma_forward(a, D, dtype, Lq, s);
 }
+
+extern "C" int tb200_attn_last_rows_fwd(const void* q, const void* k, const void* v, void* o, int32_t B, int32_t H, int32_t n_q, int32_t max_rows,
+                                        const int64_t* strides, const int32_t* cu_rows, float scale, int dtype, void* stream) {
+    using namespace tb200;
+    if (B < 0 || H < 1 || n_q < 1 || max_rows < 0) return TB200_ERR_SHAPE;
+    if (B == 0 || max_rows == 0) return TB200_OK;
+    if (q == nullptr || k == nullptr || v == nullptr || o == nullptr || strides == nullptr || cu_rows == nullptr) return TB200_ERR_NULL;
+    if (dtype != TB200_BF16 && dtype != TB200_F16) return TB200_ERR_DTYPE;
+    if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return TB200_ERR_ALIGN;
+    for (int i = 0; i < 12; ++i)
+        if (strides[i] % 8 != 0) return TB200_ERR_ALIGN;
+    if (B > 65535) return TB200_ERR_UNSUPPORTED;
+    if (!device_info().valid) return TB200_ERR_DEVICE;
+    AttnArgs a{};
+    a.q = q; a.k = k; a.v = v; a.o = o;
+    a.q_sb = strides[0]; a.q_sh = strides[1]; a.q_sl = strides[2];
+    a.k_sb = strides[3]; a.k_sh = strides[4]; a.k_sl = strides[5];
+    a.v_sb = strides[6]; a.v_sh = strides[7]; a.v_sl = strides[8];
+    a.o_sb = strides[9]; a.o_sh = strides[10]; a.o_sl = strides[11];
+    a.cu_rows = cu_rows;
+    a.q_fixed = n_q;
+    a.B = B; a.H = H; a.Lq = n_q; a.Lk = max_rows;
+    a.ns_start = max_rows;
+    a.causal = 1;
+    a.scale_log2 = scale * 1.4426950408889634f;
+    return attn_fewq_forward(a, dtype, static_cast<cudaStream_t>(stream));
+}

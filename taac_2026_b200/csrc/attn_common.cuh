@@ -23,6 +23,9 @@ struct AttnArgs {
     // cu_rows_q[b+1] - cu_rows_q[b] queries, the LAST rows of its cu_rows[b+1] - cu_rows[b] keys), and the
     // causal rule is aligned at the end: query j of lq sees keys <= j + (lk - lq).
     const int32_t* cu_rows_q;
+    // > 0 (packed keys only, without cu_rows_q): every sample has exactly this many queries, its last rows; query j of sample b is
+    // row q + b q_sb + j q_sl, its output o + b o_sb + j o_sl (so they may lie token-major).
+    int32_t q_fixed;
     const uint8_t* key_valid;  // [B, Lk] bytes (0 = padding) or nullptr; replaces seq_len / ns_start when given
     int32_t B, H, Lq, Lk;
     int32_t ns_start;           // keys >= ns_start are always valid (Lk = no such suffix)

@@ -439,63 +439,50 @@ constexpr int kFqWarps = 4;
 constexpr int kFqStages = 3;
 constexpr int kFqRows = 16;    // keys per tile = queries per tile
 
+// One sample of a few-queries launch: its keys, its queries and where they lie
+struct FewqSample {
+    int lk, lq, off;            // off: position of query 0 among the keys
+    int64_t k_row, q_at, o_at;  // first key row; element offsets of query 0 and output 0 (without the head)
+};
+__device__ __forceinline__ FewqSample fewq_sample(const AttnArgs& a, int b) {
+    FewqSample s;
+    s.k_row = a.cu_rows[b];
+    s.lq = s.lk = a.cu_rows[b + 1] - static_cast<int32_t>(s.k_row);
+    int64_t q_row = s.k_row;
+    if (a.cu_rows_q != nullptr) {
+        q_row = a.cu_rows_q[b];
+        s.lq = a.cu_rows_q[b + 1] - static_cast<int32_t>(q_row);
+    }
+    s.q_at = q_row * a.q_sl;
+    s.o_at = q_row * a.o_sl;
+    if (a.q_fixed > 0) {
+        s.lq = min(a.q_fixed, s.lk);
+        s.q_at = b * a.q_sb;
+        s.o_at = b * a.o_sb;
+    }
+    s.off = max(s.lk - s.lq, 0);
+    return s;
+}
+
+// 16 queries (rows r0 .. r0 + 15 of a (sample, head)) against the key tiles first, first + step, ...: K and V through this warp's
+// private ring, online softmax in registers.  acc: 16 x 64 unnormalised outputs, m_run: running maxima of rows g and g + 8 (raw
+// scores), l_run: this lane's share of the running sums.
 template <typename T>
-__global__ void __launch_bounds__(kFqWarps * 32, 4)
-attn_fewq_kernel(const AttnArgs a) {
-    chain_release();
-    chain_wait();
+__device__ __forceinline__ void fewq_walk(const AttnArgs& a, const FewqSample& sm, const T* q, const T* k, const T* v, T* ring, int r0, int first,
+                                          int step, float (&acc)[8][4], float (&m_run)[2], float (&l_run)[2]) {
     constexpr int D = 64;
     constexpr int CH = D / 8;
-    extern __shared__ __align__(128) uint8_t fq_smem[];
-    const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int g = lane >> 2;
-    const int t = lane & 3;
-    const int mi = lane >> 3;
-    const int64_t pair = static_cast<int64_t>(blockIdx.x) * kFqWarps + warp;
-    if (pair >= static_cast<int64_t>(a.B) * a.H) return;
-    const int b = static_cast<int>(pair / a.H);
-    const int h_own = static_cast<int>(pair - static_cast<int64_t>(b) * a.H);
-
-    const int64_t row_base = a.cu_rows[b];
-    const int lk = a.cu_rows[b + 1] - static_cast<int32_t>(row_base);
-    int64_t q_base = row_base;
-    int lq = lk;
-    if (a.cu_rows_q != nullptr) {
-        q_base = a.cu_rows_q[b];
-        lq = a.cu_rows_q[b + 1] - static_cast<int32_t>(q_base);
-    }
-    if (lq <= 0 || lk <= 0) return;   // uniform over the warp
-    const int off = max(lk - lq, 0);
+    const int g = lane >> 2, t = lane & 3, mi = lane >> 3;
     const bool causal = a.causal != 0;
-    // this warp's ring: kFqStages x (K tile, V tile) of 16 rows x 64
-    T* ring = reinterpret_cast<T*>(fq_smem) + static_cast<size_t>(warp) * kFqStages * 2 * kFqRows * D;
-
-    // Work split.  A sample of at most 16 queries: warp w owns head w of the block's heads and its only query tile.
-    // A sample with more: when the block's warps all belong to one sample (H a multiple of the warps per
-    // block), its (head, query tile) pairs are dealt to the warps head by head, warp w taking pairs w, w + 4, ...;
-    // warps that work on the same head then read the same keys and values at about the same time, so all but
-    // one of them are served by the L2 instead of re-reading a long sample from HBM once per query tile, and no
-    // warp idles when a head has fewer query tiles than the block has warps.
-    const bool together = lq > kFqRows && a.H % kFqWarps == 0;
-    const int h_first = together ? h_own - warp : h_own;
-    const int n_qt = (lq + kFqRows - 1) / kFqRows;
-    const int n_items = together ? kFqWarps * n_qt : n_qt;
-
-    for (int item = together ? warp : 0; item < n_items; item += together ? kFqWarps : 1) {
-    const int h = h_first + (together ? item / n_qt : 0);
-    const int r0 = (together ? item % n_qt : item) * kFqRows;
-    const T* q = static_cast<const T*>(a.q) + q_base * a.q_sl + static_cast<int64_t>(h) * a.q_sh;
-    const T* k = static_cast<const T*>(a.k) + row_base * a.k_sl + static_cast<int64_t>(h) * a.k_sh;
-    const T* v = static_cast<const T*>(a.v) + row_base * a.v_sl + static_cast<int64_t>(h) * a.v_sh;
-    T* o = static_cast<T*>(a.o) + q_base * a.o_sl + static_cast<int64_t>(h) * a.o_sh;
-    auto issue = [&](int tile) {   // rows [16 tile, 16 tile + 16) of K and V; rows past the sample are zero
-        T* sK = ring + static_cast<size_t>(tile % kFqStages) * 2 * kFqRows * D;
+    const int lk = sm.lk, lq = sm.lq, off = sm.off;
+    auto issue = [&](int i, int tile) {   // the walk's i-th tile: rows [16 tile, 16 tile + 16) of K and V; rows past the sample are zero
+        T* sK = ring + static_cast<size_t>(i % kFqStages) * 2 * kFqRows * D;
         T* sV = sK + kFqRows * D;
 #pragma unroll
-        for (int i = lane; i < kFqRows * CH; i += 32) {
-            const int r = i / CH;
-            const int c = i - r * CH;
+        for (int p = lane; p < kFqRows * CH; p += 32) {
+            const int r = p / CH;
+            const int c = p - r * CH;
             const int row = tile * kFqRows + r;
             const bool ok = row < lk;
             cp_async16(sK + swz<D>(r, c), k + static_cast<int64_t>(ok ? row : 0) * a.k_sl + c * 8, ok);
@@ -503,117 +490,156 @@ attn_fewq_kernel(const AttnArgs a) {
         }
     };
 
+    // keys the tile's last existing query can see
+    const int q_last = min(r0 + kFqRows, lq) - 1;
+    const int kv_end = causal ? min(lk, q_last + off + 1) : lk;
+    const int n_all = (kv_end + kFqRows - 1) / kFqRows;
+    const int n_tiles = first < n_all ? (n_all - first + step - 1) / step : 0;
+#pragma unroll
+    for (int s0 = 0; s0 < kFqStages - 1; ++s0) {
+        if (s0 < n_tiles) issue(s0, first + s0 * step);
+        cp_async_commit();
+    }
+    // Q fragments straight from global memory: rows r0 + g and r0 + g + 8, columns 16 kk + 2 t (+ 8)
+    uint32_t qf[D / 16][4];
     {
-        // keys the tile's last existing query can see
-        const int q_last = min(r0 + kFqRows, lq) - 1;
-        const int kv_end = causal ? min(lk, q_last + off + 1) : lk;
-        const int n_tiles = (kv_end + kFqRows - 1) / kFqRows;
+        const bool ok0 = r0 + g < lq, ok1 = r0 + g + 8 < lq;
+        const T* q0 = q + static_cast<int64_t>(ok0 ? r0 + g : 0) * a.q_sl + 2 * t;
+        const T* q1 = q + static_cast<int64_t>(ok1 ? r0 + g + 8 : 0) * a.q_sl + 2 * t;
 #pragma unroll
-        for (int s0 = 0; s0 < kFqStages - 1; ++s0) {
-            if (s0 < n_tiles) issue(s0);
-            cp_async_commit();
+        for (int kk = 0; kk < D / 16; ++kk) {
+            qf[kk][0] = ok0 ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16) : 0u;
+            qf[kk][1] = ok1 ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16) : 0u;
+            qf[kk][2] = ok0 ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 8) : 0u;
+            qf[kk][3] = ok1 ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16 + 8) : 0u;
         }
-        // Q fragments straight from global memory: rows r0 + g and r0 + g + 8, columns 16 kk + 2 t (+ 8)
-        uint32_t qf[D / 16][4];
-        {
-            const bool ok0 = r0 + g < lq, ok1 = r0 + g + 8 < lq;
-            const T* q0 = q + static_cast<int64_t>(ok0 ? r0 + g : 0) * a.q_sl + 2 * t;
-            const T* q1 = q + static_cast<int64_t>(ok1 ? r0 + g + 8 : 0) * a.q_sl + 2 * t;
+    }
 #pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                qf[kk][0] = ok0 ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16) : 0u;
-                qf[kk][1] = ok1 ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16) : 0u;
-                qf[kk][2] = ok0 ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 8) : 0u;
-                qf[kk][3] = ok1 ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16 + 8) : 0u;
-            }
-        }
-        float acc[D / 8][4];
+    for (int j = 0; j < D / 8; ++j)
 #pragma unroll
-        for (int j = 0; j < D / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-        float m_run[2] = {-INFINITY, -INFINITY};   // running maxima of rows g, g + 8 (raw scores)
-        float l_run[2] = {0.f, 0.f};               // this lane's share of the running sums
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+    m_run[0] = m_run[1] = -INFINITY;
+    l_run[0] = l_run[1] = 0.f;
 
-        for (int jt = 0; jt < n_tiles; ++jt) {
-            if (jt + kFqStages - 1 < n_tiles) issue(jt + kFqStages - 1);
-            cp_async_commit();
-            cp_async_wait<kFqStages - 1>();
-            __syncwarp();
-            const T* sK = ring + static_cast<size_t>(jt % kFqStages) * 2 * kFqRows * D;
-            const T* sV = sK + kFqRows * D;
-            float s[2][4];
+    for (int jt = 0; jt < n_tiles; ++jt) {
+        if (jt + kFqStages - 1 < n_tiles) issue(jt + kFqStages - 1, first + (jt + kFqStages - 1) * step);
+        cp_async_commit();
+        cp_async_wait<kFqStages - 1>();
+        __syncwarp();
+        const T* sK = ring + static_cast<size_t>(jt % kFqStages) * 2 * kFqRows * D;
+        const T* sV = sK + kFqRows * D;
+        float s[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+            uint32_t kb[4];
+            ldsm_x4(kb, sK + swz<D>((mi >> 1) * 8 + (lane & 7), kk * 2 + (mi & 1)));
+            mma16816<T>(s[0], qf[kk], kb[0], kb[1]);
+            mma16816<T>(s[1], qf[kk], kb[2], kb[3]);
+        }
+        const int c0 = (first + jt * step) * kFqRows;
+        // only the tiles on the causal edge and the sample's last tile hold keys a query must not see
+        const bool edge = (causal && c0 + kFqRows - 1 > r0 + off) || c0 + kFqRows > lk;
+        float p_scale[2];
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            const int rg = r0 + g + 8 * hr + off;   // the query's position among the keys
+            float mx = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                uint32_t kb[4];
-                ldsm_x4(kb, sK + swz<D>((mi >> 1) * 8 + (lane & 7), kk * 2 + (mi & 1)));
-                mma16816<T>(s[0], qf[kk], kb[0], kb[1]);
-                mma16816<T>(s[1], qf[kk], kb[2], kb[3]);
-            }
-            const int c0 = jt * kFqRows;
-            // only the tiles on the causal edge and the sample's last tile hold keys a query must not see
-            const bool edge = (causal && c0 + kFqRows - 1 > r0 + off) || c0 + kFqRows > lk;
-            float p_scale[2];
-#pragma unroll
-            for (int hr = 0; hr < 2; ++hr) {
-                const int rg = r0 + g + 8 * hr + off;   // the query's position among the keys
-                float mx = -INFINITY;
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int c = c0 + j * 8 + 2 * t + e;
-                        if (edge && (c >= lk || (causal && c > rg))) s[j][2 * hr + e] = -INFINITY;
-                        mx = fmaxf(mx, s[j][2 * hr + e]);
-                    }
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float m_new = fmaxf(m_run[hr], mx);
-                const float ms = (m_new == -INFINITY ? 0.f : m_new) * a.scale_log2;
-                const float corr = ex2_approx(m_run[hr] * a.scale_log2 - ms);   // first tile: exp2(-inf) = 0
-                m_run[hr] = m_new;
-                float sum = 0.f;
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float p = ex2_approx(s[j][2 * hr + e] * a.scale_log2 - ms);
-                        s[j][2 * hr + e] = p;
-                        sum += p;
-                    }
-                l_run[hr] = l_run[hr] * corr + sum;
-                p_scale[hr] = corr;
-            }
-            if (__any_sync(0xffffffffu, p_scale[0] != 1.f || p_scale[1] != 1.f)) {
-#pragma unroll
-                for (int j = 0; j < D / 8; ++j) {
-                    acc[j][0] *= p_scale[0];
-                    acc[j][1] *= p_scale[0];
-                    acc[j][2] *= p_scale[1];
-                    acc[j][3] *= p_scale[1];
+                for (int e = 0; e < 2; ++e) {
+                    const int c = c0 + j * 8 + 2 * t + e;
+                    if (edge && (c >= lk || (causal && c > rg))) s[j][2 * hr + e] = -INFINITY;
+                    mx = fmaxf(mx, s[j][2 * hr + e]);
                 }
-            }
-            uint32_t pa[4];
-            pa[0] = pack2<T>(s[0][0], s[0][1]);
-            pa[1] = pack2<T>(s[0][2], s[0][3]);
-            pa[2] = pack2<T>(s[1][0], s[1][1]);
-            pa[3] = pack2<T>(s[1][2], s[1][3]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float m_new = fmaxf(m_run[hr], mx);
+            const float ms = (m_new == -INFINITY ? 0.f : m_new) * a.scale_log2;
+            const float corr = ex2_approx(m_run[hr] * a.scale_log2 - ms);   // first tile: exp2(-inf) = 0
+            m_run[hr] = m_new;
+            float sum = 0.f;
 #pragma unroll
-            for (int jp = 0; jp < D / 16; ++jp) {
-                uint32_t vb[4];
-                ldsm_x4_t(vb, sV + swz<D>((mi & 1) * 8 + (lane & 7), jp * 2 + (mi >> 1)));
-                mma16816<T>(acc[2 * jp], pa, vb[0], vb[1]);
-                mma16816<T>(acc[2 * jp + 1], pa, vb[2], vb[3]);
-            }
-            __syncwarp();   // the stage is free for the copy issued at the top of the next iteration
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float p = ex2_approx(s[j][2 * hr + e] * a.scale_log2 - ms);
+                    s[j][2 * hr + e] = p;
+                    sum += p;
+                }
+            l_run[hr] = l_run[hr] * corr + sum;
+            p_scale[hr] = corr;
         }
-        cp_async_wait<0>();   // nothing of this query tile is in flight when the next one restarts the ring
-        __syncwarp();
+        if (__any_sync(0xffffffffu, p_scale[0] != 1.f || p_scale[1] != 1.f)) {
+#pragma unroll
+            for (int j = 0; j < D / 8; ++j) {
+                acc[j][0] *= p_scale[0];
+                acc[j][1] *= p_scale[0];
+                acc[j][2] *= p_scale[1];
+                acc[j][3] *= p_scale[1];
+            }
+        }
+        uint32_t pa[4];
+        pa[0] = pack2<T>(s[0][0], s[0][1]);
+        pa[1] = pack2<T>(s[0][2], s[0][3]);
+        pa[2] = pack2<T>(s[1][0], s[1][1]);
+        pa[3] = pack2<T>(s[1][2], s[1][3]);
+#pragma unroll
+        for (int jp = 0; jp < D / 16; ++jp) {
+            uint32_t vb[4];
+            ldsm_x4_t(vb, sV + swz<D>((mi & 1) * 8 + (lane & 7), jp * 2 + (mi >> 1)));
+            mma16816<T>(acc[2 * jp], pa, vb[0], vb[1]);
+            mma16816<T>(acc[2 * jp + 1], pa, vb[2], vb[3]);
+        }
+        __syncwarp();   // the stage is free for the copy issued at the top of the next iteration
+    }
+    cp_async_wait<0>();   // nothing of this query tile is in flight when the next one restarts the ring
+    __syncwarp();
+}
 
+template <typename T>
+__global__ void __launch_bounds__(kFqWarps * 32, 4)
+attn_fewq_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
+    extern __shared__ __align__(128) uint8_t fq_smem[];
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2;
+    const int t = lane & 3;
+    const int64_t pair = static_cast<int64_t>(blockIdx.x) * kFqWarps + warp;
+    if (pair >= static_cast<int64_t>(a.B) * a.H) return;
+    const int b = static_cast<int>(pair / a.H);
+    const int h_own = static_cast<int>(pair - static_cast<int64_t>(b) * a.H);
+    const FewqSample sm = fewq_sample(a, b);
+    if (sm.lq <= 0 || sm.lk <= 0) return;   // uniform over the warp
+    // this warp's ring: kFqStages x (K tile, V tile) of 16 rows x 64
+    T* ring = reinterpret_cast<T*>(fq_smem) + static_cast<size_t>(warp) * kFqStages * 2 * kFqRows * 64;
+
+    // Work split.  A sample of at most 16 queries: warp w owns head w of the block's heads and its only query tile.
+    // A sample with more: when the block's warps all belong to one sample (H a multiple of the warps per
+    // block), its (head, query tile) pairs are dealt to the warps head by head, warp w taking pairs w, w + 4, ...;
+    // warps that work on the same head then read the same keys and values at about the same time, so all but
+    // one of them are served by the L2 instead of re-reading a long sample from HBM once per query tile, and no
+    // warp idles when a head has fewer query tiles than the block has warps.
+    const bool together = sm.lq > kFqRows && a.H % kFqWarps == 0;
+    const int h_first = together ? h_own - warp : h_own;
+    const int n_qt = (sm.lq + kFqRows - 1) / kFqRows;
+    const int n_items = together ? kFqWarps * n_qt : n_qt;
+
+    for (int item = together ? warp : 0; item < n_items; item += together ? kFqWarps : 1) {
+        const int h = h_first + (together ? item / n_qt : 0);
+        const int r0 = (together ? item % n_qt : item) * kFqRows;
+        const T* q = static_cast<const T*>(a.q) + sm.q_at + static_cast<int64_t>(h) * a.q_sh;
+        const T* k = static_cast<const T*>(a.k) + sm.k_row * a.k_sl + static_cast<int64_t>(h) * a.k_sh;
+        const T* v = static_cast<const T*>(a.v) + sm.k_row * a.v_sl + static_cast<int64_t>(h) * a.v_sh;
+        T* o = static_cast<T*>(a.o) + sm.o_at + static_cast<int64_t>(h) * a.o_sh;
+        float acc[8][4], m_run[2], l_run[2];
+        fewq_walk<T>(a, sm, q, k, v, ring, r0, 0, 1, acc, m_run, l_run);
 #pragma unroll
         for (int hr = 0; hr < 2; ++hr) {
             float l = l_run[hr];
@@ -621,15 +647,79 @@ attn_fewq_kernel(const AttnArgs a) {
             l += __shfl_xor_sync(0xffffffffu, l, 2);
             const float inv = l > 0.f ? 1.0f / l : 0.f;
             const int r = r0 + g + 8 * hr;
-            if (r < lq) {
+            if (r < sm.lq) {
                 T* orow = o + static_cast<int64_t>(r) * a.o_sl + 2 * t;
 #pragma unroll
-                for (int j = 0; j < D / 8; ++j)
+                for (int j = 0; j < 8; ++j)
                     *reinterpret_cast<uint32_t*>(orow + j * 8) = pack2<T>(acc[j][2 * hr] * inv, acc[j][2 * hr + 1] * inv);
             }
         }
     }
-    }   // (head, query tile) pairs
+}
+
+// The same for few samples, where one warp per (sample, head) leaves the chip idle and the walk over the keys is the time (8 samples of
+// up to 580 keys, 8 heads: 55 us): a CTA owns a query tile of a (sample, head), its warps deal the key tiles among themselves and
+// their partial results meet in shared memory.
+constexpr int kFsWarps = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(kFsWarps * 32, 2)
+attn_fewq_split_kernel(const AttnArgs a) {
+    chain_release();
+    chain_wait();
+    extern __shared__ __align__(128) uint8_t fq_smem[];
+    __shared__ float s_m[kFsWarps][kFqRows], s_l[kFsWarps][kFqRows];
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int h = blockIdx.x, b = blockIdx.y, r0 = blockIdx.z * kFqRows;
+    const FewqSample sm = fewq_sample(a, b);
+    if (r0 >= sm.lq || sm.lk <= 0) return;
+    T* ring = reinterpret_cast<T*>(fq_smem) + static_cast<size_t>(warp) * kFqStages * 2 * kFqRows * 64;
+    const T* q = static_cast<const T*>(a.q) + sm.q_at + static_cast<int64_t>(h) * a.q_sh;
+    const T* k = static_cast<const T*>(a.k) + sm.k_row * a.k_sl + static_cast<int64_t>(h) * a.k_sh;
+    const T* v = static_cast<const T*>(a.v) + sm.k_row * a.v_sl + static_cast<int64_t>(h) * a.v_sh;
+    float acc[8][4], m_run[2], l_run[2];
+    fewq_walk<T>(a, sm, q, k, v, ring, r0, warp, kFsWarps, acc, m_run, l_run);
+    float* part = reinterpret_cast<float*>(ring);             // this warp's 16 x 64 partial output takes the place of its ring
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+        float l = l_run[hr];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        if (t == 0) {
+            s_m[warp][g + 8 * hr] = m_run[hr];
+            s_l[warp][g + 8 * hr] = l;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<float2*>(part + (g + 8 * hr) * 64 + j * 8 + 2 * t) = make_float2(acc[j][2 * hr], acc[j][2 * hr + 1]);
+    }
+    __syncthreads();
+    // 256 threads: row tid / 16, four columns each
+    const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kFsWarps; ++w) m = fmaxf(m, s_m[w][r]);
+    const float ms = (m == -INFINITY ? 0.f : m) * a.scale_log2;
+    float l = 0.f;
+    float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kFsWarps; ++w) {
+        const float f = ex2_approx(s_m[w][r] * a.scale_log2 - ms);     // a warp that saw no key of the row: exp2(-inf) = 0
+        const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(reinterpret_cast<const T*>(fq_smem) +
+                                                              static_cast<size_t>(w) * kFqStages * 2 * kFqRows * 64) + r * 64 + c);
+        l = fmaf(s_l[w][r], f, l);
+        o4.x = fmaf(x.x, f, o4.x);
+        o4.y = fmaf(x.y, f, o4.y);
+        o4.z = fmaf(x.z, f, o4.z);
+        o4.w = fmaf(x.w, f, o4.w);
+    }
+    if (r0 + r < sm.lq) {
+        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        T* orow = static_cast<T*>(a.o) + sm.o_at + static_cast<int64_t>(h) * a.o_sh + static_cast<int64_t>(r0 + r) * a.o_sl + c;
+        *reinterpret_cast<uint2*>(orow) = make_uint2(pack2<T>(o4.x * inv, o4.y * inv), pack2<T>(o4.z * inv, o4.w * inv));
+    }
 }
 
 template <typename T, int D>
@@ -673,8 +763,25 @@ bool attn_fewq_supported(const AttnArgs& a, int head_dim) {
            even(a.q_sl) && even(a.q_sh) && even(a.o_sl) && even(a.o_sh) &&
            (reinterpret_cast<uintptr_t>(a.q) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.o) & 3) == 0;
 }
+template <typename T>
+static int fewq_split(const AttnArgs& a, cudaStream_t stream) {
+    const size_t smem = static_cast<size_t>(kFsWarps) * kFqStages * 2 * kFqRows * 64 * sizeof(T);
+    static bool attr_set[64] = {};
+    const DeviceInfo& dev = device_info();
+    if (!attr_set[dev.index]) {
+        cudaFuncSetAttribute(attn_fewq_split_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        attr_set[dev.index] = true;
+    }
+    launch_chained(attn_fewq_split_kernel<T>, dim3(a.H, a.B, (a.Lq + kFqRows - 1) / kFqRows), kFsWarps * 32, smem, stream, a);
+    count_launch();
+    return launch_status();
+}
 int attn_fewq_forward(const AttnArgs& a, int dtype, cudaStream_t stream) {
     const int64_t pairs = static_cast<int64_t>(a.B) * a.H;
+    // below one resident set of warps (16 per SM) the keys of a (sample, head) are split; 8-byte stores need aligned rows
+    const bool wide_rows = ((a.o_sl | a.o_sh | a.o_sb) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.o) & 7) == 0;
+    if (pairs < 16ll * device_info().sm_count && wide_rows && a.Lq > 0)
+        return dtype == TB200_BF16 ? fewq_split<__nv_bfloat16>(a, stream) : fewq_split<__half>(a, stream);
     const int64_t grid = (pairs + kFqWarps - 1) / kFqWarps;
     if (grid > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (grid == 0) return TB200_OK;

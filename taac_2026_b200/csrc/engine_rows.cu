@@ -19,8 +19,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ---------------------------------------------------------------------------------------
 // small_token: out[r, :] = LayerNorm(SiLU(W x_r + b)) with x_r = [values[r, :n], mask[r, :n] as 0 / 1 (optional)], all in fp32.
-// Eight rows per CTA: a thread owns output columns and reads its weight row once for the eight of them; the activated
-// rows meet in shared memory, where one warp per row takes the statistics.
+// Eight rows per CTA: a thread owns output columns and reads its weights (transposed: neighbouring threads, neighbouring
+// addresses) once for the eight of them; the activated rows meet in shared memory, where one warp per row takes the
+// statistics.
 // ---------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -47,10 +48,9 @@ small_token_kernel(const float* __restrict__ values, int n, int64_t value_stride
         float acc[kWarps];
 #pragma unroll
         for (int r = 0; r < kWarps; ++r) acc[r] = bias[o];
-        const float* wr = w + static_cast<int64_t>(o) * in_dim;
-#pragma unroll 4
+#pragma unroll 8
         for (int c = 0; c < in_dim; ++c) {
-            const float wv = wr[c];
+            const float wv = w[static_cast<int64_t>(c) * d + o];
 #pragma unroll
             for (int r = 0; r < kWarps; ++r) acc[r] = fmaf(wv, xs[r * in_dim + c], acc[r]);
         }
@@ -117,67 +117,96 @@ ns_rows_kernel(const T* __restrict__ ns_tokens, int64_t n, int ns, int64_t batch
 
 // ---------------------------------------------------------------------------------------
 // pool_rows: seq[b] = mean of rmsnorm(row) over the sample's sequence rows, ns[b] = the same over its ns non-sequence rows, in
-// fp32 and in row order (no atomics).  With cu == nullptr the rows are token-major [ns, B, d] and there are no sequence rows.
-// Warp per sample; a lane keeps its pieces of both sums in registers.
+// fp32 (no atomics: the order of the sum does not depend on scheduling).  With cu == nullptr the rows are token-major
+// [ns, B, d] and there are no sequence rows.  The rows of a sample are dealt to the WPS warps that share it (8 where there are
+// few samples and the chain of row loads is the time, 1 where there are many), each sums its own and the sums are added in the
+// order of the warps.
 // ---------------------------------------------------------------------------------------
-template <typename T, int CPL>
+template <typename T, int CPL, int WPS>
 __global__ void __launch_bounds__(kThreads)
 pool_rows_kernel(const uint4* __restrict__ rows, const int64_t* __restrict__ cu, const int64_t* __restrict__ counts, int64_t batch, int ns,
                  int chunks, const uint4* __restrict__ gamma, float eps, float* __restrict__ seq_out, float* __restrict__ ns_out) {
     chain_release();
     chain_wait();
     constexpr int N = Vec16<T>::N;
-    const int lane = threadIdx.x & 31;
-    const int64_t b = static_cast<int64_t>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-    if (b >= batch) return;
-    const int64_t base = cu != nullptr ? cu[b] : b;
+    extern __shared__ float sums[];          // [kWarps][d], WPS > 1 only
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t b = static_cast<int64_t>(blockIdx.x) * (kWarps / WPS) + warp / WPS;
+    const bool live = b < batch;
+    const int part = warp % WPS;
+    const int d = chunks * N;
+    const int64_t base = live ? (cu != nullptr ? cu[b] : b) : 0;
     const int64_t step = cu != nullptr ? 1 : batch;
-    const int n_seq = cu != nullptr ? static_cast<int>(counts[b]) : 0;
-    const float inv_d = 1.0f / static_cast<float>(chunks * N);
-    float g[CPL][N], acc[CPL][N];
+    const int n_seq = live && cu != nullptr ? static_cast<int>(counts[b]) : 0;
+    const float inv_d = 1.0f / static_cast<float>(d);
+    float g[CPL][N];
 #pragma unroll
     for (int k = 0; k < CPL; ++k) {
         const int c = lane + 32 * k;
 #pragma unroll
-        for (int e = 0; e < N; ++e) g[k][e] = acc[k][e] = 0.f;
+        for (int e = 0; e < N; ++e) g[k][e] = 0.f;
         if (c < chunks) Vec16<T>::unpack(gamma[c], g[k]);
     }
-    auto flush = [&](float* out, int count) {
-        const float denom = static_cast<float>(count > 0 ? count : 1);
-#pragma unroll
-        for (int k = 0; k < CPL; ++k) {
-            const int c = lane + 32 * k;
-#pragma unroll
-            for (int e = 0; e < N; ++e) {
-                if (c < chunks) out[b * chunks * N + c * N + e] = acc[k][e] / denom;
-                acc[k][e] = 0.f;
-            }
-        }
-    };
-    for (int r = 0; r < n_seq + ns; ++r) {
-        if (r == n_seq && seq_out != nullptr) flush(seq_out, n_seq);
-        const uint4* row = rows + (base + r * step) * chunks;
-        float f[CPL][N];
-        float sq = 0.f;
-#pragma unroll
-        for (int k = 0; k < CPL; ++k) {
-            const int c = lane + 32 * k;
-            if (c < chunks) {
-                Vec16<T>::unpack(row[c], f[k]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < N; ++e) f[k][e] = 0.f;
-            }
-#pragma unroll
-            for (int e = 0; e < N; ++e) sq = fmaf(f[k][e], f[k][e], sq);
-        }
-        const float inv = rsqrtf(warp_sum(sq) * inv_d + eps);
+    auto mean_of = [&](int first, int count, float* out) {
+        float acc[CPL][N];
 #pragma unroll
         for (int k = 0; k < CPL; ++k)
 #pragma unroll
-            for (int e = 0; e < N; ++e) acc[k][e] += (f[k][e] * inv) * g[k][e];
-    }
-    flush(ns_out, ns);
+            for (int e = 0; e < N; ++e) acc[k][e] = 0.f;
+        for (int r = part; r < count; r += WPS) {
+            const uint4* row = rows + (base + (first + r) * step) * chunks;
+            float f[CPL][N];
+            float sq = 0.f;
+#pragma unroll
+            for (int k = 0; k < CPL; ++k) {
+                const int c = lane + 32 * k;
+                if (c < chunks) {
+                    Vec16<T>::unpack(row[c], f[k]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < N; ++e) f[k][e] = 0.f;
+                }
+#pragma unroll
+                for (int e = 0; e < N; ++e) sq = fmaf(f[k][e], f[k][e], sq);
+            }
+            const float inv = rsqrtf(warp_sum(sq) * inv_d + eps);
+#pragma unroll
+            for (int k = 0; k < CPL; ++k)
+#pragma unroll
+                for (int e = 0; e < N; ++e) acc[k][e] += (f[k][e] * inv) * g[k][e];
+        }
+        const float denom = static_cast<float>(count > 0 ? count : 1);
+        if (WPS > 1) {
+#pragma unroll
+            for (int k = 0; k < CPL; ++k) {
+                const int c = lane + 32 * k;
+                if (c < chunks) {
+#pragma unroll
+                    for (int e = 0; e < N; ++e) sums[warp * d + c * N + e] = acc[k][e];
+                }
+            }
+            __syncthreads();
+            if (live)
+                for (int i = part * 32 + lane; i < d; i += 32 * WPS) {
+                    float v = 0.f;
+#pragma unroll
+                    for (int w = 0; w < WPS; ++w) v += sums[(warp - part + w) * d + i];
+                    out[b * d + i] = v / denom;
+                }
+            __syncthreads();
+        } else if (live) {
+#pragma unroll
+            for (int k = 0; k < CPL; ++k) {
+                const int c = lane + 32 * k;
+                if (c < chunks) {
+#pragma unroll
+                    for (int e = 0; e < N; ++e) out[b * d + c * N + e] = acc[k][e] / denom;
+                }
+            }
+        }
+    };
+    if (seq_out != nullptr) mean_of(0, n_seq, seq_out);
+    mean_of(n_seq, live ? ns : 0, ns_out);
 }
 
 // embedding[b] = [seq[b] or zeros, ns[b]] in fp32, and as T for the classifier's GEMM (optional)
@@ -290,8 +319,12 @@ extern "C" int tb200_pool_rows_fwd(const void* rows, const int64_t* cu, const in
     const int chunks = d * es / 16;
     if (chunks > 256 || batch > (1ll << 33)) return TB200_ERR_UNSUPPORTED;
     if (!device_info().valid) return TB200_ERR_DEVICE;
+    const bool few = batch < 8ll * device_info().sm_count && 8 * d * static_cast<int>(sizeof(float)) <= 48 * 1024;   // under eight samples per SM
+    const dim3 grid = few ? dim3(static_cast<unsigned>(batch)) : dim3(warps_grid(batch));
+    const size_t smem = few ? 8 * d * sizeof(float) : 0;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define TB200_POOL(CPL_)                                                                                                              \
-    TB200_BY_DTYPE((launch_chained(pool_rows_kernel<T, CPL_>, warps_grid(batch), kThreads, 0, static_cast<cudaStream_t>(stream),                 \
+    TB200_BY_DTYPE((launch_chained(few ? pool_rows_kernel<T, CPL_, 8> : pool_rows_kernel<T, CPL_, 1>, grid, kThreads, smem, st,       \
         static_cast<const uint4*>(rows), cu, counts, batch, ns, chunks, static_cast<const uint4*>(gamma), eps, seq_mean, ns_mean)))
     if (chunks <= 32) { TB200_POOL(1); }
     else if (chunks <= 64) { TB200_POOL(2); }

@@ -254,7 +254,7 @@ bag_mean_kernel(BagArgs a, const void* __restrict__ ids, T* __restrict__ out) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 scatter_rows_kernel(uint4* __restrict__ dst, int64_t dst_stride_chunks, int dst_col0_chunks,
-                    const int64_t* __restrict__ ids, const uint4* __restrict__ src, int chunks, int64_t n,
+                    const int64_t* __restrict__ ids, const uint4* __restrict__ src, int64_t src_stride_chunks, int chunks, int64_t n,
                     const uint4* __restrict__ bias, int64_t rows_per_group, const uint4* __restrict__ residual,
                     int64_t res_stride_chunks, int lanes_per_row) {
     chain_release();
@@ -268,7 +268,7 @@ scatter_rows_kernel(uint4* __restrict__ dst, int64_t dst_stride_chunks, int dst_
         const int64_t row = ids[i];
         const uint4* brow = bias != nullptr ? bias + (i / rows_per_group) * chunks : nullptr;
         for (int c = lane_g; c < chunks; c += G) {
-            uint4 v = ld_nc_v4(src + i * chunks + c);
+            uint4 v = ld_nc_v4(src + i * src_stride_chunks + c);
             if (brow != nullptr || residual != nullptr) {
                 float f[N];
                 Vec16<T>::unpack(v, f);
@@ -544,7 +544,15 @@ extern "C" int tb200_gather_rows(const void* table, int64_t vocab_rows, int32_t 
 extern "C" int tb200_scatter_rows(void* dst, int64_t dst_rows, int64_t dst_stride, int32_t dst_col0, const int64_t* ids,
                                   const void* src, int64_t n, int32_t dim, const void* bias, int64_t rows_per_group,
                                   const void* residual, int64_t residual_stride, int dtype, void* stream) {
+    return tb200_scatter_rows_strided(dst, dst_rows, dst_stride, dst_col0, ids, src, dim, n, dim, bias, rows_per_group, residual, residual_stride,
+                                      dtype, stream);
+}
+
+extern "C" int tb200_scatter_rows_strided(void* dst, int64_t dst_rows, int64_t dst_stride, int32_t dst_col0, const int64_t* ids,
+                                          const void* src, int64_t src_stride, int64_t n, int32_t dim, const void* bias, int64_t rows_per_group,
+                                          const void* residual, int64_t residual_stride, int dtype, void* stream) {
     using namespace tb200;
+    if (src_stride < dim) return TB200_ERR_SHAPE;
     if (n < 0 || dim < 1 || dst_rows < 0 || dst_stride < dim || dst_col0 < 0 || dst_col0 + dim > dst_stride) return TB200_ERR_SHAPE;
     if (bias != nullptr && rows_per_group < 1) return TB200_ERR_SHAPE;
     if (residual != nullptr && residual_stride < dim) return TB200_ERR_SHAPE;
@@ -553,7 +561,7 @@ extern "C" int tb200_scatter_rows(void* dst, int64_t dst_rows, int64_t dst_strid
     if (es == 0) return TB200_ERR_DTYPE;
     if (dst == nullptr || ids == nullptr || src == nullptr) return TB200_ERR_NULL;
     if ((static_cast<int64_t>(dim) * es) % 16 != 0 || (dst_stride * es) % 16 != 0 || (static_cast<int64_t>(dst_col0) * es) % 16 != 0 ||
-        (residual != nullptr && (residual_stride * es) % 16 != 0) || !aligned16(dst) || !aligned16(src) ||
+        (src_stride * es) % 16 != 0 || (residual != nullptr && (residual_stride * es) % 16 != 0) || !aligned16(dst) || !aligned16(src) ||
         (bias != nullptr && !aligned16(bias)) || (residual != nullptr && !aligned16(residual)))
         return TB200_ERR_ALIGN;
     if (!device_info().valid) return TB200_ERR_DEVICE;
@@ -566,8 +574,8 @@ extern "C" int tb200_scatter_rows(void* dst, int64_t dst_rows, int64_t dst_strid
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define TB200_SCATTER(T)                                                                                              \
     launch_chained(scatter_rows_kernel<T>, static_cast<unsigned>(grid), kThreads, 0, s,                                          \
-        static_cast<uint4*>(dst), dst_stride * es / 16, dst_col0 * es / 16, ids, static_cast<const uint4*>(src), chunks, \
-        n, static_cast<const uint4*>(bias), rows_per_group < 1 ? 1 : rows_per_group, static_cast<const uint4*>(residual), \
+        static_cast<uint4*>(dst), dst_stride * es / 16, dst_col0 * es / 16, ids, static_cast<const uint4*>(src), \
+        src_stride * es / 16, chunks, n, static_cast<const uint4*>(bias), rows_per_group < 1 ? 1 : rows_per_group, static_cast<const uint4*>(residual), \
         residual_stride * es / 16, G)
     switch (dtype) {
         case TB200_F32: TB200_SCATTER(float); break;

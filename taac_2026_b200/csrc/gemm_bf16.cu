@@ -18,8 +18,9 @@
 
 namespace tb200 {
 void count_launch();
+bool gemm_small_serves(int groups, int64_t M, int N, int K);
 int gemm_small(const void* a, const void* w, const float* bias, const void* residual, void* out, int groups, int M, int N, int K, int act,
-               cudaStream_t stream);
+               bool shared_w, const void* norm_gamma, const void* norm_bias, float norm_eps, cudaStream_t stream);
 int gemm_narrow(const void* a, const void* w, const float* bias, const void* residual, void* out, int groups, int M, int N, int K, int act,
                 int32_t* status, cudaStream_t stream);
 
@@ -415,12 +416,9 @@ extern "C" int tb200_gemm_bf16_grouped(const void* a, const void* w, const float
     // Few rows per group: streaming the weights is what takes the time.  Measured per launch, gemm_small / gemm_narrow /
     // pair tiles, in us: 9 x (1536 x 512) at M = 8: 5.0 / 5.8 / 9.0, M = 16: 6.0 / 5.8 / 9.0, M = 32: 8.6 / 6.1 / 9.4, M = 64: - / 6.8 / 9.5,
     // M = 128: - / 8.3 / 9.6, M = 192: - / 10.8 / 10.2; 9 x (512 x 2048) at M = 32: 7.7 / 10.8 / 18, M = 128: - / 19.3 / 20; 1 x (512 x 512)
-    // at M = 32: 3.0 / 5.5 / 9.0.  gemm_small re-reads the activations in every CTA of 16 columns, so the more rows, the fewer
-    // of its CTAs may there be.
-    const int64_t small_ctas = static_cast<int64_t>(groups) * (N / 16);
-    const int64_t small_most = M <= 8 ? INT64_MAX : (M <= 16 ? 6ll * dev.sm_count : (M <= 32 && K <= 2048 ? 2ll * dev.sm_count : 0));
-    if (small_ctas <= small_most && groups <= 65535)
-        return gemm_small(a, w, bias, residual, out, groups, static_cast<int>(M), N, K, act, st);
+    // at M = 32: 3.0 / 5.5 / 9.0.
+    if (gemm_small_serves(groups, M, N, K))
+        return gemm_small(a, w, bias, residual, out, groups, static_cast<int>(M), N, K, act, false, nullptr, nullptr, 0.f, st);
     if (M <= 128 && groups <= 65535 && act != 2)
         return gemm_narrow(a, w, bias, residual, out, groups, static_cast<int>(M), N, K, act, status_word, st);
     CUtensorMap ta, twh, tow;

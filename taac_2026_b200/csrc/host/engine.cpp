@@ -37,11 +37,11 @@ struct SmallToken {
         : w(field<Tensor>(d, "w")), b(field<Tensor>(d, "b")), gamma(field<Tensor>(d, "gamma")), beta(field<Tensor>(d, "beta")) {}
     // writes [rows, d] at `out` (out_stride elements between rows)
     void run(const Tensor& values, const OptTensor& mask, void* out, int64_t out_stride, at::ScalarType type) const {
-        const int64_t n = values.size(1), in_dim = w.size(1);
+        const int64_t n = values.size(1), in_dim = w.size(0);
         check(tb200_small_token_fwd(data<float>(values), static_cast<int32_t>(n), values.stride(0),
                                     mask.has_value() ? static_cast<const uint8_t*>(mask->data_ptr()) : nullptr,
                                     mask.has_value() ? mask->stride(0) : 0, static_cast<int32_t>(in_dim), data<float>(w), data<float>(b),
-                                    data<float>(gamma), data<float>(beta), out, out_stride, values.size(0), static_cast<int32_t>(w.size(0)), 1e-5f,
+                                    data<float>(gamma), data<float>(beta), out, out_stride, values.size(0), static_cast<int32_t>(w.size(1)), 1e-5f,
                                     dtype_code(type), stream_of(values)), "cuda small_token");
     }
 };
@@ -65,7 +65,7 @@ struct Block {
     Layer qkv, q, kv, out, out_nobias, ffn1, ffn2;
     bool grouped_layers = false;          // the per-token layers run on this library's grouped GEMM
     Tensor ns_qkv_w, ns_qkv_b, ns_q_w, ns_q_b, ns_kv_w, ns_kv_b, ns_w1, ns_b1, ns_w2, ns_b2, ns_b2_folded, out_w_t;   // library form
-    Tensor g_qkv_w, g_qkv_b, g_q_w, g_q_b, g_kv_w, g_kv_b, g_w1, g_b1, g_w2, g_b2, g_b2_folded, g_out_w;              // grouped form
+    Tensor g_qkv_w, g_qkv_b, g_w1, g_b1, g_w2, g_b2, g_b2_folded, g_out_w;              // grouped form
     // e4m3 FFN: weights with their scales (fp32 blocks, or atoms of power-of-two scales)
     Tensor f_up, f_up_s, f_down, f_down_s, f_up_bf16;
     OptTensor f_b_up, f_b_down, f_b_down_folded;
@@ -86,8 +86,8 @@ struct Block {
         take("ns_qkv_w", ns_qkv_w); take("ns_qkv_b", ns_qkv_b); take("ns_q_w", ns_q_w); take("ns_q_b", ns_q_b);
         take("ns_kv_w", ns_kv_w); take("ns_kv_b", ns_kv_b); take("ns_w1", ns_w1); take("ns_b1", ns_b1);
         take("ns_w2", ns_w2); take("ns_b2", ns_b2); take("ns_b2_folded", ns_b2_folded); take("out_w_t", out_w_t);
-        take("g_qkv_w", g_qkv_w); take("g_qkv_b", g_qkv_b); take("g_q_w", g_q_w); take("g_q_b", g_q_b);
-        take("g_kv_w", g_kv_w); take("g_kv_b", g_kv_b); take("g_w1", g_w1); take("g_b1", g_b1);
+        take("g_qkv_w", g_qkv_w); take("g_qkv_b", g_qkv_b); 
+        take("g_w1", g_w1); take("g_b1", g_b1);
         take("g_w2", g_w2); take("g_b2", g_b2); take("g_b2_folded", g_b2_folded); take("g_out_w", g_out_w);
         if (d.contains("ffn_fp8")) {
             const py::object w = d["ffn_fp8"];
@@ -387,6 +387,8 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
     TORCH_CHECK(n_feat == static_cast<int64_t>(seq_tables_.size()), "OneTransInference: ", seq_tables_.size(), " sequence features expected, got ", n_feat);
     const auto& widths = p->widths;
     const auto layers = static_cast<int64_t>(blocks_.size());
+    // the non-sequence tokens need nothing the host has to wait for
+    const Tensor ns_tokens = (ns_tokens_in.has_value() ? *ns_tokens_in : native_ns_tokens(entities, *p)).contiguous();
     {   // the one host read of a forward; already there when the serving loop prepared the batch ahead of time
         py::gil_scoped_release nogil;
         p->ready.synchronize();
@@ -475,7 +477,6 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
     }
 
     // ---- the non-sequence tokens take the rows left for them
-    const Tensor ns_tokens = (ns_tokens_in.has_value() ? *ns_tokens_in : native_ns_tokens(entities, *p)).contiguous();
     Tensor x_ns = make({ns_, b, d_}, type_, device_);
     {
         const Tensor token_ids = ns_ids(first_kept ? 1 : 0), normed_ids = ns_ids(0);
@@ -488,10 +489,6 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
     auto heads_view = [&](const Tensor& m, int64_t part) {   // columns [part d, part d + d) of a [rows, parts d] matrix as [rows, H, hd]
         return m.as_strided({m.size(0), heads_, hd}, {m.size(1), hd, 1}, m.storage_offset() + part * d_);
     };
-    // a weight per non-sequence token: this library's grouped GEMM with the bias in its epilogue, or the library's
-    auto per_token = [&](const Tensor& in, const Tensor& gw, const Tensor& gb, const Tensor& w, bool grouped_layers) {
-        return grouped_layers ? grouped(in, gw, gb, false, std::nullopt, std::nullopt, status_) : at::bmm(in, w);
-    };
     for (int64_t l = 0; l < layers; ++l) {
         const Block& blk = blocks_[l];
         const bool g = blk.grouped_layers;
@@ -503,42 +500,62 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
             x_ns = gather_rows(x, ids_here).view({ns_, b, d_});
         }
         const bool selected = select_early && widths[l + 1] < widths[l];
-        const bool only_ns_kept = selected && max_rows[l + 1] == ns_ && g;
+        // every row the pyramid keeps is a non-sequence row: the rest of the block runs token-major on those alone
+        const bool only_ns_kept = selected && max_rows[l + 1] == ns_ && g && hd == 64 && (attention_kernel == 0 || attention_kernel == 4);
         const Tensor ids_next = selected ? ns_ids(l + 1) : ids_here;
         Tensor attn;
-        auto bias = [&](const Tensor& t) { return g ? OptTensor() : OptTensor(t); };
+        if (only_ns_kept) {
+            // keys and values for every row; queries, attention rows and everything behind them for the non-sequence tokens, token-major
+            // as the blocks behind this one want them.  The projection's bias is added by the norm on the fly and rides on the
+            // feed-forward's output bias into the next residual.
+            const Tensor kv = proj(x, blk.kv);
+            const Tensor qkv = grouped(x_ns, blk.g_qkv_w, blk.g_qkv_b, false, std::nullopt, std::nullopt, status_);
+            scatter_rows(kv, ids_here, qkv.narrow(2, d_, 2 * d_));
+            attn = make({ns_, b, d_}, type_, device_);
+            {
+                const int64_t st[12] = {3 * d_, hd, b * 3 * d_, 0, hd, 2 * d_, 0, hd, 2 * d_, d_, hd, b * d_};
+                const Tensor cu_here = cu32(l);
+                TB200_TIMED("attention_fewq", "seq_len"_a = py::none(), "cu_rows"_a = cu_here, "cu_rows_q"_a = cu32(l + 1), "key_valid"_a = py::none(),
+                            "batch"_a = b, "heads"_a = heads_, "lq"_a = ns_, "lk"_a = max_rows[l], "dim"_a = hd, "ns_start"_a = max_rows[l],
+                            "causal"_a = true, "self_rows"_a = false, "esize"_a = qkv.element_size());
+                check(tb200_attn_last_rows_fwd(ptr(qkv), ptr(kv), static_cast<char*>(kv.data_ptr()) + d_ * kv.element_size(), ptr(attn),
+                                               static_cast<int32_t>(b), static_cast<int32_t>(heads_), static_cast<int32_t>(ns_),
+                                               static_cast<int32_t>(max_rows[l]), st, data<int32_t>(cu_here),
+                                               static_cast<float>(1.0 / std::sqrt(static_cast<double>(hd))), dtype_code(type_), s), "cuda varlen_attention");
+            }
+            const Tensor tok = gather_rows(tokens, l == 0 && first_kept ? ids_next : ids_here).view({ns_, b, d_});
+            add_shared_linear(tok, attn, blk.g_out_w, status_);
+            const Tensor h = norm_grouped(tok, blk.ffn_norm, blk.out_b, blk.g_w1, blk.g_b1, true, status_);
+            grouped(h, blk.g_w2, blk.g_b2_folded, false, tok, tok, status_);
+            return py::make_tuple(false, tok, l + 1, true, py::none(), py::none());
+        }
         if (selected) {
             // The pyramid keeps only the last rows of every sample after this block, and a row of the block's output depends
             // on the other rows through its keys and values alone: keys and values are projected for every row, the rest
             // runs for the rows that survive.
             const Tensor src = l == 0 && first_kept ? first_src : kept_rows(l, nullptr);
             const Tensor kv = proj(x, blk.kv);
-            // rows the per-token layers overwrite need no shared query projection
-            const Tensor qm = only_ns_kept ? make({totals[l + 1], d_}, type_, device_) : proj(gather_rows(x, src), blk.q);
-            scatter_rows(kv, ids_here, per_token(x_ns, blk.g_kv_w, blk.g_kv_b, blk.ns_kv_w, g), bias(blk.ns_kv_b));
-            scatter_rows(qm, ids_next, per_token(x_ns, blk.g_q_w, blk.g_q_b, blk.ns_q_w, g), bias(blk.ns_q_b));
+            const Tensor qm = proj(gather_rows(x, src), blk.q);
+            if (g) {
+                const Tensor qkv = grouped(x_ns, blk.g_qkv_w, blk.g_qkv_b, false, std::nullopt, std::nullopt, status_);
+                scatter_rows(kv, ids_here, qkv.narrow(2, d_, 2 * d_));
+                scatter_rows(qm, ids_next, qkv.narrow(2, 0, d_));
+            } else {
+                scatter_rows(kv, ids_here, at::bmm(x_ns, blk.ns_kv_w), blk.ns_kv_b);
+                scatter_rows(qm, ids_next, at::bmm(x_ns, blk.ns_q_w), blk.ns_q_b);
+            }
             const int kernel = attention_kernel == 1 || attention_kernel == 4 ? attention_kernel : 0;
             attn = packed_attention(heads_view(qm, 0), heads_view(kv, 0), heads_view(kv, 1), cu32(l), max_rows[l], cu32(l + 1), max_rows[l + 1], kernel,
                                     status_);
             if (!(l == 0 && first_kept)) tokens = gather_rows(tokens, src);
         } else {
             const Tensor qkv = proj(x, blk.qkv);
-            scatter_rows(qkv, ids_here, per_token(x_ns, blk.g_qkv_w, blk.g_qkv_b, blk.ns_qkv_w, g), bias(blk.ns_qkv_b));
+            if (g) scatter_rows(qkv, ids_here, grouped(x_ns, blk.g_qkv_w, blk.g_qkv_b, false, std::nullopt, std::nullopt, status_));
+            else scatter_rows(qkv, ids_here, at::bmm(x_ns, blk.ns_qkv_w), blk.ns_qkv_b);
             attn = packed_attention(heads_view(qkv, 0), heads_view(qkv, 1), heads_view(qkv, 2), cu32(l), max_rows[l], std::nullopt, 0, attention_kernel,
                                     status_);
         }
         const Tensor attn2d = attn.view({-1, d_});
-        if (only_ns_kept) {
-            // the rest of the block for the non-sequence rows alone, finishing token-major as the blocks behind it want it: the
-            // projection's bias is added by the norm on the fly and rides on the feed-forward's output bias
-            proj(attn2d, blk.out_nobias, false, tokens, tokens);
-            x = rms_norm(tokens, blk.ffn_norm, blk.out_b);
-            x_ns = gather_rows(x, ids_next).view({ns_, b, d_});
-            const Tensor tok = gather_rows(tokens, ids_next).view({ns_, b, d_});
-            const Tensor h = grouped(x_ns, blk.g_w1, blk.g_b1, true, std::nullopt, std::nullopt, status_);
-            grouped(h, blk.g_w2, blk.g_b2_folded, false, tok, tok, status_);
-            return py::make_tuple(false, tok, l + 1, true, py::none(), py::none());
-        }
         const bool folded = ffn_ != kFfnBf16;
         if (folded) {
             proj(attn2d, blk.out_nobias, false, tokens, tokens);
@@ -582,9 +599,8 @@ Tensor Engine::ns_only(const Tensor& tokens, int64_t first_layer, int64_t batch,
     for (size_t l = static_cast<size_t>(first_layer); l < blocks_.size(); ++l) {
         const Block& blk = blocks_[l];
         const bool g = blk.grouped_layers;
-        Tensor x = rms_norm(tok, blk.attn_norm);
-        const Tensor qkv = g ? grouped(x, blk.g_qkv_w, blk.g_qkv_b, false, std::nullopt, std::nullopt, status_)
-                             : bias_act_rows(at::bmm(x, blk.ns_qkv_w), blk.ns_qkv_b, false);
+        const Tensor qkv = g ? norm_grouped(tok, blk.attn_norm, std::nullopt, blk.g_qkv_w, blk.g_qkv_b, false, status_)
+                             : bias_act_rows(at::bmm(rms_norm(tok, blk.attn_norm), blk.ns_qkv_w), blk.ns_qkv_b, false);
         Tensor attn = make({ns_, batch, d_}, type_, device_);
         {
             // sample-major views of the token-major tensors: (B, H, L = ns, hd)
@@ -609,15 +625,13 @@ Tensor Engine::ns_only(const Tensor& tokens, int64_t first_layer, int64_t batch,
         }
         // the output projection onto the residual stream; its bias is added by the norm on the fly and rides on the
         // feed-forward's output bias into the next residual
-        const Tensor flat = tok.view({ns_ * batch, d_}), attn2d = attn.view({ns_ * batch, d_});
-        if (g) grouped(attn2d, blk.g_out_w, std::nullopt, false, flat, flat, status_);
-        else flat.addmm_(attn2d, blk.out_w_t);
-        x = rms_norm(tok, blk.ffn_norm, blk.out_b);
         if (g) {
-            const Tensor h = grouped(x, blk.g_w1, blk.g_b1, true, std::nullopt, std::nullopt, status_);
+            add_shared_linear(tok, attn, blk.g_out_w, status_);
+            const Tensor h = norm_grouped(tok, blk.ffn_norm, blk.out_b, blk.g_w1, blk.g_b1, true, status_);
             grouped(h, blk.g_w2, blk.g_b2_folded, false, tok, tok, status_);
         } else {
-            const Tensor h = bias_act_rows(at::bmm(x, blk.ns_w1), blk.ns_b1, true);
+            tok.view({ns_ * batch, d_}).addmm_(attn.view({ns_ * batch, d_}), blk.out_w_t);
+            const Tensor h = bias_act_rows(at::bmm(rms_norm(tok, blk.ffn_norm, blk.out_b), blk.ns_w1), blk.ns_b1, true);
             tok = bias_act_rows(at::baddbmm(tok, h, blk.ns_w2), blk.ns_b2_folded, false);
         }
     }

@@ -61,11 +61,12 @@ inline void gather_rows_into(const Tensor& table, const int64_t* ids, const Tens
 }
 // dst[ids[i], col0 ..] = src[i] (+ bias[i / rows per bias row]) (+ residual[ids[i]])
 inline void scatter_rows(const Tensor& dst, const Tensor& ids, const Tensor& src, const OptTensor& bias = std::nullopt,
-                         const OptTensor& residual = std::nullopt) {
-    const int64_t n = ids.numel(), dim = src.numel() / std::max<int64_t>(n, 1);
+                         const OptTensor& residual = std::nullopt) {   // src: [.., dim], rows src.stride(-2) elements apart
+    const int64_t n = ids.numel(), dim = src.size(-1);
     const int64_t per_group = bias.has_value() ? std::max<int64_t>(n / (bias->numel() / dim), 1) : 1;
     TB200_TIMED("scatter_rows", "rows"_a = n, "dim"_a = dim, "esize"_a = dst.element_size());
-    check(tb200_scatter_rows(ptr(dst), dst.size(0), dst.size(1), 0, data<int64_t>(ids), ptr(src), n, static_cast<int32_t>(dim), ptr(bias), per_group,
+    check(tb200_scatter_rows_strided(ptr(dst), dst.size(0), dst.size(1), 0, data<int64_t>(ids), ptr(src), src.stride(-2), n,
+                                     static_cast<int32_t>(dim), ptr(bias), per_group,
                              ptr(residual), residual.has_value() ? residual->size(1) : 0, dtype_code(dst.scalar_type()), stream_of(dst)),
           "cuda scatter_rows");
 }
@@ -106,6 +107,34 @@ inline Tensor grouped(const Tensor& x, const Tensor& w, const OptTensor& b32, bo
     check(tb200_gemm_bf16_grouped(ptr(x), ptr(w), data<float>(b32), ptr(residual), ptr(out), static_cast<int32_t>(g), m, static_cast<int32_t>(n),
                                   static_cast<int32_t>(k), silu ? 1 : 0, data<int32_t>(status), stream_of(x)), "cuda grouped_linear");
     return out;
+}
+
+// A layer for few rows per group with the options of the small GEMM: one weight for all groups, RMSNorm of the activations on the
+// way in.  false: too many rows, nothing was enqueued.
+inline bool few_rows(const Tensor& x, const Tensor& w, const OptTensor& b32, bool silu, const OptTensor& residual, const Tensor& out, bool shared_w,
+                     const OptTensor& norm_gamma, const OptTensor& norm_bias) {
+    const int64_t g = x.size(0), m = x.size(1), k = x.size(2), n = w.size(-2);
+    if (m > 32) return false;
+    TB200_TIMED("gemm_bf16", "groups"_a = g, "m"_a = m, "n"_a = n, "k"_a = k, "silu"_a = silu, "residual"_a = residual.has_value());
+    const int code = tb200_gemm_bf16_few_rows(ptr(x), ptr(w), data<float>(b32), ptr(residual), ptr(out), static_cast<int32_t>(g), m,
+                                              static_cast<int32_t>(n), static_cast<int32_t>(k), silu ? 1 : 0, shared_w, ptr(norm_gamma),
+                                              ptr(norm_bias), 1e-6f, stream_of(x));
+    if (code == TB200_ERR_UNSUPPORTED) return false;
+    check(code, "cuda grouped_linear");
+    return true;
+}
+// act(rmsnorm(x + norm_bias) gamma w[g]^T + b[g]), x [G, M, K]
+inline Tensor norm_grouped(const Tensor& x, const Tensor& gamma, const OptTensor& norm_bias, const Tensor& w, const Tensor& b32, bool silu,
+                           const Tensor& status) {
+    Tensor out = make_like({x.size(0), x.size(1), w.size(-2)}, x);
+    if (few_rows(x, w, b32, silu, std::nullopt, out, false, gamma, norm_bias)) return out;
+    return grouped(rms_norm(x, gamma, norm_bias), w, b32, silu, std::nullopt, out, status);
+}
+// x += a w^T with one weight for all groups; x, a [G, M, K]
+inline void add_shared_linear(const Tensor& x, const Tensor& a, const Tensor& w, const Tensor& status) {
+    if (few_rows(a, w, std::nullopt, false, x, x, true, std::nullopt, std::nullopt)) return;
+    const Tensor flat = x.view({-1, x.size(2)});
+    grouped(a.view({-1, a.size(2)}), w, std::nullopt, false, flat, flat, status);
 }
 
 // x = act(x + bias[group]) in place, act = SiLU or identity; x [groups, rows, cols]

@@ -359,9 +359,6 @@ class OneTransInference:
                 if self.dtype == torch.bfloat16 and self.device.type == "cuda" and d_model % 256 == 0 and hidden % 256 == 0:
                     blk["g_qkv_w"] = torch.cat([wq, wk, wv], dim=1).contiguous()                       # [ns, 3d, d]
                     blk["g_qkv_b"] = blk["ns_qkv_b"].reshape(ns, 3 * d_model).float().contiguous()
-                    blk["g_q_w"], blk["g_kv_w"] = wq.contiguous(), torch.cat([wk, wv], dim=1).contiguous()
-                    blk["g_q_b"] = blk["g_qkv_b"][:, :d_model].contiguous()
-                    blk["g_kv_b"] = blk["g_qkv_b"][:, d_model:].contiguous()
                     blk["g_b2"] = blk["ns_b2"].reshape(ns, d_model).float().contiguous()
                     blk["g_w1"] = stack(p + ".ffn.ns_specific.{i}.net.0", "weight").contiguous()       # [ns, hidden, d]
                     blk["g_b1"] = blk["ns_b1"].reshape(ns, hidden).float().contiguous()
@@ -627,7 +624,7 @@ class OneTransInference:
     def _small_token(self, linear: str, norm: str) -> dict:
         """Linear -> SiLU -> LayerNorm of a handful of fp32 inputs, kept in fp32."""
         f32 = lambda name: self.w[name].float().contiguous()  # noqa: E731
-        return {"w": f32(linear + ".weight"), "b": f32(linear + ".bias"), "gamma": f32(norm + ".weight"), "beta": f32(norm + ".bias")}
+        return {"w": f32(linear + ".weight").t().contiguous(), "b": f32(linear + ".bias"), "gamma": f32(norm + ".weight"), "beta": f32(norm + ".bias")}
 
     def _entity_tokens(self, prefix: str, bank: _Bank, n_tokens: int, groups) -> dict | None:
         """What the executor needs to build an entity's tokens itself: one projection of all pooled fields.  None for the other
@@ -658,7 +655,7 @@ class OneTransInference:
         item = self._entity_tokens("item_tokenizer", self.item_bank, self.item_tokens, spec.item_ns_groups)
         dense = {name: self._small_token(name + ".project.0", name + ".project.2") if dim > 0 else None
                  for name, dim in (("user_dense", spec.user_dense_dim), ("item_dense", spec.item_dense_dim))}
-        fits = all(t is None or 8 * (t["w"].shape[1] + self.d) * 4 <= 48 * 1024 for t in dense.values())
+        fits = all(t is None or 8 * (t["w"].shape[0] + self.d) * 4 <= 48 * 1024 for t in dense.values())
         modes = {"bf16": 0, "fp8": 2 if self.ffn_precise else (3 if self.ffn_mx else 1)}
         config = {
             "d": self.d, "heads": self.heads, "ns": self.num_ns, "emb": spec.emb_dim, "ffn": modes[self.ffn_mode], "status": self.status_word,

@@ -47,7 +47,7 @@ def test_small_token(rows, n, d, masked, dtype):
     x = torch.cat([values, mask[:, :n].float()], 1) if masked else values
     want = F.layer_norm(F.silu(F.linear(x, w, b)), (d,), gamma, beta)
     out = torch.full((rows, 2 * d), 7.0, dtype=dtype, device="cuda")
-    code = _lib.load().tb200_small_token_fwd(_p(values), n, n, _p(mask), n + 1, w.shape[1], _p(w), _p(b), _p(gamma), _p(beta), _p(out), 2 * d, rows, d,
+    code = _lib.load().tb200_small_token_fwd(_p(values), n, n, _p(mask), n + 1, w.shape[1], _p(w.t().contiguous()), _p(b), _p(gamma), _p(beta), _p(out), 2 * d, rows, d,
                                              1e-5, _code(dtype), None)
     assert code == 0
     torch.cuda.synchronize()

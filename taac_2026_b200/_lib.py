@@ -57,6 +57,8 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "tb200_head_fwd": (_INT, [_P, _P, _P, _P, _P, _I64, _I32, _I32, _INT, _P]),
     "tb200_gemm_bf16_few_rows": (_INT, [_P, _P, _P, _P, _P, _I32, _I64, _I32, _I32, _I32, _I32, _P, _P, _F, _P]),
     "tb200_attn_last_rows_fwd": (_INT, [_P, _P, _P, _P, _I32, _I32, _I32, _I32, _P, _P, _F, _INT, _P]),
+    "tb200_split_f32_weights": (_INT, [_P, _P, _I64, _I32, _P]),
+    "tb200_gemm_f32_grouped": (_INT, [_P, _P, _P, _P, _P, _I32, _I64, _I32, _I32, _I32, _P, _P]),
     "tb200_mask_plan": (_INT, [_P, _I64, _I64, _I64, _I32, _I32, _I32, _I32, _P, _P, _P]),
     "tb200_attn_bwd_workspace_bytes": (_I64, [_I32, _I32, _I32]),
     "tb200_attn_bwd": (_INT, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I32, _I32, _I32, _I32, _I32, _P, _P, _P, _I32, _I32, _I32,

@@ -27,6 +27,7 @@ Layer layer_field(const py::dict& d, const std::string& w, const std::string& b3
     l.w = d[w.c_str()].cast<Tensor>();
     l.b32 = optional_field(d, b32.c_str());
     if (l.b32.has_value()) l.b = l.b32->to(l.w.scalar_type());
+    if (own_gemm_serves(l.w.scalar_type(), l.w.size(0), l.w.size(1))) l.own = own_form(l.w);
     return l;
 }
 
@@ -79,6 +80,7 @@ struct Block {
         kv = layer_field(d, "kv_w", "kv_b");
         out = layer_field(d, "out_w", "out_b32");
         out_nobias.w = out.w;
+        out_nobias.own = out.own;
         grouped_layers = d.contains("g_w1");
         auto take = [&](const char* name, Tensor& t) {
             if (d.contains(name)) t = d[name].cast<Tensor>();
@@ -89,6 +91,7 @@ struct Block {
         take("g_qkv_w", g_qkv_w); take("g_qkv_b", g_qkv_b); 
         take("g_w1", g_w1); take("g_b1", g_b1);
         take("g_w2", g_w2); take("g_b2", g_b2); take("g_b2_folded", g_b2_folded); take("g_out_w", g_out_w);
+        for (Tensor* w : {&g_qkv_w, &g_w1, &g_w2, &g_out_w}) *w = own_form(*w);
         if (d.contains("ffn_fp8")) {
             const py::object w = d["ffn_fp8"];
             const bool mx = py::hasattr(w, "a_up");
@@ -217,12 +220,10 @@ public:
 
 private:
     static Tensor i64(const Tensor& t) { return t.scalar_type() == at::kLong && t.is_contiguous() ? t : t.to(at::kLong).contiguous(); }
-    bool own_gemm(int64_t n, int64_t k) const { return type_ == at::kBFloat16 && n % 256 == 0 && k % 64 == 0; }
-
     // act(x w^T + b) (+ residual), x [M, K]: this library's GEMM where the widths are whole tiles, the library's otherwise
     Tensor proj(const Tensor& x, const Layer& l, bool silu = false, const OptTensor& residual = std::nullopt, const OptTensor& out = std::nullopt) const {
         const int64_t n = l.w.size(0), k = l.w.size(1);
-        if (own_gemm(n, k)) return grouped(x, l.w, l.b32, silu, residual, out, status_);
+        if (l.own.defined()) return grouped(x, l.own, l.b32, silu, residual, out, status_);
         Tensor y;
         {
             TB200_TIMED("cublas_linear", "m"_a = x.numel() / k, "n"_a = n, "k"_a = k);
@@ -501,7 +502,7 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
         }
         const bool selected = select_early && widths[l + 1] < widths[l];
         // every row the pyramid keeps is a non-sequence row: the rest of the block runs token-major on those alone
-        const bool only_ns_kept = selected && max_rows[l + 1] == ns_ && g && hd == 64 && (attention_kernel == 0 || attention_kernel == 4);
+        const bool only_ns_kept = selected && max_rows[l + 1] == ns_ && g && hd == 64 && type_ == at::kBFloat16 && (attention_kernel == 0 || attention_kernel == 4);
         const Tensor ids_next = selected ? ns_ids(l + 1) : ids_here;
         Tensor attn;
         if (only_ns_kept) {
@@ -646,17 +647,17 @@ py::tuple Engine::classify(const OptTensor& seq_mean, const Tensor& ns_mean, boo
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
     const int64_t b = ns_mean.size(0), actions = head_w_.size(0);
-    const bool own = own_gemm(d_, 2 * d_);
+    const bool own = classifier_.own.defined();
     Tensor joined = make({b, 2 * d_}, at::kFloat, device_), h;
     OptTensor joined_cast;
-    if (own) joined_cast = make({b, 2 * d_}, type_, device_);
+    if (own && type_ != at::kFloat) joined_cast = make({b, 2 * d_}, type_, device_);
     void* s = stream_of(ns_mean);
     check(tb200_join_summaries(data<float>(seq_mean), data<float>(ns_mean), data<float>(joined), ptr(joined_cast), b, static_cast<int32_t>(d_),
                                dtype_code(type_), s), "cuda join_summaries");
     if (own) {
         // serving mode: the wide layer on the tcgen05 GEMM; its inputs come out of a 16-bit network, so 16-bit operands with
         // fp32 accumulation lose nothing that was still there
-        h = proj(*joined_cast, classifier_, true);
+        h = proj(joined_cast.value_or(joined), classifier_, true);
     } else {
         TB200_TIMED("cublas_linear", "m"_a = b, "n"_a = d_, "k"_a = 2 * d_);
         h = at::silu(at::linear(joined, *classifier_f32_, classifier_.b32));

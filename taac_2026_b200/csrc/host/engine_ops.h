@@ -91,18 +91,40 @@ inline Tensor layer_norm(const Tensor& x, const Tensor& w, const Tensor& b, bool
     return out;
 }
 
-// One layer: weight [N, K] ([G, N, K] grouped) in the compute type, bias in fp32 for this library's GEMM and in the compute
-// type for the library's
+// A weight in the form this library's GEMMs read: as it is in bf16, as three bf16 parts [.., N, 3 K] in fp32
+inline bool own_gemm_serves(at::ScalarType type, int64_t n, int64_t k) {
+    return type == at::kBFloat16 ? n % 256 == 0 && k % 64 == 0 : (type == at::kFloat && n % 128 == 0 && k % 64 == 0);
+}
+inline Tensor own_form(const Tensor& w) {
+    if (!w.defined() || w.scalar_type() != at::kFloat) return w;
+    auto sizes = w.sizes().vec();
+    sizes.back() *= 3;
+    Tensor out = make(sizes, at::kBFloat16, w.device());
+    const Tensor src = w.contiguous();
+    check(tb200_split_f32_weights(data<float>(src), ptr(out), src.numel() / src.size(-1), static_cast<int32_t>(src.size(-1)), stream_of(src)),
+          "cuda split_f32_weights");
+    return out;
+}
+
+// One shared layer: weight [N, K] in the compute type and in the form of this library's GEMM (undefined where that does not serve
+// it), bias in fp32 for this library's GEMM and in the compute type for the library's
 struct Layer {
-    Tensor w;
+    Tensor w, own;
     OptTensor b32, b;
 };
 
-// out[g] = act(x[g] w[g]^T + b[g]) (+ residual[g]); x [G, M, K] or [M, K]; `out` may be the residual
+// out[g] = act(x[g] w[g]^T + b[g]) (+ residual[g]); x [G, M, K] or [M, K], w in the form of own_form; `out` may be the residual
 inline Tensor grouped(const Tensor& x, const Tensor& w, const OptTensor& b32, bool silu, const OptTensor& residual, const OptTensor& out_in,
                       const Tensor& status) {
     const int64_t k = x.size(-1), m = x.size(-2), g = x.dim() == 3 ? x.size(0) : 1, n = w.size(-2);
     Tensor out = out_in.has_value() ? *out_in : (x.dim() == 3 ? make_like({g, m, n}, x) : make_like({m, n}, x));
+    if (x.scalar_type() == at::kFloat) {
+        TB200_TIMED("gemm_f32", "groups"_a = g, "m"_a = m, "n"_a = n, "k"_a = k, "silu"_a = silu, "residual"_a = residual.has_value());
+        check(tb200_gemm_f32_grouped(data<float>(x), ptr(w), data<float>(b32), data<float>(residual), data<float>(out), static_cast<int32_t>(g), m,
+                                     static_cast<int32_t>(n), static_cast<int32_t>(k), silu ? 1 : 0, data<int32_t>(status), stream_of(x)),
+              "cuda gemm_f32");
+        return out;
+    }
     TB200_TIMED("gemm_bf16", "groups"_a = g, "m"_a = m, "n"_a = n, "k"_a = k, "silu"_a = silu, "residual"_a = residual.has_value());
     check(tb200_gemm_bf16_grouped(ptr(x), ptr(w), data<float>(b32), ptr(residual), ptr(out), static_cast<int32_t>(g), m, static_cast<int32_t>(n),
                                   static_cast<int32_t>(k), silu ? 1 : 0, data<int32_t>(status), stream_of(x)), "cuda grouped_linear");
@@ -114,7 +136,7 @@ inline Tensor grouped(const Tensor& x, const Tensor& w, const OptTensor& b32, bo
 inline bool few_rows(const Tensor& x, const Tensor& w, const OptTensor& b32, bool silu, const OptTensor& residual, const Tensor& out, bool shared_w,
                      const OptTensor& norm_gamma, const OptTensor& norm_bias) {
     const int64_t g = x.size(0), m = x.size(1), k = x.size(2), n = w.size(-2);
-    if (m > 32) return false;
+    if (m > 32 || x.scalar_type() != at::kBFloat16) return false;
     TB200_TIMED("gemm_bf16", "groups"_a = g, "m"_a = m, "n"_a = n, "k"_a = k, "silu"_a = silu, "residual"_a = residual.has_value());
     const int code = tb200_gemm_bf16_few_rows(ptr(x), ptr(w), data<float>(b32), ptr(residual), ptr(out), static_cast<int32_t>(g), m,
                                               static_cast<int32_t>(n), static_cast<int32_t>(k), silu ? 1 : 0, shared_w, ptr(norm_gamma),

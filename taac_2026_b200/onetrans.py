@@ -353,10 +353,11 @@ class OneTransInference:
                 blk["ns_w2"] = stack(p + ".ffn.ns_specific.{i}.net.3", "weight").transpose(1, 2).contiguous()
                 blk["ns_b2"] = stack(p + ".ffn.ns_specific.{i}.net.3", "bias").unsqueeze(1)
                 blk["ns_b2_folded"] = (blk["ns_b2"].float() + blk["out_b"].float()).to(blk["ns_b2"].dtype)
-                # The same layers for the grouped tcgen05 GEMM, which takes stacked `nn.Linear` weights as they are
-                # ([token, out, in]) and adds bias, SiLU and residual in its epilogue (bf16, widths in whole tiles).
+                # The same layers for the grouped tcgen05 GEMMs, which take stacked `nn.Linear` weights as they are
+                # ([token, out, in]) and add bias, SiLU and residual in their epilogue (widths in whole tiles).
                 hidden = blk["ns_w1"].shape[2]
-                if self.dtype == torch.bfloat16 and self.device.type == "cuda" and d_model % 256 == 0 and hidden % 256 == 0:
+                tile = {torch.bfloat16: 256, torch.float32: 128}.get(self.dtype)
+                if tile and self.device.type == "cuda" and d_model % tile == 0 and hidden % tile == 0:
                     blk["g_qkv_w"] = torch.cat([wq, wk, wv], dim=1).contiguous()                       # [ns, 3d, d]
                     blk["g_qkv_b"] = blk["ns_qkv_b"].reshape(ns, 3 * d_model).float().contiguous()
                     blk["g_b2"] = blk["ns_b2"].reshape(ns, d_model).float().contiguous()
@@ -662,7 +663,7 @@ class OneTransInference:
             "edges": self._edges, "final_norm": self._p("final_norm.weight"),
             "head_w": self.w["classifier.3.weight"].float().contiguous(), "head_b": self.w["classifier.3.bias"].float().contiguous(),
             "classifier_w": self._p("classifier.0.weight"), "classifier_b": self.w["classifier.0.bias"].float().contiguous(),
-            "classifier_w32": None if self._own_gemm(self.d, 2 * self.d) else self.w["classifier.0.weight"].float().contiguous(),
+            "classifier_w32": self.w["classifier.0.weight"].float().contiguous(),
             "project_w": self._p(prefix + ".project.0.weight"), "project_b": self.w[prefix + ".project.0.bias"].float().contiguous(),
             "ln_w": self._p(prefix + ".project.2.weight"), "ln_b": self._p(prefix + ".project.2.bias"),
             "time_table": self._p(time_key) if time_key in self.w else None, "hash_buckets": buckets,

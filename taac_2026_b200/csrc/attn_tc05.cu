@@ -231,74 +231,84 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc_s = umma_idesc(1, 1, 0, 0, kHalf, kBN);  // bf16 x bf16, Q and K both K-major
-            const uint32_t idesc_o = umma_idesc(1, 1, 0, 1, kHalf, kD);   // P K-major, V MN-major (head dim contiguous)
-            const uint32_t q_addr = smem_u32(sQ);
-            uint32_t qc = 0, kc = 0;
-            bool ok = true;
-            for (int64_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
-                int qb, h_idx, b;
-                work.decode(w, qb, h_idx, b);
-                const Plan plan = make_plan(a, b, qb * kBM);
-                if (!plan.half_on[0] || plan.n_tiles == 0) continue;
-                if (!mbar_wait_sleep(&q_full, qc & 1)) { ok = false; break; }
-                ++qc;
-                // S of tile j + 1 is issued before P V of tile j: the softmax of j runs from registers, so the
-                // tensor cores fill the S buffer again while it computes
-                auto issue_s = [&](uint32_t tile_index, bool last_of_item) -> bool {
-                    const uint32_t t = 2 * tile_index;
-                    const uint32_t slot = t % kSlots;
-                    if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1) || !mbar_wait_sleep(&s_free, (tile_index & 1) ^ 1)) return false;
-                    tc_fence_after_sync();
-                    const uint32_t k_addr = smem_u32(sKV + slot * kTileBytes);
+        // The whole warp walks the loop and one elected lane issues: addresses and descriptors are the same for all lanes, so
+        // they live in uniform registers, where the instruction wants them.  Under `if (lane == 0)` every tcgen05.mma first
+        // moved its five operands there, about 100 cycles each.
+        const uint32_t idesc_s = umma_idesc(1, 1, 0, 0, kHalf, kBN);  // bf16 x bf16, Q and K both K-major
+        const uint32_t idesc_o = umma_idesc(1, 1, 0, 1, kHalf, kD);   // P K-major, V MN-major (head dim contiguous)
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t q_desc = umma_desc_sw128(smem_u32(sQ), 1024, 16);
+        const uint64_t k_desc = umma_desc_sw128(smem_u32(sKV), 1024, 16);
+        const uint64_t v_desc = umma_desc_sw128(smem_u32(sKV), 1024, 1024);
+        uint32_t qc = 0, kc = 0;
+        bool ok = true;
+        for (int64_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
+            int qb, h_idx, b;
+            work.decode(w, qb, h_idx, b);
+            const Plan plan = make_plan(a, b, qb * kBM);
+            if (!plan.half_on[0] || plan.n_tiles == 0) continue;
+            if (!mbar_wait_sleep(&q_full, qc & 1)) { ok = false; break; }
+            ++qc;
+            // S of tile j + 1 is issued before P V of tile j: the softmax of j runs from registers, so the
+            // tensor cores fill the S buffer again while it computes
+            auto issue_s = [&](uint32_t tile_index, bool last_of_item) -> bool {
+                const uint32_t t = 2 * tile_index;
+                const uint32_t slot = t % kSlots;
+                if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1) || !mbar_wait_sleep(&s_free, (tile_index & 1) ^ 1)) return false;
+                __syncwarp();
+                tc_fence_after_sync();
+                const uint64_t kd = k_desc + slot * (kTileBytes >> 4);
+                if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kD / 16; ++k) {
-                        mma_f16_ss(tmem_base + kTmemS, umma_desc_sw128(q_addr + k * 32, 1024, 16),
-                                   umma_desc_sw128(k_addr + k * 32, 1024, 16), idesc_s, k > 0 ? 1u : 0u);
-                    }
+                    for (int k = 0; k < kD / 16; ++k) mma_f16_ss(tmem + kTmemS, q_desc + 2 * k, kd + 2 * k, idesc_s, k > 0 ? 1u : 0u);
                     tc_commit(&s_full);
                     tc_commit(&kv_empty[slot]);             // K tile free once the S product has read it
                     if (last_of_item) tc_commit(&q_empty);   // and so is Q after the item's last S product
-                    return true;
-                };
-                int n_active = 0;
-                for (int j = 0; j < plan.n_tiles; ++j) n_active += plan.active(j, 0) ? 1 : 0;
-                if (n_active == 0) {          // nothing visible: hand Q back to the producer directly
-                    mbar_arrive(&q_empty);
-                    continue;
                 }
-                // Per tile the issuer follows the order in which the softmax warps release things: first half of P
-                // -> P V over keys [0, 64); S buffer free -> S of the next tile; second half of P -> rest of P V.
-                // The first half of P V and the next S product run while the softmax still works on the tile.
-                if (!issue_s(kc, n_active == 1)) { ok = false; break; }
-                for (int i = 0; i < n_active && ok; ++i) {
-                    const uint32_t t = 2 * kc + 1;
-                    const uint32_t slot = t % kSlots;
-                    const uint32_t v_addr = smem_u32(sKV + slot * kTileBytes);
-                    if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1)) { ok = false; break; }
-#pragma unroll 1
-                    for (int half = 0; half < 2; ++half) {
-                        if (half == 1 && i + 1 < n_active && !issue_s(kc + 1, i + 2 == n_active)) { ok = false; break; }
-                        if (!mbar_wait_sleep(&p_full[half], kc & 1)) { ok = false; break; }
-                        tc_fence_after_sync();
+                __syncwarp();
+                return true;
+            };
+            int n_active = 0;
+            for (int j = 0; j < plan.n_tiles; ++j) n_active += plan.active(j, 0) ? 1 : 0;
+            if (n_active == 0) {          // nothing visible: hand Q back to the producer directly
+                if (elect_one()) mbar_arrive(&q_empty);
+                continue;
+            }
+            // Per tile the issuer follows the order in which the softmax warps release things: first half of P
+            // -> P V over keys [0, 64); S buffer free -> S of the next tile; second half of P -> rest of P V.
+            // The first half of P V and the next S product run while the softmax still works on the tile.
+            if (!issue_s(kc, n_active == 1)) { ok = false; break; }
+            for (int i = 0; i < n_active && ok; ++i) {
+                const uint32_t t = 2 * kc + 1;
+                const uint32_t slot = t % kSlots;
+                const uint64_t vd = v_desc + slot * (kTileBytes >> 4);
+                if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1)) { ok = false; break; }
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    if (half == 1 && i + 1 < n_active && !issue_s(kc + 1, i + 2 == n_active)) { ok = false; break; }
+                    if (!mbar_wait_sleep(&p_full[half], kc & 1)) { ok = false; break; }
+                    __syncwarp();
+                    tc_fence_after_sync();
+                    if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < kBN / 32; ++kk) {
                             const int k = half * (kBN / 32) + kk;
                             // A: P from TMEM, 16 keys = 8 columns per step; B: V, MN-major, 16 key rows = 2 KB per step
-                            mma_f16_ts(tmem_base + kTmemO, tmem_base + kTmemP + k * 8,
-                                       umma_desc_sw128(v_addr + k * 2048, 1024, 1024), idesc_o, (k > 0 || i > 0) ? 1u : 0u);
+                            mma_f16_ts(tmem + kTmemO, tmem + kTmemP + k * 8, vd + k * (2048 >> 4), idesc_o, (k > 0 || i > 0) ? 1u : 0u);
+                        }
+                        if (half == 1) {
+                            tc_commit(&o_full);
+                            tc_commit(&kv_empty[slot]);
                         }
                     }
-                    if (!ok) break;
-                    tc_commit(&o_full);
-                    tc_commit(&kv_empty[slot]);
-                    ++kc;
+                    __syncwarp();
                 }
+                if (!ok) break;
+                ++kc;
             }
-            if (!ok) {
-                if (args.status != nullptr) atomicExch(args.status, 1);
-            }
+        }
+        if (!ok) {
+            if (args.status != nullptr) atomicExch(args.status, 1);
         }
     } else {
         // ------------------------------------------------------------------ softmax + output

@@ -122,24 +122,16 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 //     the list, so the CTAs that run at the same time read the K / V tiles of a few samples and find them in the L2
 //     (measured on 256 samples of 32..1024 keys: 4-5 % faster, causal or not; on equal lengths under a causal mask
 //     the block-major order is the faster one by the same margin).
-struct Work {
-    int n_qb, heads, batch;
-    int64_t total;
+struct Work {   // 32 bits throughout: three roles decode every item, and a 64-bit division is a subroutine
+    uint32_t n_qb, heads, batch, total;
     bool sample_major;
-    __device__ __forceinline__ void decode(int64_t w, int& qb, int& h, int& b) const {
-        if (sample_major) {
-            const int per_b = n_qb * heads;
-            b = static_cast<int>(w / per_b);
-            const int rem = static_cast<int>(w % per_b);
-            qb = n_qb - 1 - rem / heads;
-            h = rem % heads;
-            return;
-        }
-        const int64_t per_qb = static_cast<int64_t>(heads) * batch;
-        qb = n_qb - 1 - static_cast<int>(w / per_qb);
-        const int rem = static_cast<int>(w % per_qb);
-        h = rem % heads;
-        b = rem / heads;
+    __device__ __forceinline__ void decode(uint32_t w, int& qb, int& h, int& b) const {
+        const uint32_t by_head = w / heads;
+        h = static_cast<int>(w - by_head * heads);
+        const uint32_t inner = sample_major ? n_qb : batch;
+        const uint32_t outer = by_head / inner, rem = by_head - outer * inner;
+        b = static_cast<int>(sample_major ? outer : rem);
+        qb = static_cast<int>(n_qb - 1 - (sample_major ? rem : outer));
     }
 };
 
@@ -164,7 +156,7 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     work.n_qb = (a.Lq + kBM - 1) / kBM;
     work.heads = a.H;
     work.batch = a.B;
-    work.total = static_cast<int64_t>(work.n_qb) * a.H * a.B;
+    work.total = work.n_qb * work.heads * work.batch;
     work.sample_major = a.seq_len != nullptr || a.cu_rows != nullptr;
 
     if (threadIdx.x == 0) {
@@ -200,7 +192,7 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             tma_prefetch_desc(&tmap_v);
             uint32_t qc = 0, kc = 0;
             bool ok = true;
-            for (int64_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
+            for (uint32_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
                 int qb, h_idx, b;
                 work.decode(w, qb, h_idx, b);
                 const Plan plan = make_plan(a, b, qb * kBM);
@@ -242,7 +234,7 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const uint64_t v_desc = umma_desc_sw128(smem_u32(sKV), 1024, 1024);
         uint32_t qc = 0, kc = 0;
         bool ok = true;
-        for (int64_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
+        for (uint32_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
             int qb, h_idx, b;
             work.decode(w, qb, h_idx, b);
             const Plan plan = make_plan(a, b, qb * kBM);
@@ -322,7 +314,7 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         uint32_t kc = 0;
         bool ok = true;
 
-        for (int64_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
+        for (uint32_t w = blockIdx.x; w < work.total && ok; w += gridDim.x) {
             int qb, h_idx, b;
             work.decode(w, qb, h_idx, b);
             const int m0 = qb * kBM;
@@ -355,6 +347,7 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 // pass 1, row max: the four chunk loads are issued together, so one TMEM latency is exposed
                 float mx0 = -INFINITY, mx1 = -INFINITY;
                 uint32_t chunk_live = 0xfu;   // bit c: some row of the warp sees a key of chunk c
+                uint32_t chunk_cut = 0u;      // bit c: some row of the warp does not see all of chunk c
                 {
                     uint32_t sr[4][32];
 #pragma unroll
@@ -371,9 +364,13 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                                 chunk_live &= ~(1u << c);
                                 continue;
                             }
+                            // on the diagonal one chunk per warp is cut, the ones left of it are visible as a whole
+                            if (!__all_sync(0xffffffffu, vis == 0xffffffffu)) {
+                                chunk_cut |= 1u << c;
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                if (!((vis >> i) & 1u)) sr[c][i] = 0xff800000u;  // -inf
+                                for (int i = 0; i < 32; ++i)
+                                    if (!((vis >> i) & 1u)) sr[c][i] = 0xff800000u;  // -inf
+                            }
                         }
 #pragma unroll
                         for (int i = 0; i < 32; i += 4) {
@@ -431,10 +428,12 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                             tmem_st_x16(t_p + c * 16, zero);
                             return;
                         }
-                        const uint32_t vis = chunk_mask(n0 + c * 32);
+                        if ((chunk_cut >> c) & 1u) {
+                            const uint32_t vis = chunk_mask(n0 + c * 32);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (!((vis >> i) & 1u)) r[i] = 0xff800000u;
+                            for (int i = 0; i < 32; ++i)
+                                if (!((vis >> i) & 1u)) r[i] = 0xff800000u;
+                        }
                     }
                     uint32_t pk[16];
 #pragma unroll
@@ -602,6 +601,7 @@ int attn_tc05_forward(const AttnArgs& a, int max_lq, int64_t total_rows, int32_t
     Tc05Args args{a, status};
     (void)max_lq;
     const int64_t items = static_cast<int64_t>((a.Lq + kBM - 1) / kBM) * a.H * a.B;
+    if (items >= (1ll << 31)) return TB200_ERR_UNSUPPORTED;   // their output rows alone would be 256 GB
     int64_t grid = static_cast<int64_t>(dev.sm_count) * 2;  // persistent: two CTAs per SM
     if (grid > items) grid = items;
     // A launch of one round starts under its predecessor (28 x 8 heads of 256 rows in a training step: 13 us less per step);

@@ -223,9 +223,8 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        // The whole warp walks the loop and one elected lane issues: addresses and descriptors are the same for all lanes, so
-        // they live in uniform registers, where the instruction wants them.  Under `if (lane == 0)` every tcgen05.mma first
-        // moved its five operands there, about 100 cycles each.
+        // The whole warp walks the loop and one elected lane issues (see mbar_wait_warp): with one lane in the loop the twelve
+        // MMAs of a key tile took 1.2 k of its 3.1 k cycles.
         const uint32_t idesc_s = umma_idesc(1, 1, 0, 0, kHalf, kBN);  // bf16 x bf16, Q and K both K-major
         const uint32_t idesc_o = umma_idesc(1, 1, 0, 1, kHalf, kD);   // P K-major, V MN-major (head dim contiguous)
         const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
@@ -239,15 +238,14 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             work.decode(w, qb, h_idx, b);
             const Plan plan = make_plan(a, b, qb * kBM);
             if (!plan.half_on[0] || plan.n_tiles == 0) continue;
-            if (!mbar_wait_sleep(&q_full, qc & 1)) { ok = false; break; }
+            if (!mbar_wait_warp(&q_full, qc & 1)) { ok = false; break; }
             ++qc;
             // S of tile j + 1 is issued before P V of tile j: the softmax of j runs from registers, so the
             // tensor cores fill the S buffer again while it computes
             auto issue_s = [&](uint32_t tile_index, bool last_of_item) -> bool {
                 const uint32_t t = 2 * tile_index;
                 const uint32_t slot = t % kSlots;
-                if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1) || !mbar_wait_sleep(&s_free, (tile_index & 1) ^ 1)) return false;
-                __syncwarp();
+                if (!mbar_wait_warp(&kv_full[slot], (t / kSlots) & 1) || !mbar_wait_warp(&s_free, (tile_index & 1) ^ 1)) return false;
                 tc_fence_after_sync();
                 const uint64_t kd = k_desc + slot * (kTileBytes >> 4);
                 if (elect_one()) {
@@ -274,12 +272,11 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 const uint32_t t = 2 * kc + 1;
                 const uint32_t slot = t % kSlots;
                 const uint64_t vd = v_desc + slot * (kTileBytes >> 4);
-                if (!mbar_wait_sleep(&kv_full[slot], (t / kSlots) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(&kv_full[slot], (t / kSlots) & 1)) { ok = false; break; }
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     if (half == 1 && i + 1 < n_active && !issue_s(kc + 1, i + 2 == n_active)) { ok = false; break; }
-                    if (!mbar_wait_sleep(&p_full[half], kc & 1)) { ok = false; break; }
-                    __syncwarp();
+                    if (!mbar_wait_warp(&p_full[half], kc & 1)) { ok = false; break; }
                     tc_fence_after_sync();
                     if (elect_one()) {
 #pragma unroll

@@ -229,9 +229,10 @@ ffn_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0 && sc.active) {
+        if (sc.active) {    // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t idesc = umma_idesc(0, 0, 0, 0, kBM, kBN);  // e4m3 x e4m3 -> f32, both K-major
-            // This one thread sets the pace of the tensor pipe, so its loop carries no division and builds each
+            // This warp sets the pace of the tensor pipe, so its loop carries no division and builds each
             // descriptor with one add: the start-address field counts 16-byte units, a 32-byte K step adds 2.
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
@@ -240,12 +241,12 @@ ffn_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
             bool ok = true;
             for (int n = sc.n_first; n < n_tiles && ok; n += sc.n_step) {
                 if (B_RES) {
-                    if (!mbar_wait_sleep(&b_full, b_phase)) { ok = false; break; }
+                    if (!mbar_wait_warp(&b_full, b_phase)) { ok = false; break; }
                     b_phase ^= 1;
                 }
                 for (int64_t m = sc.j; m < m_tiles && ok; m += sc.G) {
                     for (int kb = 0; kb < k_blocks; ++kb) {
-                        if (!mbar_wait_sleep(&tmem_empty[buf], aph ^ 1) || !mbar_wait_sleep(&full_bar[s], ph)) {
+                        if (!mbar_wait_warp(&tmem_empty[buf], aph ^ 1) || !mbar_wait_warp(&full_bar[s], ph)) {
                             ok = false;
                             break;
                         }
@@ -254,11 +255,14 @@ ffn_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                         const uint32_t b_lo = B_RES ? bres_lo + static_cast<uint32_t>(kb) * (kBBytes >> 4) : a_lo + (kABytes >> 4);
                         const uint64_t da = desc0 + a_lo;
                         const uint64_t db = desc0 + b_lo;
-                        const uint32_t d_tmem = tmem_base + buf * kBN;
+                        const uint32_t d_tmem = tmem + buf * kBN;
+                        if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < kBK / 32; ++k) mma_f8_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, k > 0 ? 1u : 0u);
-                        tc_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs have read it
-                        tc_commit(&tmem_full[buf]);   // the partial product of this K block is complete
+                            for (int k = 0; k < kBK / 32; ++k) mma_f8_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, k > 0 ? 1u : 0u);
+                            tc_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs have read it
+                            tc_commit(&tmem_full[buf]);   // the partial product of this K block is complete
+                        }
+                        __syncwarp();
                         if (++s == STAGES) {
                             s = 0;
                             ph ^= 1;

@@ -258,7 +258,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0 && sc.active) {
+        if (sc.active) {    // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint64_t sf_desc0 = umma_desc_noswizzle(0, 128, 0);      // 32 rows x 16 bytes: four 8-row groups 128 B apart
             const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
@@ -268,49 +269,55 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             bool ok = true;
             for (int n = sc.n_first; n < n_tiles && ok; n += sc.n_step) {
                 if (B_RES) {
-                    if (!mbar_wait_sleep(&b_full, b_phase)) { ok = false; break; }
+                    if (!mbar_wait_warp(&b_full, b_phase)) { ok = false; break; }
                     b_phase ^= 1;
                     tc_fence_after_sync();
                     // the resident weight tile's scale factors go into tensor memory once per column tile
                     // (ordered behind the MMAs of the previous column tile, which read the same columns)
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         const uint32_t src = sfbres_lo + static_cast<uint32_t>(kb) * (kSfbBytes >> 4);
-                        tc_cp_32x128b_warpx4(tmem_base + kTmemSfbRes + kb * 8, sf_desc0 + src);
-                        tc_cp_32x128b_warpx4(tmem_base + kTmemSfbRes + kb * 8 + 4, sf_desc0 + src + (kSfAtom >> 4));
+                        if (elect_one()) {
+                            tc_cp_32x128b_warpx4(tmem + kTmemSfbRes + kb * 8, sf_desc0 + src);
+                            tc_cp_32x128b_warpx4(tmem + kTmemSfbRes + kb * 8 + 4, sf_desc0 + src + (kSfAtom >> 4));
+                        }
+                        __syncwarp();
                     }
                 }
                 for (int64_t m = sc.j; m < m_tiles && ok; m += sc.G, ++tile) {
                     // the epilogue has read the previous tile out of the accumulator
-                    if (!mbar_wait_sleep(&tmem_empty, (tile & 1) ^ 1)) { ok = false; break; }
+                    if (!mbar_wait_warp(&tmem_empty, (tile & 1) ^ 1)) { ok = false; break; }
                     tc_fence_after_sync();
                     for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                        if (!mbar_wait_sleep(&full_bar[s], ph)) { ok = false; break; }
+                        if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
                         tc_fence_after_sync();
                         const uint32_t a_lo = ring_lo + s * (STAGE_BYTES >> 4);
                         const uint32_t b_lo = B_RES ? bres_lo + static_cast<uint32_t>(kb) * (kBBytes >> 4) : a_lo + (kABytes >> 4);
                         const uint32_t sfa_lo = a_lo + (kSfaInStage >> 4);
                         const uint32_t sfb_lo = B_RES ? sfbres_lo + static_cast<uint32_t>(kb) * (kSfbBytes >> 4) : a_lo + (kSfbInStage >> 4);
                         // scale factors of this K block -> TMEM slot (it & 1): 4 columns for A, 8 for B
-                        const uint32_t t_sfa = tmem_base + kTmemSf + (it & 1) * kSfSlotCols;
-                        const uint32_t t_sfb = B_RES ? tmem_base + kTmemSfbRes + kb * 8 : t_sfa + 4;
-                        tc_cp_32x128b_warpx4(t_sfa, sf_desc0 + sfa_lo);
-                        if (!B_RES) {
-                            tc_cp_32x128b_warpx4(t_sfb, sf_desc0 + sfb_lo);
-                            tc_cp_32x128b_warpx4(t_sfb + 4, sf_desc0 + sfb_lo + (kSfAtom >> 4));
-                        }
+                        const uint32_t t_sfa = tmem + kTmemSf + (it & 1) * kSfSlotCols;
+                        const uint32_t t_sfb = B_RES ? tmem + kTmemSfbRes + kb * 8 : t_sfa + 4;
                         const uint64_t da = desc0 + a_lo;
                         const uint64_t db = desc0 + b_lo;
+                        if (elect_one()) {
+                            tc_cp_32x128b_warpx4(t_sfa, sf_desc0 + sfa_lo);
+                            if (!B_RES) {
+                                tc_cp_32x128b_warpx4(t_sfb, sf_desc0 + sfb_lo);
+                                tc_cp_32x128b_warpx4(t_sfb + 4, sf_desc0 + sfb_lo + (kSfAtom >> 4));
+                            }
 #pragma unroll
-                        for (int k = 0; k < kBK / 32; ++k)
-                            mma_mxf8_ss(tmem_base, da + 2 * k, db + 2 * k, umma_idesc_mx(kBM, kBN, k, k), (kb > 0 || k > 0) ? 1u : 0u,
-                                        t_sfa, t_sfb);
-                        tc_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs have read it
+                            for (int k = 0; k < kBK / 32; ++k)
+                                mma_mxf8_ss(tmem, da + 2 * k, db + 2 * k, umma_idesc_mx(kBM, kBN, k, k), (kb > 0 || k > 0) ? 1u : 0u,
+                                            t_sfa, t_sfb);
+                            tc_commit(&empty_bar[s]);     // the stage may be refilled once these MMAs have read it
+                        }
+                        __syncwarp();
                         if (++s == STAGES) {
                             s = 0;
                             ph ^= 1;
                         }
                     }
-                    if (ok) tc_commit(&tmem_full);    // the tile's accumulator is complete
+                    if (ok && elect_one()) tc_commit(&tmem_full);    // the tile's accumulator is complete
                 }
             }
             if (!ok) {
@@ -688,7 +695,8 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader only)
-        if (lane == 0 && rank == 0 && active) {
+        if (rank == 0 && active) {    // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint64_t sf_desc0 = umma_desc_noswizzle(0, 128, 0);
             const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
@@ -698,45 +706,51 @@ mx_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             bool ok = true;
             for (int n = n_first; n < n_tiles && ok; n += n_step) {
                 if (B_RES) {
-                    if (!mbar_wait_sleep(&b_full, b_phase)) { ok = false; break; }
+                    if (!mbar_wait_warp(&b_full, b_phase)) { ok = false; break; }
                     b_phase ^= 1;
                     tc_fence_after_sync();
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         const uint32_t src = sfbres_lo + static_cast<uint32_t>(kb) * (kSfbBytes >> 4);
-                        tc_cp_32x128b_warpx4_pair(tmem_base + kTmemSfbRes + kb * 8, sf_desc0 + src);
-                        tc_cp_32x128b_warpx4_pair(tmem_base + kTmemSfbRes + kb * 8 + 4, sf_desc0 + src + (kSfAtom >> 4));
+                        if (elect_one()) {
+                            tc_cp_32x128b_warpx4_pair(tmem + kTmemSfbRes + kb * 8, sf_desc0 + src);
+                            tc_cp_32x128b_warpx4_pair(tmem + kTmemSfbRes + kb * 8 + 4, sf_desc0 + src + (kSfAtom >> 4));
+                        }
+                        __syncwarp();
                     }
                 }
                 for (int64_t m = row_first; m < m_tiles && ok; m += row_step, ++tile) {
-                    if (!mbar_wait_sleep(&tmem_empty, (tile & 1) ^ 1)) { ok = false; break; }
+                    if (!mbar_wait_warp(&tmem_empty, (tile & 1) ^ 1)) { ok = false; break; }
                     tc_fence_after_sync();
                     for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                        if (!mbar_wait_sleep(&full_bar[s], ph)) { ok = false; break; }
+                        if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
                         tc_fence_after_sync();
                         const uint32_t a_lo = ring_lo + s * (STAGE_BYTES >> 4);
                         const uint32_t b_lo = B_RES ? bres_lo + static_cast<uint32_t>(kb) * (kBHalfBytes >> 4) : a_lo + (kABytes >> 4);
                         const uint32_t sfa_lo = a_lo + (kSfaInStage >> 4);
                         const uint32_t sfb_lo = a_lo + (kSfbInStage >> 4);
-                        const uint32_t t_sfa = tmem_base + kTmemSf + (it & 1) * kSfSlotCols;
-                        const uint32_t t_sfb = B_RES ? tmem_base + kTmemSfbRes + kb * 8 : t_sfa + 4;
-                        tc_cp_32x128b_warpx4_pair(t_sfa, sf_desc0 + sfa_lo);
-                        if (!B_RES) {
-                            tc_cp_32x128b_warpx4_pair(t_sfb, sf_desc0 + sfb_lo);
-                            tc_cp_32x128b_warpx4_pair(t_sfb + 4, sf_desc0 + sfb_lo + (kSfAtom >> 4));
-                        }
+                        const uint32_t t_sfa = tmem + kTmemSf + (it & 1) * kSfSlotCols;
+                        const uint32_t t_sfb = B_RES ? tmem + kTmemSfbRes + kb * 8 : t_sfa + 4;
                         const uint64_t da = desc0 + a_lo;
                         const uint64_t db = desc0 + b_lo;
+                        if (elect_one()) {
+                            tc_cp_32x128b_warpx4_pair(t_sfa, sf_desc0 + sfa_lo);
+                            if (!B_RES) {
+                                tc_cp_32x128b_warpx4_pair(t_sfb, sf_desc0 + sfb_lo);
+                                tc_cp_32x128b_warpx4_pair(t_sfb + 4, sf_desc0 + sfb_lo + (kSfAtom >> 4));
+                            }
 #pragma unroll
-                        for (int k = 0; k < kBK / 32; ++k)
-                            mma_mxf8_ss_pair(tmem_base, da + 2 * k, db + 2 * k, umma_idesc_mx(2 * kBM, kBN, k, k), (kb > 0 || k > 0) ? 1u : 0u,
-                                             t_sfa, t_sfb);
-                        tc_commit_pair(&empty_bar[s]);
+                            for (int k = 0; k < kBK / 32; ++k)
+                                mma_mxf8_ss_pair(tmem, da + 2 * k, db + 2 * k, umma_idesc_mx(2 * kBM, kBN, k, k), (kb > 0 || k > 0) ? 1u : 0u,
+                                                 t_sfa, t_sfb);
+                            tc_commit_pair(&empty_bar[s]);
+                        }
+                        __syncwarp();
                         if (++s == STAGES) {
                             s = 0;
                             ph ^= 1;
                         }
                     }
-                    if (ok) tc_commit_pair(&tmem_full);
+                    if (ok && elect_one()) tc_commit_pair(&tmem_full);
                 }
             }
             if (!ok) {

@@ -200,32 +200,37 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {    // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t idesc = umma_idesc(1, 1, 0, 0, 2 * kBM, kBN);
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
             uint32_t s = 0, ph = 0, buf = 0, aph = 0;
             bool ok = true;
             for (int64_t t = pair; t < total && ok; t += n_pairs) {
-                if (!mbar_wait_sleep(&tmem_empty[buf], aph ^ 1)) { ok = false; break; }
+                if (!mbar_wait_warp(&tmem_empty[buf], aph ^ 1)) { ok = false; break; }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + buf * kBN;
+                const uint32_t d_tmem = tmem + buf * kBN;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait_sleep(&full_bar[s], ph)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint32_t a_lo = ring_lo + s * (kStagePBytes >> 4);
                     const uint64_t da = desc0 + a_lo;
                     const uint64_t db = desc0 + a_lo + (kABytes >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBKBytes / 32; ++k) mma_f16_ss_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                    tc_commit_pair(&empty_bar[s]);
+                        for (int k = 0; k < kBKBytes / 32; ++k) mma_f16_ss_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        tc_commit_pair(&empty_bar[s]);
+                    }
+                    __syncwarp();
                     if (++s == kStagesP) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
                 if (!ok) break;
-                tc_commit_pair(&tmem_full[buf]);
+                if (elect_one()) tc_commit_pair(&tmem_full[buf]);
+                __syncwarp();
                 aph ^= buf;
                 buf ^= 1;
             }

@@ -139,7 +139,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Args g) {
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {   // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t idesc = umma_idesc(1, 1, 0, 0, kTile, kTile);
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint32_t base_lo = (smem_u32(smem) & 0x3FFFFu) >> 4;
@@ -147,24 +148,28 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Args g) {
             uint32_t it = 0, tile = 0;
             for (int64_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++tile) {
                 const uint32_t buf = tile & 1;
-                if (!mbar_wait_sleep(&tmem_empty[buf], ((tile >> 1) & 1) ^ 1)) { ok = false; break; }
+                if (!mbar_wait_warp(&tmem_empty[buf], ((tile >> 1) & 1) ^ 1)) { ok = false; break; }
                 tc_fence_after_sync();
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const uint32_t s = it % kStages;
-                    if (!mbar_wait_sleep(&full_bar[s], (it / kStages) & 1)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full_bar[s], (it / kStages) & 1)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t at = desc0 + base_lo + s * (kStageBytes >> 4);
                     // (part of A, part of W), smallest products first
                     constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pw[6] = {0, 1, 2, 0, 1, 0};
+                    if (elect_one()) {
 #pragma unroll
-                    for (int c = 0; c < 6; ++c)
+                        for (int c = 0; c < 6; ++c)
 #pragma unroll
-                        for (int k = 0; k < kBK / 16; ++k)
-                            mma_f16_ss(tmem_base + buf * kTile, at + pa[c] * kPart + 2 * k, at + (3 + pw[c]) * kPart + 2 * k, idesc,
-                                       (kb | c | k) != 0 ? 1u : 0u);
-                    tc_commit(&empty_bar[s]);
+                            for (int k = 0; k < kBK / 16; ++k)
+                                mma_f16_ss(tmem + buf * kTile, at + pa[c] * kPart + 2 * k, at + (3 + pw[c]) * kPart + 2 * k, idesc,
+                                           (kb | c | k) != 0 ? 1u : 0u);
+                        tc_commit(&empty_bar[s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) tc_commit(&tmem_full[buf]);
+                if (ok && elect_one()) tc_commit(&tmem_full[buf]);
+                __syncwarp();
             }
         }
     } else if (warp < 6) {

@@ -129,21 +129,25 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {   // all lanes walk the loop, an elected one issues (see mbar_wait_warp)
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
             const uint32_t idesc = umma_idesc(1, 1, 0, 0, kTile, static_cast<uint32_t>(g.m_pad));
             const uint64_t desc0 = umma_desc_sw128(0, 1024, 16);
             const uint32_t ring_lo = (smem_u32(ring) & 0x3FFFFu) >> 4;
             for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
                 const int s = it % g.stages;
-                if (!mbar_wait_sleep(&full_bar[s], (it / g.stages) & 1)) { ok = false; break; }
+                if (!mbar_wait_warp(&full_bar[s], (it / g.stages) & 1)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint64_t dw = desc0 + ring_lo + s * (stage_bytes >> 4);
                 const uint64_t da = dw + (kWBytes >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mma_f16_ss(tmem, dw + 2 * k, da + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
-                tc_commit(&empty_bar[s]);
+                    for (int k = 0; k < 4; ++k) mma_f16_ss(tmem_u, dw + 2 * k, da + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+                    tc_commit(&empty_bar[s]);
+                }
+                __syncwarp();
             }
-            tc_commit(&acc_full);    // after a wait that gave up the partial products still end here, and the epilogue writes garbage
+            if (elect_one()) tc_commit(&acc_full);    // after a wait that gave up the partial products still end here, and the epilogue writes garbage
         }
     } else {
         ok = mbar_wait_sleep(&acc_full, 0);

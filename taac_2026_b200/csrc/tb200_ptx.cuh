@@ -116,6 +116,12 @@ __device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity) 
     }
     return true;
 }
+// The same by all lanes of a warp, with one outcome.  For warps that issue tensor-core instructions: their loops run in all
+// lanes and one elected lane issues, so that addresses and descriptors are uniform values.  A tcgen05.mma wants its operands
+// in uniform registers; under `if (lane == 0)` each one was preceded by moving them there, about 100 cycles an instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_sleep(bar, parity)) != 0;
+}
 
 // ---------------------------------------------------------------------------
 // proxy fences

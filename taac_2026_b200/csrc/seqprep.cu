@@ -229,8 +229,10 @@ token_index_kernel(const int64_t* __restrict__ values, const int64_t* __restrict
 //     counts[l][b] = max(n0[b] - (S[0] - S[l]), 0)            rows[l][b] = counts[l][b] + ns
 //     cu[l] = exclusive prefix sum of rows[l]   (B + 1 entries, as int64 and as int32)
 //     meta[l] = (sum_b rows[l][b], max_b rows[l][b])          ns_rows0[b][j] = cu[0][b] + counts[0][b] + j
-// One CTA per layer: a thread owns one sample of a 1024-sample tile (coalesced reads), the tile's rows go through a
-// block scan (warp shuffles + one shared array of warp totals) and the running total is carried from tile to tile.
+// Up to 64 CTAs per layer, each for a span of tiles of 1024 samples (one tile up to 65536 samples): a thread owns one sample
+// of a tile (coalesced reads), the tile's rows go through a block scan (warp shuffles + one shared array of warp totals) and
+// the running total is carried from tile to tile.  What lies before the span is summed up from the lengths again, a few
+// loads per thread: with one CTA per layer the row ids of 8192 samples came from nine CTAs, 137 us, now 23 us.
 // It replaces some ninety one-line tensor operations per batch.
 // ---------------------------------------------------------------------------------------
 constexpr int kPlanThreads = 1024;
@@ -250,25 +252,48 @@ pyramid_plan_kernel(const int64_t* __restrict__ lengths, int batch, int max_len,
     __shared__ int64_t warp_sum[32];
     __shared__ int64_t warp_max[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int l = blockIdx.x;
+    const int l = blockIdx.y;
     const int width = widths.w[0];
     const int64_t drop = width - widths.w[l];
     int64_t* cu_l = cu + static_cast<int64_t>(l) * (batch + 1);
     int32_t* cu32_l = cu32 + static_cast<int64_t>(l) * (batch + 1);
+    const int64_t tiles = (static_cast<int64_t>(batch) + kPlanThreads - 1) / kPlanThreads;
+    const int64_t span = (tiles + gridDim.x - 1) / gridDim.x * kPlanThreads;   // samples per CTA
+    const int64_t first = min(blockIdx.x * span, static_cast<int64_t>(batch)), last = min(first + span, static_cast<int64_t>(batch));
+    auto raw_of = [&](int64_t b) -> int64_t {
+        const int64_t len = lengths[b];
+        return len < 0 ? 0 : (len > max_len ? max_len : len);
+    };
+    auto kept = [&](int64_t raw) -> int64_t {
+        const int64_t n0 = raw < width ? raw : width;
+        return n0 > drop ? n0 - drop : 0;
+    };
     int64_t running = 0, mx = 0;
-    for (int tile = 0; tile < batch; tile += kPlanThreads) {
-        const int b = tile + tid;
+    if (first > 0) {
+        for (int64_t b = tid; b < first; b += kPlanThreads) {
+            const int64_t r = kept(raw_of(b)) + ns;
+            running += r;
+            mx = max(mx, r);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) running += __shfl_xor_sync(0xffffffffu, running, o);
+        if (lane == 0) warp_sum[warp] = running;
+        __syncthreads();
+        running = 0;
+        for (int w = 0; w < 32; ++w) running += warp_sum[w];
+        __syncthreads();
+    }
+    for (int64_t tile = first; tile < last; tile += kPlanThreads) {
+        const int64_t b = tile + tid;
         int64_t c = 0, r = 0;
-        if (b < batch) {
-            const int64_t len = lengths[b];
-            const int64_t raw = len < 0 ? 0 : (len > max_len ? max_len : len);
-            const int64_t n0 = raw < width ? raw : width;
-            c = n0 > drop ? n0 - drop : 0;
+        if (b < last) {
+            const int64_t raw = raw_of(b);
+            c = kept(raw);
             r = c + ns;
             counts[static_cast<int64_t>(l) * batch + b] = c;
             if (l == 0) {
                 start[b] = raw > width ? raw - width : 0;
-                n0_out[b] = n0;
+                n0_out[b] = raw < width ? raw : width;
             }
         }
         mx = max(mx, r);
@@ -287,17 +312,18 @@ pyramid_plan_kernel(const int64_t* __restrict__ lengths, int batch, int max_len,
             tile_total += v;
         }
         const int64_t first_row = running + before + incl - r;
-        if (b < batch) {
+        if (b < last) {
             cu_l[b] = first_row;
             cu32_l[b] = static_cast<int32_t>(first_row);
             if (l == 0)
-                for (int j = 0; j < ns; ++j) ns_rows0[static_cast<int64_t>(b) * ns + j] = first_row + c + j;
+                for (int j = 0; j < ns; ++j) ns_rows0[b * ns + j] = first_row + c + j;
             if (ns_rows != nullptr)
                 for (int j = 0; j < ns; ++j) ns_rows[(static_cast<int64_t>(l) * ns + j) * batch + b] = first_row + c + j;
         }
         running += tile_total;
         __syncthreads();                                    // warp_sum is rewritten by the next tile
     }
+    if (blockIdx.x + 1 != gridDim.x) return;                // the last CTA of a layer has seen every sample
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) warp_max[warp] = mx;
@@ -360,7 +386,10 @@ extern "C" int tb200_pyramid_plan_rows(const int64_t* lengths, int32_t batch, in
     // the int32 offsets must hold the largest total: every sample at most widths[0] + ns rows
     if ((static_cast<int64_t>(widths[0]) + ns) * batch > 0x7FFFFFFFll) return TB200_ERR_SHAPE;
     if (!device_info().valid) return TB200_ERR_DEVICE;
-    launch_chained(pyramid_plan_kernel, static_cast<unsigned>(n_layers + 1), kPlanThreads, 0, static_cast<cudaStream_t>(stream),
+    const int tiles = batch / kPlanThreads + (batch % kPlanThreads != 0 ? 1 : 0);
+    const int parts = tiles < 1 ? 1 : (tiles < 64 ? tiles : 64);
+    launch_chained(pyramid_plan_kernel, dim3(static_cast<unsigned>(parts), static_cast<unsigned>(n_layers + 1)), kPlanThreads, 0,
+        static_cast<cudaStream_t>(stream),
         lengths, batch, max_len, w, ns, start, n0, counts, cu, cu32, meta, ns_rows0, ns_rows);
     count_launch();
     return launch_status();

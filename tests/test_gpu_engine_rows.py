@@ -110,3 +110,38 @@ def test_join_and_head(batch, d, actions):
     want = h.float() @ w.t() + b
     torch.testing.assert_close(logits, want, atol=2e-5, rtol=2e-5)
     torch.testing.assert_close(probs, torch.sigmoid(want), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("ns,d", [(9, 64), (4, 264), (1, 512), (3, 1024)])
+def test_pooled_means_of_many_samples(ns, d, dtype):
+    """More than eight samples per SM: one warp per sample, rows four at a time and the remainder."""
+    batch = 8 * torch.cuda.get_device_properties(0).multi_processor_count + 5
+    g = torch.Generator(device="cuda").manual_seed(d)
+    lens = torch.randint(0, 11, (batch,), device="cuda", generator=g)
+    cu = torch.zeros(batch + 1, dtype=torch.int64, device="cuda")
+    cu[1:] = torch.cumsum(lens + ns, 0)
+    total = int(cu[-1])
+    tokens = torch.randn(total, d, device="cuda", generator=g).to(dtype)
+    w = torch.rand(d, device="cuda", generator=g).to(dtype)
+    seq = torch.empty(batch * d + 1, device="cuda")[1:].view(batch, d)   # off a 16-byte boundary
+    mean = torch.empty(batch, d, device="cuda")
+    assert _lib.load().tb200_pool_rows_fwd(_p(tokens), _p(cu), _p(lens), batch, ns, d, _p(w), 1e-6, _p(seq), _p(mean), _code(dtype), None) == 0
+    torch.cuda.synchronize()
+    owner = torch.repeat_interleave(torch.arange(batch, device="cuda"), lens + ns)
+    is_seq = torch.arange(total, device="cuda") - cu[:-1][owner] < lens[owner]
+    rows = _rms(tokens.double(), w.double())
+    for mask, count, got in ((is_seq, lens.clamp_min(1), seq), (~is_seq, torch.full_like(lens, ns), mean)):
+        want = torch.zeros(batch, d, dtype=torch.float64, device="cuda").index_add_(0, owner[mask], rows[mask]) / count[:, None]
+        torch.testing.assert_close(got.double(), want, atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("batch,d", [(3, 1), (7, 6), (5, 100), (300, 512), (4, 1100)])
+def test_join_widths(batch, d):
+    """Single values, rows that share a CTA, a row per CTA, rows wider than a CTA."""
+    seq, ns = torch.randn(batch, d, device="cuda"), torch.randn(batch, d, device="cuda")
+    for cast_type, code in ((torch.bfloat16, _lib.BF16), (torch.float16, _lib.F16)):
+        joined, cast = torch.empty(batch, 2 * d, device="cuda"), torch.empty(batch, 2 * d, dtype=cast_type, device="cuda")
+        assert _lib.load().tb200_join_summaries(_p(seq), _p(ns), _p(joined), _p(cast), batch, d, code, None) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(joined, torch.cat([seq, ns], 1)) and torch.equal(cast, joined.to(cast_type))

@@ -71,3 +71,9 @@ def test_missing_rows_inside_the_pooling_kernel(dtype):
     got = ops.fields_bag_mean(fields, ids, missing, rows)
     assert torch.equal(got, want)
     assert torch.equal(ops.fields_bag_mean(fields, ids, torch.zeros_like(missing), rows), plain)
+
+
+@pytest.mark.parametrize("batch,max_len,keep,layers,ns", [(1024, 40, 33, 2, 3), (1025, 40, 33, 2, 3), (66_600, 12, 8, 1, 1)])
+def test_plan_over_several_tiles_and_spans(batch, max_len, keep, layers, ns):
+    """One tile exactly, one sample into the second, and more tiles than a layer has CTAs."""
+    test_plan_matches_tensor_arithmetic(batch, max_len, keep, layers, ns)

@@ -43,3 +43,62 @@ def test_against_float64(m, groups, n, k):
     res = [torch.randn(*s, device="cuda", generator=g2) for s in ((groups, m, k), (groups, m, k), (groups, n, k), (groups, n), (groups, m, n))][-1].double()
     want = pre * torch.sigmoid(pre) + res
     assert bool(((r.double() - want).abs() <= 1e-6 + 4e-6 * (pre.abs() + res.abs())).all())
+
+
+def _product(a, w):
+    m, k, n = a.shape[0], a.shape[1], w.shape[0]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    lib = _lib.load()
+    split, out = torch.empty(n, 3 * k, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert lib.tb200_split_f32_weights(p(w), p(split), n, k, None) == 0
+    assert lib.tb200_gemm_f32_grouped(p(a), p(split), None, None, p(out), 1, m, n, k, 0, p(status), None) == 0
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    return out
+
+
+@pytest.mark.parametrize("k", [64, 128, 256, 512, 2560])
+@pytest.mark.parametrize("kind", ["normal", "wide", "positive"])
+def test_no_further_from_float64_than_an_fp32_gemm(k, kind):
+    """The form that this GEMM replaced is the library's SGEMM: its distance from the float64 product, on the same operands, is the
+    bound (2-norm and largest element; both errors are sums of some 4e5 independent roundings, so a tenth covers their spread)."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, w = torch.randn(1000, k, device="cuda", generator=g), torch.randn(384, k, device="cuda", generator=g)
+    if kind == "wide":
+        a = a * torch.exp(2 * torch.randn(1000, k, device="cuda", generator=g))
+    if kind == "positive":       # no cancellation: an accumulator that cuts off instead of rounding shows as a bias
+        a, w = a.abs(), w.abs()
+    exact = a.double() @ w.double().t()
+    old = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    try:
+        theirs = (a @ w.t()).double() - exact
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = old
+    ours = _product(a, w).double() - exact
+    assert ours.norm() <= 1.1 * theirs.norm()
+    assert ours.abs().max() <= 2 * theirs.abs().max()
+
+
+@pytest.mark.parametrize("m,k", [(1, 64), (129, 64), (1000, 128), (40_000, 64)])
+def test_rows_without_a_split(m, k):
+    """A value that is not finite, or rounds to an infinite bf16, gives the row what fp32 arithmetic gives; the rows beside it keep
+    their results.  The longest case has several tiles per CTA, so that the marks of one tile are reused."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, w = torch.randn(m, k, device="cuda", generator=g), torch.randn(256, k, device="cuda", generator=g)
+    rows = torch.arange(0, m, 97, device="cuda")
+    values = torch.tensor([float("inf"), float("-inf"), 3.4e38, float("nan")], device="cuda")[torch.arange(rows.numel(), device="cuda") % 4]
+    a[rows, rows % k] = values
+    w[:, :] = torch.where(w.abs() < 0.1, 0.1, w)      # no product of an infinity with nearly nothing
+    clean = _product(torch.where(a.abs() < 1e30, a, 0.0), w)
+    got = _product(a, w)
+    keep = torch.ones(m, dtype=torch.bool, device="cuda")
+    keep[rows] = False
+    assert torch.equal(got[keep], clean[keep])
+    want = a[rows].double() @ w.double().t()
+    want = torch.where(want.abs() > 3.4028235e38, torch.sign(want) * float("inf"), want)
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got[rows]), torch.isnan(want))
+    assert torch.equal(got[rows][torch.isinf(want)].double(), want[torch.isinf(want)])
+    torch.testing.assert_close(got[rows][finite].double(), want[finite], rtol=1e-5, atol=0)

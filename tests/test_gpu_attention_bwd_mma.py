@@ -50,3 +50,38 @@ def test_backward_at_tile_edges(lq, lk, dim, causal, ns, padded_self, key_map, d
     for name, x, want in zip(("dq", "dk", "dv"), got, (qr.grad, kr.grad, vr.grad)):
         err = (x.float().cpu() - want).abs().max().item()
         assert err <= tol * max(1.0, want.abs().max().item()), f"{name}: {err}"
+
+
+@pytest.mark.parametrize("dtype,size", [(torch.bfloat16, 1.0), (torch.bfloat16, 1e-6), (torch.float16, 1.0), (torch.float16, 2e4), (torch.float16, 1e-4),
+                                        (torch.float16, 1e-6)])
+@pytest.mark.parametrize("length,dim", [(40, 32), (130, 64), (300, 64), (200, 128)])
+def test_gradients_of_any_size_keep_their_bits(length, dim, dtype, size):
+    """Upstream gradients as loss scaling makes them and as small as fp16 holds them, against float64 for the same 16-bit output.
+
+    Bound per element: the rounding of the result (half a unit: 2^-9 / 2^-12 of its value, 2^-25 where fp16 is subnormal; doubled)
+    plus 2^-16 of the sum's absolute terms: 2^-18 for the two parts of P and dS, 2^-21 for two exp2 of 2 ulp, some 2^-18 for the fp32 sums
+    of 32 to 128 terms in the scores and in dP.  One 16-bit part (2^-9, 2^-12) exceeds it, and so does a split that leaves fp16's range."""
+    g = torch.Generator(device="cuda").manual_seed(length)
+    batch, heads = 2, 3
+    q, k, v, d_o = (torch.randn(batch, heads, length, dim, device="cuda", generator=g).to(dtype) for _ in range(4))
+    d_o = (d_o.float().clamp(-3, 3) * size).to(dtype)
+    lens = torch.tensor([length, length * 2 // 3], dtype=torch.int32, device="cuda")
+    out = ops.varlen_attention(q, k, v, seq_len=lens, causal=True)
+    got = ops.attention_backward(q, k, v, out, d_o, seq_len=lens, causal=True)
+    qd, kd, vd, od, gd = (t.double() for t in (q, k, v, out, d_o))
+    scale = dim ** -0.5
+    pos = torch.arange(length, device="cuda")
+    seen = (pos[None, :] <= pos[:, None])[None] & (pos[None, None, :] < lens[:, None, None])
+    p = torch.softmax((qd @ kd.transpose(-1, -2) * scale).masked_fill(~seen[:, None], float("-inf")), -1)
+    ds = p * (gd @ vd.transpose(-1, -2) - (gd * od).sum(-1, keepdim=True))
+    ds_abs = p * (gd.abs() @ vd.abs().transpose(-1, -2) + (gd * od).abs().sum(-1, keepdim=True))
+    unit = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    step = 2.0 ** -24 if dtype == torch.float16 else 0.0
+    for name, x, want, terms in (("dq", got[0], ds @ kd * scale, ds_abs @ kd.abs() * scale),
+                                 ("dk", got[1], ds.transpose(-1, -2) @ qd * scale, ds_abs.transpose(-1, -2) @ qd.abs() * scale),
+                                 ("dv", got[2], p.transpose(-1, -2) @ gd, p.transpose(-1, -2) @ gd.abs())):
+        fits = want.abs() < torch.finfo(dtype).max * 0.999
+        err = (x.double() - want).abs()[fits]
+        bound = (unit * want.abs() + step + 2.0 ** -16 * terms)[fits]
+        assert bool((err <= bound).all()), f"{name}: {(err / bound.clamp_min(1e-300)).max().item():.2f} of the bound"
+        assert bool((x[~fits].abs() > 0.99 * torch.finfo(dtype).max).all()), name

@@ -5,8 +5,10 @@
 //
 // The algorithm and its row layout are described at OneTransInference in onetrans.py; the comments here name the steps.
 #include <ATen/cuda/CUDAEvent.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <pybind11/stl.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -22,12 +24,63 @@ OptTensor optional_field(const py::dict& d, const char* name) {
     if (!d.contains(name) || d[name].is_none()) return std::nullopt;
     return d[name].cast<Tensor>();
 }
-Layer layer_field(const py::dict& d, const std::string& w, const std::string& b32) {
+
+// Tensors made from weights on one stream (three-part splits, casts).  They hold for as long as their sources keep their content,
+// which the sources' version counters tell.
+class Derived {
+public:
+    // the form of a weight that this library's GEMM reads
+    Tensor own(const Tensor& w) { return made_from(w, own_form(w)); }
+    Tensor cast(const Tensor& b, at::ScalarType type) { return made_from(b, b.to(type)); }
+    void watch(const Tensor& source) {
+        sources_.push_back({source, version(source), source.defined() ? source.data_ptr() : nullptr});
+    }
+    bool unchanged() const {
+        return std::all_of(sources_.begin(), sources_.end(), [](const Source& s) { return version(s.t) == s.version && s.t.data_ptr() == s.data; });
+    }
+private:
+    struct Source {
+        Tensor t;
+        int64_t version;
+        const void* data;
+    };
+    static int64_t version(const Tensor& t) { return t.defined() && !t.is_inference() ? static_cast<int64_t>(t._version()) : 0; }
+    Tensor made_from(const Tensor& source, Tensor t) {
+        if (t.defined() && !t.is_same(source)) {
+            watch(source);
+        }
+        return t;
+    }
+    std::vector<Source> sources_;
+};
+
+// The entries of a dict at one time.  It holds the objects, so that an equal address is the same object.
+class Entries {
+public:
+    explicit Entries(const py::dict& d) : dict_(d) {
+        for (const auto& item : d) values_.push_back(py::reinterpret_borrow<py::object>(item.second));
+    }
+    bool same() const {
+        Py_ssize_t at = 0;
+        PyObject *key, *value;
+        size_t i = 0;
+        while (PyDict_Next(dict_.ptr(), &at, &key, &value))
+            if (i == values_.size() || values_[i++].ptr() != value) return false;
+        return i == values_.size();
+    }
+    bool of(const py::handle& d) const { return dict_.ptr() == d.ptr(); }
+
+private:
+    py::dict dict_;
+    std::vector<py::object> values_;
+};
+
+Layer layer_field(const py::dict& d, const std::string& w, const std::string& b32, Derived& derived) {
     Layer l;
     l.w = d[w.c_str()].cast<Tensor>();
     l.b32 = optional_field(d, b32.c_str());
-    if (l.b32.has_value()) l.b = l.b32->to(l.w.scalar_type());
-    if (own_gemm_serves(l.w.scalar_type(), l.w.size(0), l.w.size(1))) l.own = own_form(l.w);
+    if (own_gemm_serves(l.w.scalar_type(), l.w.size(0), l.w.size(1))) l.own = derived.own(l.w);
+    else if (l.b32.has_value()) l.b = derived.cast(*l.b32, l.w.scalar_type());
     return l;
 }
 
@@ -54,9 +107,9 @@ struct EntityTokens {
     Layer project;
     Tensor gamma, beta;
     int64_t n_fields, max_bag, dim, n_tokens;
-    explicit EntityTokens(const py::dict& d)
+    EntityTokens(const py::dict& d, Derived& derived)
         : ptrs(field<Tensor>(d, "ptrs")), rows(field<Tensor>(d, "rows")), offsets(field<Tensor>(d, "offsets")), lengths(field<Tensor>(d, "lengths")),
-          missing_rows(optional_field(d, "missing_rows")), project(layer_field(d, "w", "b32")), gamma(field<Tensor>(d, "gamma")),
+          missing_rows(optional_field(d, "missing_rows")), project(layer_field(d, "w", "b32", derived)), gamma(field<Tensor>(d, "gamma")),
           beta(field<Tensor>(d, "beta")), n_fields(field<int64_t>(d, "n_fields")), max_bag(field<int64_t>(d, "max_bag")),
           dim(field<int64_t>(d, "dim")), n_tokens(field<int64_t>(d, "n_tokens")) {}
 };
@@ -71,14 +124,14 @@ struct Block {
     Tensor f_up, f_up_s, f_down, f_down_s, f_up_bf16;
     OptTensor f_b_up, f_b_down, f_b_down_folded;
 
-    explicit Block(const py::dict& d) {
+    Block(const py::dict& d, Derived& derived) {
         attn_norm = field<Tensor>(d, "attn_norm");
         ffn_norm = field<Tensor>(d, "ffn_norm");
         out_b = field<Tensor>(d, "out_b");
-        qkv = layer_field(d, "qkv_w", "qkv_b");
-        q = layer_field(d, "q_w", "q_b");
-        kv = layer_field(d, "kv_w", "kv_b");
-        out = layer_field(d, "out_w", "out_b32");
+        qkv = layer_field(d, "qkv_w", "qkv_b", derived);
+        q = layer_field(d, "q_w", "q_b", derived);
+        kv = layer_field(d, "kv_w", "kv_b", derived);
+        out = layer_field(d, "out_w", "out_b32", derived);
         out_nobias.w = out.w;
         out_nobias.own = out.own;
         grouped_layers = d.contains("g_w1");
@@ -91,7 +144,7 @@ struct Block {
         take("g_qkv_w", g_qkv_w); take("g_qkv_b", g_qkv_b); 
         take("g_w1", g_w1); take("g_b1", g_b1);
         take("g_w2", g_w2); take("g_b2", g_b2); take("g_b2_folded", g_b2_folded); take("g_out_w", g_out_w);
-        for (Tensor* w : {&g_qkv_w, &g_w1, &g_w2, &g_out_w}) *w = own_form(*w);
+        for (Tensor* w : {&g_qkv_w, &g_w1, &g_w2, &g_out_w}) *w = derived.own(*w);
         if (d.contains("ffn_fp8")) {
             const py::object w = d["ffn_fp8"];
             const bool mx = py::hasattr(w, "a_up");
@@ -104,9 +157,33 @@ struct Block {
             f_b_down_folded = d["ffn_fp8_folded"].attr("b_down").cast<OptTensor>();
             if (!mx && !w.attr("w_up_bf16").is_none()) f_up_bf16 = w.attr("w_up_bf16").cast<Tensor>();
         } else {
-            ffn1 = layer_field(d, "ffn_w1", "ffn_b1");
-            ffn2 = layer_field(d, "ffn_w2", "ffn_b2");
+            ffn1 = layer_field(d, "ffn_w1", "ffn_b1", derived);
+            ffn2 = layer_field(d, "ffn_w2", "ffn_b2", derived);
         }
+    }
+};
+
+// The blocks as the forward reads them, with what they were made from
+struct BlockSet {
+    std::vector<Block> blocks;
+    std::vector<Entries> entries;      // a block's dict, then those of its FFN weight objects
+    std::vector<size_t> first;         // a block's place in `entries`
+    Derived derived;
+    explicit BlockSet(const py::list& dicts) {
+        for (const auto& d : dicts) {
+            const auto dict = d.cast<py::dict>();
+            blocks.emplace_back(dict, derived);
+            first.push_back(entries.size());
+            entries.emplace_back(dict);
+            for (const char* name : {"ffn_fp8", "ffn_fp8_folded"})
+                if (dict.contains(name)) entries.emplace_back(dict[name].attr("__dict__").cast<py::dict>());
+        }
+    }
+    bool serves(const py::list& dicts) const {
+        if (dicts.size() != blocks.size()) return false;
+        for (size_t i = 0; i < first.size(); ++i)
+            if (!entries[first[i]].of(PyList_GET_ITEM(dicts.ptr(), static_cast<Py_ssize_t>(i)))) return false;
+        return std::all_of(entries.begin(), entries.end(), [](const Entries& e) { return e.same(); }) && derived.unchanged();
     }
 };
 
@@ -127,19 +204,39 @@ public:
         : d_(field<int64_t>(cfg, "d")), heads_(field<int64_t>(cfg, "heads")), ns_(field<int64_t>(cfg, "ns")), emb_(field<int64_t>(cfg, "emb")),
           ffn_(field<int>(cfg, "ffn")), status_(field<Tensor>(cfg, "status")), edges_(field<Tensor>(cfg, "edges")),
           final_norm_(field<Tensor>(cfg, "final_norm")), head_w_(field<Tensor>(cfg, "head_w")), head_b_(field<Tensor>(cfg, "head_b")),
-          classifier_(layer_field(cfg, "classifier_w", "classifier_b")), classifier_f32_(optional_field(cfg, "classifier_w32")),
-          project_(layer_field(cfg, "project_w", "project_b")), ln_w_(field<Tensor>(cfg, "ln_w")), ln_b_(field<Tensor>(cfg, "ln_b")),
+          classifier_(layer_field(cfg, "classifier_w", "classifier_b", derived_)), classifier_f32_(optional_field(cfg, "classifier_w32")),
+          project_(layer_field(cfg, "project_w", "project_b", derived_)), ln_w_(field<Tensor>(cfg, "ln_w")), ln_b_(field<Tensor>(cfg, "ln_b")),
           time_table_(optional_field(cfg, "time_table")), hash_buckets_(field<Tensor>(cfg, "hash_buckets")) {
         for (const auto& t : cfg["seq_tables"]) seq_tables_.push_back(t.cast<OptTensor>());
         type_ = final_norm_.scalar_type();
         device_ = final_norm_.device();
         stats_.emplace(cfg["stats"].cast<py::dict>());
         if (cfg.contains("user") && !cfg["user"].is_none()) {
-            user_.emplace(cfg["user"].cast<py::dict>());
-            item_.emplace(cfg["item"].cast<py::dict>());
+            user_.emplace(cfg["user"].cast<py::dict>(), derived_);
+            item_.emplace(cfg["item"].cast<py::dict>(), derived_);
             if (!cfg["user_dense"].is_none()) user_dense_.emplace(cfg["user_dense"].cast<py::dict>());
             if (!cfg["item_dense"].is_none()) item_dense_.emplace(cfg["item_dense"].cast<py::dict>());
         }
+        weights_ = cfg["weights"].cast<py::dict>();
+        for (const auto& name : cfg["watched"]) {
+            const py::object value = weights_[name];
+            watched_.emplace_back(py::reinterpret_borrow<py::object>(name), value);
+            derived_.watch(value.cast<Tensor>());
+        }
+    }
+
+    // Are the weights that were cast, transposed or split for this executor still those of the model, with the same content?
+    bool current() const {
+        for (const auto& [name, value] : watched_)
+            if (PyDict_GetItem(weights_.ptr(), name.ptr()) != value.ptr()) return false;
+        return derived_.unchanged();
+    }
+
+    // The blocks of these dicts, read again where an entry, or the content of a weight that was converted, has changed.  The caller
+    // holds on to the set: another thread may load the next one while this forward waits without the interpreter's lock.
+    std::shared_ptr<BlockSet> load_blocks(const py::list& dicts) {
+        if (loaded_ == nullptr || !loaded_->serves(dicts)) loaded_ = std::make_shared<BlockSet>(dicts);
+        return loaded_;
     }
 
     bool assembles_ns_tokens() const { return user_.has_value(); }
@@ -236,18 +333,10 @@ private:
         return *out;
     }
 
-    void load_blocks(const py::list& dicts) {
-        size_t entries = 0;
-        for (const auto& d : dicts) entries += py::len(d);
-        if (entries == block_entries_ && blocks_.size() == dicts.size()) return;
-        blocks_.clear();
-        for (const auto& d : dicts) blocks_.emplace_back(d.cast<py::dict>());
-        block_entries_ = entries;
-    }
-
     Tensor native_ns_tokens(const py::tuple& entities, const Prepared& p);
     Tensor shared_ffn(const Block& blk, const Tensor& x, const Tensor& tokens, bool folded) const;
 
+    Derived derived_;                 // before the members that are made with it
     int64_t d_, heads_, ns_, emb_;
     int ffn_;
     Tensor status_, edges_, final_norm_, head_w_, head_b_;
@@ -262,8 +351,9 @@ private:
     at::Device device_{at::kCUDA};
     std::optional<SmallToken> stats_, user_dense_, item_dense_;
     std::optional<EntityTokens> user_, item_;
-    std::vector<Block> blocks_;
-    size_t block_entries_ = 0;
+    std::shared_ptr<BlockSet> loaded_;
+    py::dict weights_;                                        // the model's weights by name
+    std::vector<std::pair<py::object, py::object>> watched_;  // names and tensors of those that were converted for this executor
     std::vector<Tensor> ring_;
     size_t ring_next_ = 0;
 };
@@ -382,12 +472,13 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
                          bool select_early, bool one_kernel, int attention_kernel, bool timing) {
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
-    load_blocks(block_dicts);
+    const auto loaded = load_blocks(block_dicts);
+    const std::vector<Block>& stack = loaded->blocks;
     const Tensor values = i64(values_in), request = i64(request_in);
     const int64_t b = p->batch, n_feat = values.size(1), max_len = values.size(2);
     TORCH_CHECK(n_feat == static_cast<int64_t>(seq_tables_.size()), "OneTransInference: ", seq_tables_.size(), " sequence features expected, got ", n_feat);
     const auto& widths = p->widths;
-    const auto layers = static_cast<int64_t>(blocks_.size());
+    const auto layers = static_cast<int64_t>(stack.size());
     // the non-sequence tokens need nothing the host has to wait for
     const Tensor ns_tokens = (ns_tokens_in.has_value() ? *ns_tokens_in : native_ns_tokens(entities, *p)).contiguous();
     {   // the one host read of a forward; already there when the serving loop prepared the batch ahead of time
@@ -441,7 +532,7 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
     Tensor first_src;
     if (first_kept) first_src = kept_rows(0, &row_dst);
     const int64_t rows_out = first_kept ? totals[1] : total0;
-    const Tensor& first_norm = blocks_[0].attn_norm;
+    const Tensor& first_norm = stack[0].attn_norm;
     const Tensor& table_a = has_time ? *time_table_ : positions;
     const int64_t* ids_a = has_time ? data<int64_t>(buckets) : data<int64_t>(pos);
     Tensor tokens = make({rows_out, d_}, type_, device_), x = make({total0, d_}, type_, device_);
@@ -491,7 +582,7 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
         return m.as_strided({m.size(0), heads_, hd}, {m.size(1), hd, 1}, m.storage_offset() + part * d_);
     };
     for (int64_t l = 0; l < layers; ++l) {
-        const Block& blk = blocks_[l];
+        const Block& blk = stack[l];
         const bool g = blk.grouped_layers;
         if (max_rows[l] == ns_)   // no sample has a sequence token left from here on
             return py::make_tuple(false, tokens, l, false, py::none(), py::none());
@@ -594,11 +685,12 @@ Tensor Engine::ns_only(const Tensor& tokens, int64_t first_layer, int64_t batch,
                        bool timing) {
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
-    load_blocks(block_dicts);
+    const auto loaded = load_blocks(block_dicts);
+    const std::vector<Block>& stack = loaded->blocks;
     const int64_t hd = d_ / heads_;
     Tensor tok = (token_major ? tokens : tokens.view({batch, ns_, d_}).transpose(0, 1)).contiguous().view({ns_, batch, d_});
-    for (size_t l = static_cast<size_t>(first_layer); l < blocks_.size(); ++l) {
-        const Block& blk = blocks_[l];
+    for (size_t l = static_cast<size_t>(first_layer); l < stack.size(); ++l) {
+        const Block& blk = stack[l];
         const bool g = blk.grouped_layers;
         const Tensor qkv = g ? norm_grouped(tok, blk.attn_norm, std::nullopt, blk.g_qkv_w, blk.g_qkv_b, false, status_)
                              : bias_act_rows(at::bmm(rms_norm(tok, blk.attn_norm), blk.ns_qkv_w), blk.ns_qkv_b, false);
@@ -679,6 +771,8 @@ void bind_engine(PyObject* module) {
         .def("tensors", &Prepared::tensors);
     py::class_<Engine>(m, "Engine")
         .def(py::init<py::dict>())
+        .def("current", &Engine::current)
+        .def("load_blocks", [](Engine& e, const py::list& dicts) { e.load_blocks(dicts); })
         .def("assembles_ns_tokens", &Engine::assembles_ns_tokens)
         .def("prepare", &Engine::prepare)
         .def("blocks", &Engine::blocks)

@@ -642,8 +642,10 @@ class OneTransInference:
                 "gamma": self._p(prefix + ".project.2.weight"), "beta": self._p(prefix + ".project.2.bias")}
 
     def _executor(self):
-        """The native executor of the packed layout (built on first use; it shares this engine's weights)."""
-        if self._native is not None:
+        """The native executor of the packed layout, built on first use.  It reads this engine's weights where they are; what it
+        had to convert (casts, transposes, the three-part split of fp32 weights) is made again when a weight has been replaced or
+        changed in place since."""
+        if self._native is not None and self._native.current():
             return self._native
         spec = self.spec
         domain = self.domains[0]
@@ -669,6 +671,10 @@ class OneTransInference:
             "time_table": self._p(time_key) if time_key in self.w else None, "hash_buckets": buckets,
             "seq_tables": [table for _kind, table in entries], "stats": self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2"),
         }
+        # weights that are converted above, by the names under which they can change
+        layers = [f"{name}.{i}" for name in ("classifier", "sequence_stats_projector", "user_dense.project", "item_dense.project",
+                                             prefix + ".project", "user_tokenizer.project", "item_tokenizer.project") for i in (0, 2, 3)]
+        config.update(weights=self.w, watched=[f"{name}.{kind}" for name in layers for kind in ("weight", "bias") if f"{name}.{kind}" in self.w])
         if user is not None and item is not None and fits:
             config.update(user=user, item=item, user_dense=dense["user_dense"], item_dense=dense["item_dense"])
         self._native = _lib.native().Engine(config)

@@ -5,6 +5,7 @@
 //
 // The algorithm and its row layout are described at OneTransInference in onetrans.py; the comments here name the steps.
 #include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <pybind11/stl.h>
 
@@ -26,7 +27,8 @@ OptTensor optional_field(const py::dict& d, const char* name) {
 }
 
 // Tensors made from weights on one stream (three-part splits, casts).  They hold for as long as their sources keep their content,
-// which the sources' version counters tell.
+// which the sources' version counters tell, and a call on another stream is ordered behind their kernels by an event and noted
+// with the allocator, so that they outlive it.
 class Derived {
 public:
     // the form of a weight that this library's GEMM reads
@@ -35,9 +37,24 @@ public:
     void watch(const Tensor& source) {
         sources_.push_back({source, version(source), source.defined() ? source.data_ptr() : nullptr});
     }
+    void keep(const Tensor& t) { made_.push_back(t); }
+    // everything was enqueued on the current stream
+    void seal(const at::Device& device) {
+        stream_ = c10::cuda::getCurrentCUDAStream(device.index()).unwrap();
+        ready_.record(c10::cuda::CUDAStream(*stream_));
+    }
     bool unchanged() const {
         return std::all_of(sources_.begin(), sources_.end(), [](const Source& s) { return version(s.t) == s.version && s.t.data_ptr() == s.data; });
     }
+    // before the current stream reads them
+    void use(const at::Device& device) {
+        const auto current = c10::cuda::getCurrentCUDAStream(device.index());
+        if (current.unwrap() == *stream_ || std::find(users_.begin(), users_.end(), current.unwrap()) != users_.end()) return;
+        ready_.block(current);
+        for (const Tensor& t : made_) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), current);
+        users_.push_back(current.unwrap());
+    }
+
 private:
     struct Source {
         Tensor t;
@@ -48,10 +65,15 @@ private:
     Tensor made_from(const Tensor& source, Tensor t) {
         if (t.defined() && !t.is_same(source)) {
             watch(source);
+            keep(t);
         }
         return t;
     }
     std::vector<Source> sources_;
+    std::vector<Tensor> made_;
+    std::vector<c10::Stream> users_;
+    std::optional<c10::Stream> stream_;
+    at::cuda::CUDAEvent ready_;
 };
 
 // The entries of a dict at one time.  It holds the objects, so that an equal address is the same object.
@@ -169,7 +191,7 @@ struct BlockSet {
     std::vector<Entries> entries;      // a block's dict, then those of its FFN weight objects
     std::vector<size_t> first;         // a block's place in `entries`
     Derived derived;
-    explicit BlockSet(const py::list& dicts) {
+    explicit BlockSet(const py::list& dicts, const at::Device& device) {
         for (const auto& d : dicts) {
             const auto dict = d.cast<py::dict>();
             blocks.emplace_back(dict, derived);
@@ -178,6 +200,7 @@ struct BlockSet {
             for (const char* name : {"ffn_fp8", "ffn_fp8_folded"})
                 if (dict.contains(name)) entries.emplace_back(dict[name].attr("__dict__").cast<py::dict>());
         }
+        derived.seal(device);
     }
     bool serves(const py::list& dicts) const {
         if (dicts.size() != blocks.size()) return false;
@@ -217,12 +240,14 @@ public:
             if (!cfg["user_dense"].is_none()) user_dense_.emplace(cfg["user_dense"].cast<py::dict>());
             if (!cfg["item_dense"].is_none()) item_dense_.emplace(cfg["item_dense"].cast<py::dict>());
         }
+        keep_tensors(cfg);
         weights_ = cfg["weights"].cast<py::dict>();
         for (const auto& name : cfg["watched"]) {
             const py::object value = weights_[name];
             watched_.emplace_back(py::reinterpret_borrow<py::object>(name), value);
             derived_.watch(value.cast<Tensor>());
         }
+        derived_.seal(device_);
     }
 
     // Are the weights that were cast, transposed or split for this executor still those of the model, with the same content?
@@ -235,7 +260,9 @@ public:
     // The blocks of these dicts, read again where an entry, or the content of a weight that was converted, has changed.  The caller
     // holds on to the set: another thread may load the next one while this forward waits without the interpreter's lock.
     std::shared_ptr<BlockSet> load_blocks(const py::list& dicts) {
-        if (loaded_ == nullptr || !loaded_->serves(dicts)) loaded_ = std::make_shared<BlockSet>(dicts);
+        if (loaded_ == nullptr || !loaded_->serves(dicts)) loaded_ = std::make_shared<BlockSet>(dicts, device_);
+        loaded_->derived.use(device_);
+        derived_.use(device_);
         return loaded_;
     }
 
@@ -331,6 +358,13 @@ private:
         if (!out.has_value()) return y;
         out->copy_(y);
         return *out;
+    }
+
+    void keep_tensors(const py::dict& d) {
+        for (const auto& item : d) {
+            if (THPVariable_Check(item.second.ptr())) derived_.keep(item.second.cast<Tensor>());
+            else if (py::isinstance<py::dict>(item.second) && item.first.cast<std::string>() != "weights") keep_tensors(item.second.cast<py::dict>());
+        }
     }
 
     Tensor native_ns_tokens(const py::tuple& entities, const Prepared& p);
@@ -739,6 +773,7 @@ py::tuple Engine::classify(const OptTensor& seq_mean, const Tensor& ns_mean, boo
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
     const int64_t b = ns_mean.size(0), actions = head_w_.size(0);
+    derived_.use(device_);
     const bool own = classifier_.own.defined();
     Tensor joined = make({b, 2 * d_}, at::kFloat, device_), h;
     OptTensor joined_cast;

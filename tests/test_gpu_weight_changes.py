@@ -1,4 +1,4 @@
-"""Weights that change under a model that has scored already: scores are those of a model
+"""Weights that change under a model that has scored already, and first calls on several streams: scores are those of a model
 built from the present weights.  The forward keeps casts, transposes and three-part splits of weights; none of them may outlive the
 tensor, or the content, it was made from."""
 from __future__ import annotations
@@ -98,3 +98,24 @@ def test_weights_replaced_by_name_are_read(name):
     assert not torch.equal(expected, first)
     assert torch.equal(model.scores(batch), expected)
 
+
+@pytest.mark.parametrize("order", ["prepare", "scores"])
+def test_first_calls_on_two_streams(order):
+    """The first call enqueues the splits of the weights behind 20 ms of other work on its stream; a call on another stream has to wait
+    for them."""
+    spec, batch = _spec(), _batch()
+    weights = random_state_dict(spec, seed=5, device="cuda", dtype=torch.float32)
+    expected = _model(spec, weights, torch.float32).scores(batch).clone()
+    for _ in range(3):
+        model = _model(spec, weights, torch.float32)
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(40_000_000)
+            if order == "prepare":
+                model.prepare(batch)                              # converts what lies outside the blocks
+            else:
+                model._executor().load_blocks(model.blocks)       # and the blocks
+        got = model.scores(batch)
+        torch.cuda.synchronize()
+        assert torch.equal(got, expected)

@@ -94,8 +94,11 @@ def _link_host(objs: list[Path], verbose: bool) -> None:
     import torch
 
     torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    # The C++ runtime is torch's shared one, by name: a compiler that has the static library alone would put a second runtime into the
+    # module, and a stream or an exception that crosses between the two ends the process.
     _run([os.environ.get("CXX", "g++"), "-shared", "-o", str(NATIVE_PATH), *map(str, objs), f"-L{PKG_DIR}", "-l:libtb200.so", f"-L{torch_lib}",
-          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"], "link of the host module", verbose)
+          "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-l:libstdc++.so.6", "-Wl,-rpath,$ORIGIN"],
+         "link of the host module", verbose)
 
 
 def build(*, verbose: bool = False, force: bool = False, ptxas_info: bool = False) -> Path:
@@ -116,7 +119,7 @@ def build(*, verbose: bool = False, force: bool = False, ptxas_info: bool = Fals
         proc = subprocess.run(cmd, capture_output=True, text=True)
         if proc.returncode != 0:
             raise RuntimeError(f"link failed:\n{proc.stdout}\n{proc.stderr}")
-    if force or _stale(NATIVE_PATH, [*host_objs, LIB_PATH]):
+    if force or _stale(NATIVE_PATH, [*host_objs, LIB_PATH, Path(__file__)]):
         _link_host(host_objs, verbose)
     return LIB_PATH
 

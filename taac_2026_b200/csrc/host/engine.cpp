@@ -26,6 +26,43 @@ OptTensor optional_field(const py::dict& d, const char* name) {
     return d[name].cast<Tensor>();
 }
 
+// Kernels get the tensors of a record as raw pointers and row counts.  Before the first launch each one that is read has to be on the
+// engine's device with the rows and columns that are read (size -1: any, columns: at least).
+void require(const OptTensor& t, const char* name, const at::Device& device, at::IntArrayRef sizes) {
+    TORCH_CHECK(t.has_value() && t->defined(), "OneTransInference: ", name, " is missing");
+    TORCH_CHECK(t->device() == device, "OneTransInference requires all tensors of a record to live on ", device, ": ", name, " is on ", t->device());
+    bool fits = t->dim() == static_cast<int64_t>(sizes.size());
+    for (size_t i = 0; fits && i < sizes.size(); ++i) fits = sizes[i] < 0 || t->size(static_cast<int64_t>(i)) == sizes[i];
+    TORCH_CHECK(fits, "OneTransInference: ", name, " has shape ", t->sizes(), ", expected ", sizes, " (-1: any)");
+}
+void require_columns(const Tensor& t, const char* name, int64_t columns) {
+    TORCH_CHECK(t.size(1) >= columns, "OneTransInference: ", name, " has ", t.size(1), " columns, ", columns, " are read");
+}
+void check_sequence(const at::Device& device, int64_t batch, int64_t features, int64_t length, const Tensor& values, const OptTensor& lengths,
+                    const OptTensor& stamps, const Tensor& request) {
+    require(values, "values", device, {batch, features, length});
+    if (lengths.has_value()) require(lengths, "lengths", device, {batch});
+    if (stamps.has_value()) require(stamps, "timestamps", device, {batch, length});
+    require(request, "request_timestamp", device, {batch});
+}
+// `fields` > 0: the missing flags of that many fields are read; `dense` > 0: so many dense values
+void check_entity(const at::Device& device, int64_t batch, const Tensor& ids, int64_t id_columns, const OptTensor& missing, int64_t fields,
+                  const OptTensor& values, const OptTensor& values_missing, int64_t dense) {
+    require(ids, "int_values", device, {batch, -1});
+    require_columns(ids, "int_values", id_columns);
+    if (fields > 0) {
+        require(missing, "int_missing_mask", device, {batch, -1});
+        require_columns(*missing, "int_missing_mask", fields);
+    }
+    if (dense > 0) {
+        require(values, "dense_values", device, {batch, dense});
+        if (values_missing.has_value()) {
+            require(values_missing, "dense_missing_mask", device, {batch, -1});
+            require_columns(*values_missing, "dense_missing_mask", dense);
+        }
+    }
+}
+
 // Tensors made from weights on one stream (three-part splits, casts).  They hold for as long as their sources keep their content,
 // which the sources' version counters tell, and a call on another stream is ordered behind their kernels by an event and noted
 // with the allocator, so that they outlive it.
@@ -109,8 +146,10 @@ Layer layer_field(const py::dict& d, const std::string& w, const std::string& b3
 // LayerNorm(SiLU(W [values, mask] + b)) of a small fp32 input, all fp32
 struct SmallToken {
     Tensor w, b, gamma, beta;
+    int64_t inputs;    // values of a row; the weight has as many columns again for their missing flags where there are such
     explicit SmallToken(const py::dict& d)
-        : w(field<Tensor>(d, "w")), b(field<Tensor>(d, "b")), gamma(field<Tensor>(d, "gamma")), beta(field<Tensor>(d, "beta")) {}
+        : w(field<Tensor>(d, "w")), b(field<Tensor>(d, "b")), gamma(field<Tensor>(d, "gamma")), beta(field<Tensor>(d, "beta")),
+          inputs(field<int64_t>(d, "inputs")) {}
     // writes [rows, d] at `out` (out_stride elements between rows)
     void run(const Tensor& values, const OptTensor& mask, void* out, int64_t out_stride, at::ScalarType type) const {
         const int64_t n = values.size(1), in_dim = w.size(0);
@@ -128,12 +167,13 @@ struct EntityTokens {
     OptTensor missing_rows;
     Layer project;
     Tensor gamma, beta;
-    int64_t n_fields, max_bag, dim, n_tokens;
+    int64_t n_fields, max_bag, dim, n_tokens, id_columns;
     EntityTokens(const py::dict& d, Derived& derived)
         : ptrs(field<Tensor>(d, "ptrs")), rows(field<Tensor>(d, "rows")), offsets(field<Tensor>(d, "offsets")), lengths(field<Tensor>(d, "lengths")),
           missing_rows(optional_field(d, "missing_rows")), project(layer_field(d, "w", "b32", derived)), gamma(field<Tensor>(d, "gamma")),
           beta(field<Tensor>(d, "beta")), n_fields(field<int64_t>(d, "n_fields")), max_bag(field<int64_t>(d, "max_bag")),
-          dim(field<int64_t>(d, "dim")), n_tokens(field<int64_t>(d, "n_tokens")) {}
+          dim(field<int64_t>(d, "dim")), n_tokens(field<int64_t>(d, "n_tokens")),
+          id_columns(field<int64_t>(d, "id_columns")) {}
 };
 
 struct Block {
@@ -212,7 +252,7 @@ struct BlockSet {
 
 // What `prepare` leaves for the forward of the same batch
 struct Prepared {
-    int64_t batch = 0;
+    int64_t batch = 0, length = 0;
     std::vector<int64_t> widths;
     Tensor src_map, stats, start, n0, counts, cu, cu32, ns_rows, meta;   // meta: pinned host memory
     at::cuda::CUDAEvent ready;
@@ -274,13 +314,15 @@ public:
                                       std::vector<int64_t> widths, bool timing) {
         Timing::on() = timing;
         const c10::cuda::CUDAGuard guard(device_);
+        TORCH_CHECK(values_in.dim() == 3 && values_in.size(1) >= 1 && values_in.size(2) >= 1 && values_in.size(2) <= 8192,
+                    "sequence_prepare needs values [B, F, L] with at least one feature and 1 <= L <= 8192");
+        check_sequence(device_, values_in.size(0), -1, values_in.size(2), values_in, lengths_in, stamps_in, request_in);
         const Tensor values = i64(values_in), lengths = i64(lengths_in), stamps = i64(stamps_in), request = i64(request_in);
-        TORCH_CHECK(values.dim() == 3 && stamps.dim() == 2 && lengths.dim() == 1 && values.is_cuda() && values.size(1) >= 1 && values.size(2) >= 1 &&
-                        values.size(2) <= 8192, "sequence_prepare needs int64 values [B, F, L] on the GPU with at least one feature and 1 <= L <= 8192");
         const int64_t b = values.size(0), f = values.size(1), len = values.size(2);
         const auto layers = static_cast<int64_t>(widths.size()) - 1;
         auto p = std::make_shared<Prepared>();
         p->batch = b;
+        p->length = len;
         p->widths = std::move(widths);
         Tensor new_len = make({b}, at::kLong, device_);
         p->src_map = make({b, len}, at::kInt, device_);
@@ -508,9 +550,21 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
     const c10::cuda::CUDAGuard guard(device_);
     const auto loaded = load_blocks(block_dicts);
     const std::vector<Block>& stack = loaded->blocks;
+    const int64_t b = p->batch, n_feat = static_cast<int64_t>(seq_tables_.size()), max_len = p->length;
+    check_sequence(device_, b, n_feat, max_len, values_in, std::nullopt, time_table_.has_value() ? stamps_in : std::nullopt, request_in);
+    if (ns_tokens_in.has_value()) {
+        require(ns_tokens_in, "ns_tokens", device_, {b, ns_, d_});
+    } else {
+        for (int who = 0; who < 2; ++who) {
+            const EntityTokens& e = who == 0 ? *user_ : *item_;
+            const auto& dense = who == 0 ? user_dense_ : item_dense_;
+            const py::tuple parts = entities[who].cast<py::tuple>();
+            const auto optional = [&](int i) { return parts[i].is_none() ? OptTensor() : OptTensor(parts[i].cast<Tensor>()); };
+            check_entity(device_, b, parts[0].cast<Tensor>(), e.id_columns, optional(1), e.missing_rows.has_value() ? e.n_fields : 0, optional(2),
+                         optional(3), dense.has_value() ? dense->inputs : 0);
+        }
+    }
     const Tensor values = i64(values_in), request = i64(request_in);
-    const int64_t b = p->batch, n_feat = values.size(1), max_len = values.size(2);
-    TORCH_CHECK(n_feat == static_cast<int64_t>(seq_tables_.size()), "OneTransInference: ", seq_tables_.size(), " sequence features expected, got ", n_feat);
     const auto& widths = p->widths;
     const auto layers = static_cast<int64_t>(stack.size());
     // the non-sequence tokens need nothing the host has to wait for
@@ -799,6 +853,8 @@ py::tuple Engine::classify(const OptTensor& seq_mean, const Tensor& ns_mean, boo
 
 void bind_engine(PyObject* module) {
     auto m = py::reinterpret_borrow<py::module_>(module);
+    m.def("check_sequence", &check_sequence);
+    m.def("check_entity", &check_entity);
     py::class_<Prepared, std::shared_ptr<Prepared>>(m, "Prepared")
         .def_readonly("batch", &Prepared::batch)
         .def_readonly("widths", &Prepared::widths)

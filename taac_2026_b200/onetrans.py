@@ -622,12 +622,13 @@ class OneTransInference:
         """Device tensors of a ``prepare`` result (for ``Tensor.record_stream`` when it was made on another stream)."""
         return prepared.tensors()
 
-    def _small_token(self, linear: str, norm: str) -> dict:
+    def _small_token(self, linear: str, norm: str, inputs: int) -> dict:
         """Linear -> SiLU -> LayerNorm of a handful of fp32 inputs, kept in fp32."""
         f32 = lambda name: self.w[name].float().contiguous()  # noqa: E731
-        return {"w": f32(linear + ".weight").t().contiguous(), "b": f32(linear + ".bias"), "gamma": f32(norm + ".weight"), "beta": f32(norm + ".bias")}
+        return {"w": f32(linear + ".weight").t().contiguous(), "b": f32(linear + ".bias"), "gamma": f32(norm + ".weight"), "beta": f32(norm + ".bias"),
+                "inputs": inputs}
 
-    def _entity_tokens(self, prefix: str, bank: _Bank, n_tokens: int, groups) -> dict | None:
+    def _entity_tokens(self, prefix: str, bank: _Bank, specs, n_tokens: int, groups) -> dict | None:
         """What the executor needs to build an entity's tokens itself: one projection of all pooled fields.  None for the other
         forms (hashed ids, tokens per group, no fields), which `_ns_tokens` builds."""
         n_groups = len(list(groups)) or bank.n_fields
@@ -637,7 +638,8 @@ class OneTransInference:
         key = prefix + ".missing_embeddings"
         f = bank.fields
         return {"ptrs": f.ptrs, "rows": f.rows, "offsets": f.offsets, "lengths": f.lengths, "n_fields": f.n_fields, "max_bag": f.max_bag,
-                "dim": f.dim, "n_tokens": n_tokens, "missing_rows": self._p(key)[: f.n_fields].contiguous() if key in self.w else None,
+                "dim": f.dim, "n_tokens": n_tokens, "id_columns": max(offset + length for _vocab, offset, length in specs if length > 0),
+                "missing_rows": self._p(key)[: f.n_fields].contiguous() if key in self.w else None,
                 "w": self._p(prefix + ".project.0.weight"), "b32": self.w[prefix + ".project.0.bias"].float().contiguous(),
                 "gamma": self._p(prefix + ".project.2.weight"), "beta": self._p(prefix + ".project.2.bias")}
 
@@ -654,9 +656,9 @@ class OneTransInference:
         buckets = torch.tensor([-1 if table is None else (table.shape[0] - 1 if kind == "compressed" else 0) for kind, table in entries],
                                dtype=torch.long, device=self.device)
         time_key = prefix + ".time_embedding.weight"
-        user = self._entity_tokens("user_tokenizer", self.user_bank, self.user_tokens, spec.user_ns_groups)
-        item = self._entity_tokens("item_tokenizer", self.item_bank, self.item_tokens, spec.item_ns_groups)
-        dense = {name: self._small_token(name + ".project.0", name + ".project.2") if dim > 0 else None
+        user = self._entity_tokens("user_tokenizer", self.user_bank, spec.user_int_specs, self.user_tokens, spec.user_ns_groups)
+        item = self._entity_tokens("item_tokenizer", self.item_bank, spec.item_int_specs, self.item_tokens, spec.item_ns_groups)
+        dense = {name: self._small_token(name + ".project.0", name + ".project.2", dim) if dim > 0 else None
                  for name, dim in (("user_dense", spec.user_dense_dim), ("item_dense", spec.item_dense_dim))}
         fits = all(t is None or 8 * (t["w"].shape[0] + self.d) * 4 <= 48 * 1024 for t in dense.values())
         modes = {"bf16": 0, "fp8": 2 if self.ffn_precise else (3 if self.ffn_mx else 1)}
@@ -669,7 +671,7 @@ class OneTransInference:
             "project_w": self._p(prefix + ".project.0.weight"), "project_b": self.w[prefix + ".project.0.bias"].float().contiguous(),
             "ln_w": self._p(prefix + ".project.2.weight"), "ln_b": self._p(prefix + ".project.2.bias"),
             "time_table": self._p(time_key) if time_key in self.w else None, "hash_buckets": buckets,
-            "seq_tables": [table for _kind, table in entries], "stats": self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2"),
+            "seq_tables": [table for _kind, table in entries], "stats": self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2", 6),
         }
         # weights that are converted above, by the names under which they can change
         layers = [f"{name}.{i}" for name in ("classifier", "sequence_stats_projector", "user_dense.project", "item_dense.project",

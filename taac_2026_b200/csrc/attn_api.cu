@@ -93,7 +93,6 @@ extern "C" int tb200_attn_last_rows_fwd(const void* q, const void* k, const void
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return TB200_ERR_ALIGN;
     for (int i = 0; i < 12; ++i)
         if (strides[i] % 8 != 0) return TB200_ERR_ALIGN;
-    if (B > 65535) return TB200_ERR_UNSUPPORTED;
     if (!device_info().valid) return TB200_ERR_DEVICE;
     AttnArgs a{};
     a.q = q; a.k = k; a.v = v; a.o = o;

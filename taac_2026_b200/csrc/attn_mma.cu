@@ -778,7 +778,8 @@ static int fewq_split(const AttnArgs& a, cudaStream_t stream) {
 }
 int attn_fewq_forward(const AttnArgs& a, int dtype, cudaStream_t stream) {
     const int64_t pairs = static_cast<int64_t>(a.B) * a.H;
-    // below one resident set of warps (16 per SM) the keys of a (sample, head) are split; 8-byte stores need aligned rows
+    // below one resident set of warps (16 per SM) the keys of a (sample, head) are split (so few samples fit a grid's y dimension); 8-byte
+    // stores need aligned rows
     const bool wide_rows = ((a.o_sl | a.o_sh | a.o_sb) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.o) & 7) == 0;
     if (pairs < 16ll * device_info().sm_count && wide_rows && a.Lq > 0)
         return dtype == TB200_BF16 ? fewq_split<__nv_bfloat16>(a, stream) : fewq_split<__half>(a, stream);

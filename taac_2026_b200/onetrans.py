@@ -660,7 +660,9 @@ class OneTransInference:
         item = self._entity_tokens("item_tokenizer", self.item_bank, spec.item_int_specs, self.item_tokens, spec.item_ns_groups)
         dense = {name: self._small_token(name + ".project.0", name + ".project.2", dim) if dim > 0 else None
                  for name, dim in (("user_dense", spec.user_dense_dim), ("item_dense", spec.item_dense_dim))}
-        fits = all(t is None or 8 * (t["w"].shape[0] + self.d) * 4 <= 48 * 1024 for t in dense.values())
+        stats = self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2", 6)
+        # the kernel of the small tokens keeps eight rows of inputs and outputs in 48 KB; wider ones are built by `_ns_tokens`
+        fits = all(t is None or 8 * (t["w"].shape[0] + self.d) * 4 <= 48 * 1024 for t in (stats, *dense.values()))
         modes = {"bf16": 0, "fp8": 2 if self.ffn_precise else (3 if self.ffn_mx else 1)}
         config = {
             "d": self.d, "heads": self.heads, "ns": self.num_ns, "emb": spec.emb_dim, "ffn": modes[self.ffn_mode], "status": self.status_word,
@@ -671,7 +673,7 @@ class OneTransInference:
             "project_w": self._p(prefix + ".project.0.weight"), "project_b": self.w[prefix + ".project.0.bias"].float().contiguous(),
             "ln_w": self._p(prefix + ".project.2.weight"), "ln_b": self._p(prefix + ".project.2.bias"),
             "time_table": self._p(time_key) if time_key in self.w else None, "hash_buckets": buckets,
-            "seq_tables": [table for _kind, table in entries], "stats": self._small_token("sequence_stats_projector.0", "sequence_stats_projector.2", 6),
+            "seq_tables": [table for _kind, table in entries], "stats": stats,
         }
         # weights that are converted above, by the names under which they can change
         layers = [f"{name}.{i}" for name in ("classifier", "sequence_stats_projector", "user_dense.project", "item_dense.project",

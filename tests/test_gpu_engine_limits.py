@@ -30,3 +30,15 @@ def test_more_samples_than_a_grid_dimension():
     values = torch.where(torch.arange(seq.values.shape[2], device="cuda") < lens[:, None, None], seq.values, 0)
     batch = dataclasses.replace(batch, sequences={"seq_a": dataclasses.replace(seq, values=values, lengths=lens)})
     assert torch.equal(model.scores(batch), model.scores(batch, micro_batch=20_000))
+
+
+@pytest.mark.parametrize("dense", [0, 4])
+def test_wide_model_without_dense_features(dense):
+    """d_model 1536: the statistics token does not fit the small-token kernel, whether or not there are dense ones.  The padded layout
+    computes the same scores with other kernels: bf16 results around one half, a few units of 2^-9 of the logits apart."""
+    spec = dataclasses.replace(_spec(1536, heads=24, dense=dense), num_blocks=1, user_ns_tokens=1, item_ns_tokens=1)
+    weights = random_state_dict(spec, seed=2, device="cuda", dtype=torch.bfloat16)
+    batch = _batch(9, dense=dense)
+    got = OneTransInference(weights, spec, dtype=torch.bfloat16).scores(batch)
+    want = OneTransInference(weights, spec, dtype=torch.bfloat16, packed=False).scores(batch)
+    torch.testing.assert_close(got, want, rtol=0, atol=4e-3)

@@ -35,6 +35,11 @@ int64_t integer(PyObject* o) {
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
+bool truth(PyObject* o) {   // as `if o:` takes it
+    const int v = PyObject_IsTrue(o);
+    if (v < 0) throw python_error();
+    return v != 0;
+}
 // a tensor or None?
 bool is_optional(PyObject* o) { return o == Py_None || THPVariable_Check(o); }
 
@@ -136,7 +141,7 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* args, Py_ssize_t) {
     const Tensor& w = tensor(args[1]);
     const Tensor& b = tensor(args[2]);
     const double eps = number(args[3]);
-    const bool pre_silu = args[4] == Py_True;
+    const bool pre_silu = truth(args[4]);
     if (x.dim() < 2 || w.dim() != 1 || b.dim() != 1 || x.size(-1) != w.size(0) || x.size(-1) != b.size(0) || x.size(-1) < 1 ||
         dtype_code(x.scalar_type()) < 0 || !dense(x, x.scalar_type()) || !dense(w, x.scalar_type()) || !dense(b, x.scalar_type()) ||
         x.device() != w.device() || x.device() != b.device())
@@ -295,7 +300,7 @@ PyObject* py_varlen_attention(PyObject*, PyObject* const* args, Py_ssize_t) {
     const Tensor& q = tensor(args[0]);
     const Tensor& k = tensor(args[1]);
     const Tensor& v = tensor(args[2]);
-    const bool token_major = args[8] == Py_True;
+    const bool token_major = truth(args[8]);
     const int hd = token_major ? 2 : 1, ld = token_major ? 1 : 2;
     if (!attention_operands(q, k, v) || q.size(hd) != k.size(hd)) Py_RETURN_NONE;
     Mask mask;
@@ -308,8 +313,8 @@ PyObject* py_varlen_attention(PyObject*, PyObject* const* args, Py_ssize_t) {
     }
     if (status.has_value() && (status->scalar_type() != at::kInt || status->numel() != 1)) Py_RETURN_NONE;
     mask.ns_start = args[4] == Py_None ? k.size(ld) : integer(args[4]);
-    mask.causal = PyObject_IsTrue(args[5]);
-    mask.self_rows = PyObject_IsTrue(args[6]);
+    mask.causal = truth(args[5]);
+    mask.self_rows = truth(args[6]);
     const double scale = args[7] == Py_None ? 1.0 / std::sqrt(static_cast<double>(q.size(3))) : number(args[7]);
     const int kernel = static_cast<int>(integer(args[9]));
     const c10::cuda::CUDAGuard guard(q.device());
@@ -366,7 +371,7 @@ PyObject* py_flash_attention(PyObject*, PyObject* const* args, Py_ssize_t) {
     const Tensor& v = tensor(args[2]);
     if (!attention_operands(q, k, v) || q.size(1) != k.size(1)) Py_RETURN_NONE;
     const auto attn_mask = optional_tensor(args[3]);
-    const bool is_causal = PyObject_IsTrue(args[4]);
+    const bool is_causal = truth(args[4]);
     const bool grad = wants_grad(q) || wants_grad(k) || wants_grad(v);
     if (grad && (q.size(2) > 4096 || k.size(2) > 4096 || q.size(1) > 65535)) Py_RETURN_NONE;
     const c10::cuda::CUDAGuard guard(q.device());
@@ -411,7 +416,7 @@ bool ffn_operands(PyObject* const* args, at::ScalarType up_type, FfnOperands& f)
     f.s_down = tensor(args[5]);
     f.b_down = optional_tensor(args[6]);
     f.hidden = integer(args[7]);
-    f.gated = PyObject_IsTrue(args[8]);
+    f.gated = truth(args[8]);
     f.residual = optional_tensor(args[9]);
     f.status = optional_tensor(args[10]);
     if (x.dim() < 1 || !dense(x, at::kBFloat16) || x.size(-1) < 1 || x.numel() == 0) return false;

@@ -2,6 +2,7 @@
 its 16-byte pieces, and the refusal of masks that neither recognises."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 import torch
 
@@ -54,3 +55,12 @@ def test_one_wrong_element_is_refused(flip):
     mask[b, 0, i, j] ^= True
     with pytest.raises(RuntimeError, match="cuda flash_attention"):
         ops.flash_attention(q, k, v, attn_mask=mask.expand(-1, heads, -1, -1))
+
+
+@pytest.mark.parametrize("flag", [1, True, np.bool_(True)])
+def test_flags_are_read_as_python_reads_them(flag):
+    x, w, b = torch.randn(33, 64, device="cuda"), torch.rand(64, device="cuda"), torch.rand(64, device="cuda")
+    want = torch.nn.functional.layer_norm(torch.nn.functional.silu(x), (64,), w, b, 1e-5)
+    torch.testing.assert_close(ops.layer_norm(x, w, b, pre_silu=flag), want, atol=1e-5, rtol=1e-5)
+    q, k, v = (torch.randn(2, 2, 20, 64, device="cuda").bfloat16() for _ in range(3))
+    assert torch.equal(ops.varlen_attention(q, k, v, causal=flag), ops.varlen_attention(q, k, v, causal=True))

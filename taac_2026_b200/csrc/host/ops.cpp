@@ -438,6 +438,11 @@ bool ffn_operands(PyObject* const* args, at::ScalarType up_type, FfnOperands& f)
     return true;
 }
 
+// the scales of an [n, k] weight: one per 128 x 128 block, `atom` > 0: an atom of so many bytes each
+bool scales_fit(const Tensor& s, const Tensor& w, int64_t atom) {
+    return s.dim() == (atom > 0 ? 3 : 2) && s.size(0) == w.size(0) / 128 && s.size(1) == w.size(1) / 128 && (atom == 0 || s.size(2) == atom);
+}
+
 Tensor ffn_result(const FfnOperands& f) {
     auto sizes = f.x.sizes().vec();
     sizes.back() = f.d_out;
@@ -449,7 +454,8 @@ Tensor ffn_result(const FfnOperands& f) {
 PyObject* ffn_fp8(PyObject* const* args, bool precise) {
     FfnOperands f;
     if (!ffn_operands(args, precise ? at::kBFloat16 : at::kFloat8_e4m3fn, f)) Py_RETURN_NONE;
-    if (!dense(f.s_down, at::kFloat) || (!precise && !dense(f.s_up, at::kFloat))) Py_RETURN_NONE;
+    if (!dense(f.s_down, at::kFloat) || !scales_fit(f.s_down, f.w_down, 0)) Py_RETURN_NONE;
+    if (!precise && (!dense(f.s_up, at::kFloat) || !scales_fit(f.s_up, f.w_up, 0))) Py_RETURN_NONE;
     const c10::cuda::CUDAGuard guard(f.x.device());
     if (!tb200_device_ok()) Py_RETURN_NONE;
     const int64_t d = f.x.size(-1), m = f.x.numel() / d;
@@ -495,7 +501,9 @@ PyObject* py_ffn_fp8_precise(PyObject*, PyObject* const* args, Py_ssize_t) {
 PyObject* py_ffn_mx(PyObject*, PyObject* const* args, Py_ssize_t) {
     HANDLE_TH_ERRORS
     FfnOperands f;
-    if (!ffn_operands(args, at::kFloat8_e4m3fn, f) || !dense(f.s_up, at::kByte) || !dense(f.s_down, at::kByte)) Py_RETURN_NONE;
+    if (!ffn_operands(args, at::kFloat8_e4m3fn, f) || !dense(f.s_up, at::kByte) || !dense(f.s_down, at::kByte) ||
+        !scales_fit(f.s_up, f.w_up, 512) || !scales_fit(f.s_down, f.w_down, 512))
+        Py_RETURN_NONE;
     const c10::cuda::CUDAGuard guard(f.x.device());
     if (!tb200_device_ok()) Py_RETURN_NONE;
     const int64_t d = f.x.size(-1), m = f.x.numel() / d, tiles = (m + 127) / 128;

@@ -64,3 +64,20 @@ def test_flags_are_read_as_python_reads_them(flag):
     torch.testing.assert_close(ops.layer_norm(x, w, b, pre_silu=flag), want, atol=1e-5, rtol=1e-5)
     q, k, v = (torch.randn(2, 2, 20, 64, device="cuda").bfloat16() for _ in range(3))
     assert torch.equal(ops.varlen_attention(q, k, v, causal=flag), ops.varlen_attention(q, k, v, causal=True))
+
+
+@pytest.mark.parametrize("make,call,name", [(ops.Fp8FfnWeights, ops.ffn_fp8, "s"), (ops.MxFfnWeights, ops.ffn_mx, "a")])
+def test_ffn_scales_of_another_shape_are_refused(make, call, name):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(40, 256, device="cuda", generator=g).bfloat16()
+    w = [(0.05 * torch.randn(*s, device="cuda", generator=g)).bfloat16() for s in ((512, 256), (256, 512))]
+    weights = make(*w, gated=False)
+    want = call(x, weights).clone()
+    for attr in (name + "_up", name + "_down"):
+        whole = getattr(weights, attr)
+        for wrong in (whole[:-1].contiguous(), whole[:, :1].contiguous()):
+            setattr(weights, attr, wrong)
+            with pytest.raises(ValueError):
+                call(x, weights)
+        setattr(weights, attr, whole)
+    assert torch.equal(call(x, weights), want)

@@ -30,7 +30,12 @@ double number(PyObject* o) {
     if (v == -1.0 && PyErr_Occurred()) throw python_error();
     return v;
 }
-int64_t integer(PyObject* o) {
+int64_t integer(PyObject* o) {   // as int(o) takes it
+    if (PyFloat_Check(o)) {
+        const double v = PyFloat_AS_DOUBLE(o);
+        TORCH_CHECK_VALUE(std::fabs(v) < 9.2e18, "cannot convert ", v, " to an integer");
+        return static_cast<int64_t>(v);
+    }
     const long long v = PyLong_AsLongLong(o);
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;

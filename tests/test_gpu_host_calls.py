@@ -81,3 +81,11 @@ def test_ffn_scales_of_another_shape_are_refused(make, call, name):
                 call(x, weights)
         setattr(weights, attr, whole)
     assert torch.equal(call(x, weights), want)
+
+
+def test_whole_numbers_may_come_as_floats():
+    q, k, v = (torch.randn(2, 2, 40, 64, device="cuda").bfloat16() for _ in range(3))
+    lens = torch.tensor([12, 30], dtype=torch.int32, device="cuda")
+    assert torch.equal(ops.varlen_attention(q, k, v, seq_len=lens, ns_start=36.0), ops.varlen_attention(q, k, v, seq_len=lens, ns_start=36))
+    ids = torch.randint(0, 50, (9, 4), device="cuda")
+    assert ops.embedding_bag_mean_backward(ids, torch.ones(9, 64, device="cuda"), 50.0).shape == (50, 64)

@@ -218,6 +218,8 @@ class OneTransInference:
             raise RuntimeError("ffn='fp8' needs bf16 activations, d_model % 256 == 0 and hidden % 256 == 0")
         self.ffn_mode = ffn
         self.packed = bool(packed)
+        if self.packed and len(spec.seq_vocab_sizes) == 1:
+            _lib.native()      # the packed forward is enqueued by the host module; say so here if it does not load
         self.d = spec.d_model
         heads = max(1, spec.num_heads)
         if self.d % heads:  # choose_num_heads (modeling/sequence.py:70-78)

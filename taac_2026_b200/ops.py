@@ -79,17 +79,30 @@ def kernel_timing_on() -> bool:
     return _TIMING is not None
 
 
+class _NoHost:
+    """Stands for a host module that does not load: every call is left to the general path."""
+
+    def __getattr__(self, name: str):
+        return lambda *args: None
+
+
 class _LazyHost:
-    """Stands for the host module until the first call."""
+    """Stands for the host module until the first call with the library in place."""
 
     def __getattr__(self, name: str):
         global _host
-        _host = _lib.native()
+        if not _lib.library_available():      # the general path looks at the arguments before it says so
+            return lambda *args: None
+        try:
+            _host = _lib.native()
+        except RuntimeError:
+            _host = _NoHost()
         return getattr(_host, name)
 
 
 # The plain form of an operator call (contiguous CUDA tensors of one type, nothing timed) goes to the host module, which
-# answers None for every other form and for what the library rejects; the code below then handles it or words the error.
+# answers None for every other form and for what the library rejects; the code below then handles it or words the error.  The
+# operators need the C library alone: without the host module they take the code below for every form.
 _host: Any = _LazyHost()
 
 

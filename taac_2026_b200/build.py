@@ -75,12 +75,24 @@ def _run(cmd: list[str], what: str, verbose: bool) -> None:
         raise RuntimeError(f"{what} failed:\n{proc.stdout}\n{proc.stderr}")
 
 
-def _compile_host(src: Path, verbose: bool) -> Path:
+def _host_toolchain() -> Path:
+    """A file that names the torch, the interpreter and the compiler that the host module is built with, rewritten (and so newer than
+    the objects) when one of them changes: a module built against another torch does not load."""
+    import torch
+
+    stamp = BUILD / "host_toolchain.txt"
+    text = f"{torch.__version__} {torch.__file__} {sys.version} {os.environ.get('CXX', 'g++')}\n"
+    if not stamp.exists() or stamp.read_text() != text:
+        stamp.write_text(text)
+    return stamp
+
+
+def _compile_host(src: Path, stamp: Path, verbose: bool) -> Path:
     import torch
     from torch.utils.cpp_extension import include_paths
 
     obj = BUILD / ("host_" + src.stem + ".o")
-    if not _stale(obj, [src, *sorted(HOST.glob("*.h")), *sorted(INCLUDE.glob("*.h")), Path(__file__)]):
+    if not _stale(obj, [src, *sorted(HOST.glob("*.h")), *sorted(INCLUDE.glob("*.h")), Path(__file__), stamp]):
         return obj
     cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
     paths = [*include_paths(), sysconfig.get_paths()["include"], str(cuda_include)]
@@ -108,8 +120,9 @@ def build(*, verbose: bool = False, force: bool = False, ptxas_info: bool = Fals
         for obj in BUILD.glob("*.o"):
             obj.unlink()
     srcs = sources()
+    stamp = _host_toolchain()
     with ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 1)) as pool:
-        host = [pool.submit(_compile_host, s, verbose) for s in sorted(HOST.glob("*.cpp"))]
+        host = [pool.submit(_compile_host, s, stamp, verbose) for s in sorted(HOST.glob("*.cpp"))]
         objs = list(pool.map(lambda s: _compile(s, verbose, ptxas_info), srcs))
         host_objs = [h.result() for h in host]
     if force or _stale(LIB_PATH, objs):
@@ -119,7 +132,7 @@ def build(*, verbose: bool = False, force: bool = False, ptxas_info: bool = Fals
         proc = subprocess.run(cmd, capture_output=True, text=True)
         if proc.returncode != 0:
             raise RuntimeError(f"link failed:\n{proc.stdout}\n{proc.stderr}")
-    if force or _stale(NATIVE_PATH, [*host_objs, LIB_PATH, Path(__file__)]):
+    if force or _stale(NATIVE_PATH, [*host_objs, LIB_PATH, Path(__file__), stamp]):
         _link_host(host_objs, verbose)
     return LIB_PATH
 

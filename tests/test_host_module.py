@@ -1,6 +1,9 @@
 """The host module (``_native.so``): how it is built, and the operators without it."""
 from __future__ import annotations
 
+import time
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -58,3 +61,32 @@ def test_operators_run_without_the_host_module(monkeypatch):
     monkeypatch.setattr(_lib, "native", _unloadable)
     for a, b in zip(results(), want):
         assert torch.equal(a, b)
+
+
+def test_another_torch_makes_the_host_objects_stale(monkeypatch, tmp_path):
+    commands = []
+    monkeypatch.setattr(build, "BUILD", tmp_path)
+
+    def run(cmd, what, verbose):
+        commands.append(what)
+        Path(cmd[-1]).write_bytes(b"")
+
+    monkeypatch.setattr(build, "_run", run)
+    src = next(iter(sorted(build.HOST.glob("*.cpp"))))
+
+    def compiled() -> int:
+        commands.clear()
+        build._compile_host(src, build._host_toolchain(), False)
+        return len(commands)
+
+    assert compiled() == 1
+    assert compiled() == 0
+    time.sleep(0.02)       # file times
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    assert compiled() == 1
+    assert compiled() == 0
+    time.sleep(0.02)
+    monkeypatch.undo()     # back to the first one: its objects are gone
+    monkeypatch.setattr(build, "BUILD", tmp_path)
+    monkeypatch.setattr(build, "_run", run)
+    assert compiled() == 1

@@ -5,6 +5,7 @@
 //
 // The algorithm and its row layout are described at OneTransInference in onetrans.py; the comments here name the steps.
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <pybind11/stl.h>
@@ -368,7 +369,10 @@ public:
                                           data<int64_t>(p->counts), data<int64_t>(p->cu), data<int32_t>(p->cu32), data<int64_t>(p->meta),
                                           data<int64_t>(ns_rows0), data<int64_t>(p->ns_rows), s), "cuda pyramid_plan");
         }
-        p->ready.record(c10::cuda::getCurrentCUDAStream(device_.index()));
+        const auto stream = c10::cuda::getCurrentCUDAStream(device_.index());
+        // the kernel writes the landing buffer: its memory is not given out before, also when nobody waits for the result
+        at::getHostAllocator(at::kCUDA)->record_event(p->meta.data_ptr(), p->meta.storage().data_ptr().get_context(), stream.unwrap());
+        p->ready.record(stream);
         return p;
     }
 

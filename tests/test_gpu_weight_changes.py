@@ -119,3 +119,19 @@ def test_first_calls_on_two_streams(order):
         got = model.scores(batch)
         torch.cuda.synchronize()
         assert torch.equal(got, expected)
+
+
+def test_a_dropped_result_keeps_its_landing_buffer():
+    """The plan kernel of a prepared batch waits behind 20 ms of other work and writes pinned memory; the engine and the result are gone by
+    then.  Pinned tensors that are made in between keep their values."""
+    spec, batch = _spec(), _batch()
+    model = _model(spec, random_state_dict(spec, seed=6, device="cuda", dtype=torch.bfloat16), torch.bfloat16)
+    model.scores(batch)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(40_000_000)
+    for _ in range(4):                      # every buffer of the ring
+        model.prepare(batch)
+    model._native = None
+    taken = [torch.full((2 * (spec.num_blocks + 1),), -7, dtype=torch.int64).pin_memory() for _ in range(16)]
+    torch.cuda.synchronize()
+    assert all(bool((t == -7).all()) for t in taken)

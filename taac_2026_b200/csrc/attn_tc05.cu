@@ -22,13 +22,13 @@
 // Key tiles without a visible key are skipped; masks come as lengths, never as a matrix.
 // Every mbarrier wait is bounded; a wait that gives up raises the status word and all roles drain
 // through the final barrier, where TMEM is released.
-#include <cudaTypedefs.h>
 
 #include <type_traits>
 
 #include "attn_common.cuh"
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -538,23 +538,6 @@ attn_tc05_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess) {
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        } else {
-            cudaGetLastError();
-        }
-    }
-    return fn;
-}
-
 // bf16 tensor addressed as (d, row, head, batch) with element strides (1, sl, sh, sb); tiles of 128 rows x 64
 bool make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t heads, int64_t batch, int64_t sl, int64_t sh,
                int64_t sb) {
@@ -601,7 +584,7 @@ int attn_tc05_forward(const AttnArgs& a, int max_lq, int64_t total_rows, int32_t
     if (items >= (1ll << 31)) return TB200_ERR_UNSUPPORTED;   // their output rows alone would be 256 GB
     int64_t grid = static_cast<int64_t>(dev.sm_count) * 2;  // persistent: two CTAs per SM
     if (grid > items) grid = items;
-    // A launch of one round starts under its predecessor (28 x 8 heads of 256 rows in a training step: 13 us less per step);
+    // A launch of at most two items per CTA starts under its predecessor (28 x 8 heads of 256 rows in a training step: 13 us less per step);
     // with several rounds per CTA the successor's CTAs take their slots in the order in which this launch's run out of items,
     // which costs the striped walk 4 % (256 ragged samples of up to 1024 rows back to back: 528 against 500 us).
     if (items <= 2 * grid) launch_chained(attn_tc05_kernel, static_cast<unsigned>(grid), kThreads, smem, stream, tq, tk, tv, args);

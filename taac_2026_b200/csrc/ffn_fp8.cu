@@ -23,12 +23,12 @@
 // Every wait on an mbarrier is bounded; a wait that gives up raises the status word and all roles
 // drain out through the same final barrier, where the TMEM allocation is released.
 #include <cuda_fp8.h>
-#include <cudaTypedefs.h>
 
 #include <mutex>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -525,23 +525,6 @@ quant_act_kernel(const uint4* __restrict__ x, uint2* __restrict__ q, float* __re
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess) {
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        } else {
-            cudaGetLastError();
-        }
-    }
-    return fn;
-}
-
 // [rows, k_bytes] row-major bytes, tiles of box_rows x 128 bytes, 128-byte swizzle, zero fill outside
 bool make_tmap_bytes(CUtensorMap* map, const void* base, uint64_t k_bytes, uint64_t rows, uint64_t pitch_bytes,
                      uint32_t box_rows) {

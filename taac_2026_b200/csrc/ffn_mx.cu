@@ -30,10 +30,10 @@
 #include <cstdlib>
 
 #include <cuda_fp8.h>
-#include <cudaTypedefs.h>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -510,14 +510,6 @@ constexpr uint32_t kBHalfBytes = kBBytes / 2;                 // 16 KB: this CTA
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;                   // shared::cluster address of the pair's even CTA
 constexpr int kEpiWarps = kEpiThreads / 32;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, int32_t c0, int32_t c1, uint64_t* leader_bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -974,23 +966,6 @@ quant_act_mx_kernel(const uint4* __restrict__ x, uint2* __restrict__ q, uint8_t*
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess) {
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        } else {
-            cudaGetLastError();
-        }
-    }
-    return fn;
-}
-
 // [rows, k_bytes] row-major bytes, tiles of box_rows x 128 bytes, 128-byte swizzle, zero fill outside
 bool make_tmap_bytes(CUtensorMap* map, const void* base, uint64_t k_bytes, uint64_t rows, uint64_t pitch_bytes, uint32_t box_rows) {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();

@@ -11,10 +11,10 @@
 // tile would be mostly padding (the dispatch at the end of this file says where the lines lie).
 // Every wait on an mbarrier is bounded; a wait that gives up raises the status word and all roles drain out
 // through the final barrier, where the TMEM allocation is released.
-#include <cudaTypedefs.h>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -75,14 +75,6 @@ constexpr uint32_t kWarpBoxBytes = 32 * 128;                  // one epilogue wa
 constexpr size_t kSmemPBytes = static_cast<size_t>(kStagesP) * kStagePBytes + kEpiWarpsP * kWarpBoxBytes + 1024;
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;                   // shared::cluster address of the pair's even CTA
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, int32_t c0, int32_t c1, int32_t c2,
                                                  uint64_t* leader_bar) {
     asm volatile(
@@ -366,23 +358,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         tc_fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess) {
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        } else {
-            cudaGetLastError();
-        }
-    }
-    return fn;
 }
 
 // [groups, rows, row_bytes] bytes, boxes of box_rows x box_bytes (128 or 64) inside one group, swizzle of the box width

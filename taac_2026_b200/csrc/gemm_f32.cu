@@ -22,10 +22,10 @@
 // A row with an infinity, a NaN or a value that rounds to an infinite bf16 has no such split (inf - inf): its outputs are
 // computed again in plain fp32.
 // Two stages of {A: 3 x 16 KB, W: 3 x 16 KB}.  Every wait is bounded and reports through the status word.
-#include <cudaTypedefs.h>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -318,18 +318,6 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const F32Args g) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTmemCols);
     }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess && res == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        cudaGetLastError();
-        return nullptr;
-    }();
-    return fn;
 }
 
 }  // namespace

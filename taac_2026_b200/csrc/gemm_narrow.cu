@@ -1,4 +1,4 @@
-// Grouped bf16 GEMM for 9 .. 256 rows per group on tcgen05 with the operands' roles exchanged:
+// Grouped bf16 GEMM for 9 .. 128 rows per group on tcgen05 with the operands' roles exchanged:
 //     out[g]^T = act(w[g] a[g]^T + bias[g]) (+ residual[g]^T),   a: [groups, M, K], w: [groups, N, K]
 // so that the 128-row side of the tensor-core tile is 128 output columns (always full) and its free side is M, padded to
 // 16.  The layers are bound by streaming their weights: 9 groups of 1536 x 512 give 108 CTAs here instead of 54 tiles of
@@ -11,10 +11,10 @@
 // fp32 partial tile in its own shared memory and the CTAs of the cluster each sum a share of the rows over the ranks in
 // order through distributed shared memory.  Every wait is bounded; one that gives up raises the status word and the roles
 // drain through the barriers.
-#include <cudaTypedefs.h>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -39,14 +39,6 @@ struct NarrowArgs {
     uint32_t tmem_cols;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float ld_peer(uint32_t smem_addr, uint32_t rank) {
     uint32_t at;
     float v;
@@ -208,18 +200,6 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess && res == cudaDriverEntryPointSuccess)
-            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        cudaGetLastError();
-        return nullptr;
-    }();
-    return fn;
-}
-
 // [groups, rows, row_bytes] bytes, boxes of box_rows x 128 bytes inside one group
 bool make_map(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t groups, uint32_t box_rows) {
     const auto fn = encode_fn();
@@ -237,7 +217,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tw, const NarrowArgs& g, in
     static bool attr_set[64] = {};
     const DeviceInfo& dev = device_info();
     if (!attr_set[dev.index]) {
-        cudaFuncSetAttribute(gemm_narrow_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(160 * 1024));
+        cudaFuncSetAttribute(gemm_narrow_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRingBytes + 1024));
         attr_set[dev.index] = true;
     }
     cudaLaunchConfig_t cfg{};
@@ -260,7 +240,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tw, const NarrowArgs& g, in
 
 }  // namespace
 
-// 1 <= M <= 256, N % 128 == 0, K % 64 == 0, act 0 or 1
+// 1 <= M <= 128 (beyond that the 256-row tiles are faster), N % 128 == 0, K % 64 == 0, act 0 or 1
 int gemm_narrow(const void* a, const void* w, const float* bias, const void* residual, void* out, int groups, int M, int N, int K, int act,
                 int32_t* status, cudaStream_t stream) {
     NarrowArgs g{};

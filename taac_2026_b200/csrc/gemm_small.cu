@@ -1,5 +1,5 @@
 // Grouped bf16 GEMM for a handful of rows per group: the same layers as gemm_bf16.cu at request-sized batches,
-//     out[g] = act(a[g] w[g]^T + bias[g]) (+ residual[g]),   a: [groups, M, K] with M <= 8, w: [groups, N, K].
+//     out[g] = act(a[g] w[g]^T + bias[g]) (+ residual[g]),   a: [groups, M, K] with M <= 32, w: [groups, N, K].
 //
 // Bound by streaming the weights (9 groups of 1536 x 512: 14 MB, 2.2 us of HBM time); a 128 x 256 tile per CTA puts 54 of 148
 // SMs to work and took 9 us (18 us for 512 x 2048, now 4.7 and 4.8).  Here a CTA owns 16 output columns of one group and its eight warps split K, so that every

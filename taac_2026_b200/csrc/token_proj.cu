@@ -28,10 +28,10 @@
 // The two exchanges per tile are cluster barriers; every thread of both CTAs walks the same tile list, so they always
 // meet.  Every mbarrier wait is bounded; a warp whose wait gives up raises the status word and keeps walking, so
 // nothing is left waiting for it.  No TMA load carries multicast.
-#include <cudaTypedefs.h>
 
 #include "tb200_common.cuh"
 #include "tb200_ptx.cuh"
+#include "tb200_tmap.cuh"
 
 namespace tb200 {
 void count_launch();
@@ -69,14 +69,6 @@ struct TPArgs {
     float ln_eps, rms_eps;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // shared::cluster address of the same variable in the CTA of rank `peer`
 __device__ __forceinline__ uint32_t map_to_peer(uint32_t local_addr, uint32_t peer) {
     uint32_t r;
@@ -509,23 +501,6 @@ token_project_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 2 * NC);
     }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess) {
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        } else {
-            cudaGetLastError();
-        }
-    }
-    return fn;
 }
 
 // [1, rows, row_bytes] bytes, boxes of box_rows x box_bytes (128 or 64), swizzle of the box width

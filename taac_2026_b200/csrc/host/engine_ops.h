@@ -26,7 +26,13 @@ public:
     Timed(const char* name, const py::dict& meta) : scope_(py::module_::import("taac_2026_b200.ops").attr("timed")(name, **meta)) {
         scope_.attr("__enter__")();
     }
-    ~Timed() { scope_.attr("__exit__")(py::none(), py::none(), py::none()); }
+    ~Timed() {   // also while an error of the launch is on its way: nothing may be thrown from here
+        try {
+            scope_.attr("__exit__")(py::none(), py::none(), py::none());
+        } catch (py::error_already_set& e) {
+            e.discard_as_unraisable("kernel timing");
+        }
+    }
 
 private:
     py::object scope_;
@@ -78,16 +84,6 @@ inline Tensor rms_norm(const Tensor& x, const Tensor& w, const OptTensor& in_bia
     TB200_TIMED("rms_norm", "rows"_a = rows, "cols"_a = cols, "esize"_a = x.element_size());
     check(in_bias.has_value() ? tb200_rmsnorm_bias_fwd(ptr(x), ptr(*in_bias), ptr(w), ptr(out), rows, cols, 1e-6f, dt, stream_of(x))
                               : tb200_rmsnorm_fwd(ptr(x), ptr(w), ptr(out), rows, cols, 1e-6f, dt, stream_of(x)), "cuda rms_norm");
-    return out;
-}
-inline Tensor layer_norm(const Tensor& x, const Tensor& w, const Tensor& b, bool pre_silu) {
-    const auto cols = static_cast<int32_t>(x.size(-1));
-    const int64_t rows = x.numel() / cols;
-    Tensor out = make_like(x.sizes(), x);
-    const int dt = dtype_code(x.scalar_type());
-    TB200_TIMED("layer_norm", "rows"_a = rows, "cols"_a = cols, "esize"_a = x.element_size());
-    check(pre_silu ? tb200_layernorm_silu_fwd(ptr(x), ptr(w), ptr(b), ptr(out), rows, cols, 1e-5f, dt, stream_of(x))
-                   : tb200_layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(out), rows, cols, 1e-5f, dt, stream_of(x)), "cuda layer_norm");
     return out;
 }
 

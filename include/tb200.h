@@ -516,7 +516,8 @@ int tb200_gemm_bf16_few_rows(const void* a, const void* w, const float* bias, co
  * w [rows, K] fp32 -> w_split [rows, 3 K] bf16 = [h | m | l], w = h + m + l.  Once per weight. */
 int tb200_split_f32_weights(const float* w, void* w_split, int64_t rows, int32_t K, void* stream);
 /* out[g] = act(a[g] @ w[g]^T + bias[g]) (+ residual[g]), everything fp32 (w_split [groups, N, 3 K] as above): products of the three-part
- * bf16 forms of both operands, kept down to 2^-24, accumulated in fp32.  act 0 = none, 1 = SiLU; out may be residual.  N % 128 == 0,
+ * bf16 forms of both operands, kept down to 2^-24, summed per 64-wide block of K and the blocks added in fp32; rows with a value that
+ * is infinite, NaN or rounds to an infinite bf16 in plain fp32.  act 0 = none, 1 = SiLU; out may be residual.  N % 128 == 0,
  * K % 64 == 0; 16-byte aligned pointers. */
 int tb200_gemm_f32_grouped(const float* a, const void* w_split, const float* bias, const float* residual, float* out, int32_t groups,
                            int64_t M, int32_t N, int32_t K, int32_t act, int32_t* status_word, void* stream);

@@ -171,12 +171,14 @@ class OneTransInference:
     """Forward-only OneTrans on one GPU.
 
     ``dtype`` is the activation / weight type of the dense path: ``torch.bfloat16`` (serving) or
-    ``torch.float32`` (score-parity runs against the reference's fp32 torch path: dense layers in fp32 through
-    the library, attention through this library's plain fp32 kernel, so nothing between the inputs and the
-    scores is rounded to 16 bits).
+    ``torch.float32`` (score-parity runs against the reference's fp32 torch path: dense layers with three bf16 parts of
+    both operands, no further from the exact product than an fp32 GEMM, attention through this library's plain fp32 kernel, so
+    nothing between the inputs and the scores has fewer than 24 significant bits; widths that are not whole tiles of 128 go to the
+    library's fp32 GEMM).
 
     ``ffn="fp8"`` runs the shared FFN of every block through the e4m3 block-scaled tcgen05 GEMMs
-    (bf16 activations only; needs d_model % 256 == 0 and hidden % 256 == 0); ``"bf16"`` uses cuBLAS.
+    (bf16 activations only; needs d_model % 256 == 0 and hidden % 256 == 0); ``"bf16"`` runs it on this library's bf16 GEMM where the
+    widths are whole tiles of 256 and on cuBLAS otherwise.
 
     ``packed=True`` (single sequence domain) stores only VALID tokens: padded positions never influence
     a score (they are masked as keys, excluded from the pooled means, and as queries only produce rows
@@ -409,9 +411,6 @@ class OneTransInference:
             out.copy_(y)
             return out
         return y
-
-    def _grouped(self, x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, **kw) -> torch.Tensor:
-        return ops.grouped_linear(x, weight, bias, status=self.status_word, **kw)
 
     def raise_if_incomplete(self) -> None:
         """Read the engine's status word (a 4-byte device-to-host copy, which waits for the work enqueued so far)

@@ -771,8 +771,9 @@ def attention_backward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: t
                        padded_query_self: bool = False, key_valid: torch.Tensor | None = None,
                        scale: float | None = None) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """(dq, dk, dv) of ``varlen_attention(q, k, v, ...)`` in the (B, H, L, D) layout for the upstream gradient
-    ``grad_out`` — the plain fp32-arithmetic form of the reference's flash-attention backward
-    (attention/kernels/tilelang.py:440-701): scores are recomputed, nothing is accumulated with atomics."""
+    ``grad_out`` — the reference's flash-attention backward (attention/kernels/tilelang.py:440-701): scores are
+    recomputed, nothing is accumulated with atomics.  16-bit tensors of head_dim 32, 64 or 128 run on the tensor cores with P and
+    dS in two 16-bit parts, the rest in fp32 on the CUDA cores."""
     _require_backend("attention_backward", "cuda")
     _require_cuda_tensors("cuda attention_backward", q, k, v, out, grad_out, seq_len, key_valid)
     if q.dtype not in _DTYPE_CODES or not (q.dtype == k.dtype == v.dtype):

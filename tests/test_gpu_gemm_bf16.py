@@ -89,7 +89,7 @@ def test_grouped_linear_rejects_unsupported_shapes():
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_gated_epilogue(groups, rows, n, k, with_bias):
     """act 2: the weight rows of every 256-column tile are [128 gate rows | 128 value rows]; out = silu(gate) * value.
-    Rows up to 128 take the single-CTA kernel, more rows the CTA-pair kernel."""
+    Rows from 33 on take the CTA-pair kernel (`test_gpu_gemm_few_rows.py` has the fewer ones)."""
     g = torch.Generator().manual_seed(groups * 77 + rows)
     x = torch.randn(groups, rows, k, generator=g).bfloat16().cuda()
     w = (torch.randn(groups, n, k, generator=g) * k ** -0.5).bfloat16().cuda()

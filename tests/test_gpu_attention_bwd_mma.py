@@ -4,7 +4,7 @@ autograd of the fp32 masked softmax.
 Tolerance: inputs are exact in both, P and dS enter their products with at least 16 significant bits and accumulate in fp32,
 so a gradient is off by its own rounding (2^-9 of its value for bf16, 2^-12 for fp16), by the 16-bit rounding of the forward's output in
 delta = rowsum(dO O) (which moves dS by P times 2^-9 |dO||O|) and by the approximate exp2 (2 ulp); 1e-2 (bf16) and 2e-3 (fp16) of the
-largest gradient bound their sum."""
+largest gradient bound their sum.  How many bits P and dS keep shows in `test_gradients_of_any_size_keep_their_bits`."""
 from __future__ import annotations
 
 import pytest

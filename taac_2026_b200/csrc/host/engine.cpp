@@ -552,10 +552,10 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
                          bool select_early, bool one_kernel, int attention_kernel, bool timing) {
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
-    const auto loaded = load_blocks(block_dicts);
-    const std::vector<Block>& stack = loaded->blocks;
+    derived_.use(device_);
     const int64_t b = p->batch, n_feat = static_cast<int64_t>(seq_tables_.size()), max_len = p->length;
-    check_sequence(device_, b, n_feat, max_len, values_in, std::nullopt, time_table_.has_value() ? stamps_in : std::nullopt, request_in);
+    check_sequence(device_, b, n_feat, max_len, values_in, std::nullopt, std::nullopt, request_in);
+    if (time_table_.has_value()) require(stamps_in, "timestamps", device_, {b, max_len});
     if (ns_tokens_in.has_value()) {
         require(ns_tokens_in, "ns_tokens", device_, {b, ns_, d_});
     } else {
@@ -569,10 +569,13 @@ py::tuple Engine::blocks(const std::shared_ptr<Prepared>& p, const Tensor& value
         }
     }
     const Tensor values = i64(values_in), request = i64(request_in);
-    const auto& widths = p->widths;
-    const auto layers = static_cast<int64_t>(stack.size());
     // the non-sequence tokens need nothing the host has to wait for
     const Tensor ns_tokens = (ns_tokens_in.has_value() ? *ns_tokens_in : native_ns_tokens(entities, *p)).contiguous();
+    const auto loaded = load_blocks(block_dicts);
+    const std::vector<Block>& stack = loaded->blocks;
+    const auto& widths = p->widths;
+    const auto layers = static_cast<int64_t>(stack.size());
+    TORCH_CHECK(static_cast<int64_t>(widths.size()) == layers + 1, "OneTransInference: prepared for ", widths.size() - 1, " blocks, the model has ", layers);
     {   // the one host read of a forward; already there when the serving loop prepared the batch ahead of time
         py::gil_scoped_release nogil;
         p->ready.synchronize();
@@ -777,7 +780,8 @@ Tensor Engine::ns_only(const Tensor& tokens, int64_t first_layer, int64_t batch,
                        bool timing) {
     Timing::on() = timing;
     const c10::cuda::CUDAGuard guard(device_);
-    const auto loaded = load_blocks(block_dicts);
+    const auto loaded = loaded_ != nullptr ? loaded_ : load_blocks(block_dicts);   // `blocks` has looked at them in this forward
+    loaded->derived.use(device_);
     const std::vector<Block>& stack = loaded->blocks;
     const int64_t hd = d_ / heads_;
     Tensor tok = (token_major ? tokens : tokens.view({batch, ns_, d_}).transpose(0, 1)).contiguous().view({ns_, batch, d_});

@@ -604,8 +604,9 @@ class OneTransInference:
         if not (self.packed and len(self.domains) == 1):
             return None
         seq = inputs.sequences[self.domains[0]]
-        return self._executor().prepare(seq.values, seq.lengths, seq.timestamps, inputs.request_timestamp,
-                                        self._schedule(seq.values.shape[2]), ops.kernel_timing_on())
+        executor = self._native or self._executor()    # reads no weight: `_predict_packed` looks at those
+        return executor.prepare(seq.values, seq.lengths, seq.timestamps, inputs.request_timestamp,
+                                self._schedule(seq.values.shape[2]), ops.kernel_timing_on())
 
     def _schedule(self, max_len: int) -> list[int]:
         """Static schedule of padded sequence widths (layer 0 .. end) for inputs of ``max_len`` positions."""
@@ -809,7 +810,8 @@ class OneTransInference:
         takes the per-token projections and the per-token FeedForward, and every sample attends causally over
         its ``ns`` tokens.  The block then is six batched or shared matrix products on a token-major
         ``[ns, B, d]`` tensor with no gathers, scatters or shared-weight work that would be overwritten."""
-        return self._executor().ns_only(tokens, first_layer, batch, token_major, self.blocks, self.attention_kernel, ops.kernel_timing_on())
+        executor = self._native or self._executor()    # looked at when this forward began
+        return executor.ns_only(tokens, first_layer, batch, token_major, self.blocks, self.attention_kernel, ops.kernel_timing_on())
 
     @torch.inference_mode()
     def scores(self, inputs, micro_batch: int | None = None, prepared=None) -> torch.Tensor:

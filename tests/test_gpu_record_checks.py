@@ -51,3 +51,17 @@ def test_malformed_records_are_refused():
     with pytest.raises(RuntimeError, match="shape"):
         model.scores(_with(batch, "seq", values=seq.values[:, :, :-1].contiguous(), timestamps=seq.timestamps[:, :-1].contiguous()), prepared=prepared)
     assert torch.equal(model.scores(batch), want)
+
+
+def test_another_number_of_blocks_is_refused():
+    """The row plan is made for the model's blocks: its totals end where they end."""
+    spec, batch = _spec(256), _batch()
+    model = OneTransInference(random_state_dict(spec, seed=1, device="cuda", dtype=torch.bfloat16), spec, dtype=torch.bfloat16)
+    want = model.scores(batch).clone()
+    blocks = model.blocks
+    for other in (blocks[:1], blocks + blocks):
+        model.blocks = other
+        with pytest.raises(RuntimeError, match="blocks"):
+            model.scores(batch)
+    model.blocks = blocks
+    assert torch.equal(model.scores(batch), want)
